@@ -526,12 +526,14 @@ __global__ void __launch_bounds__(256, 4) k_probe(ProbeArgs A) {
     }
     push_warp(want, v, A.front[0], &A.cnt[0], A.cap, &A.words->err);
   }
-  if (!grid_barrier(A.words, A.timeout_ns)) return;
+  __shared__ unsigned long long sh[2];
+  const unsigned long long* src[2] = {&A.cnt[0], nullptr};
+  if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
   uint32_t i = 0;
   uint64_t removed = 0;
   bool stopped = false;
   while (true) {
-    const uint64_t nf = ld_acquire_u64(&A.cnt[i % 3]);
+    const uint64_t nf = sh[0];
     if (nf == 0) break;
     removed += nf;
     // Every block reads the same counts, so all of them stop together.
@@ -562,13 +564,17 @@ __global__ void __launch_bounds__(256, 4) k_probe(ProbeArgs A) {
       A.cnt[(i + 2) % 3] = 0;        // read at the start of round i-1
       A.cnt[3 + ((i + 1) & 1)] = 0;  // big count of round i-1, read before the barrier ending it
     }
-    if (!grid_barrier(A.words, A.timeout_ns)) return;
-    const uint64_t nbig = ld_acquire_u64(bc);
+    // sh[0]: the next frontier's size so far (final when there are no big
+    // rows, whose windows add to it); sh[1]: this round's big rows.
+    src[0] = nc;
+    src[1] = bc;
+    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+    const uint64_t nbig = sh[1];
     if (nbig) {
       // Rows longer than big_row: their 256-entry windows dealt to every warp.
       deal_big_windows<256>(A.big, nbig, A.off, woff, wtmp,
                             [&](uint64_t b, uint64_t e) { drop_neighbours_wide(A, b, e, nx, nc); });
-      if (!grid_barrier(A.words, A.timeout_ns)) return;
+      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
     }
     ++i;
   }
@@ -646,18 +652,8 @@ __device__ __forceinline__ void drop_neighbours_core(const DecompArgs& A, uint64
   }
 }
 
-// One thread per block reads a device counter after a grid barrier and
-// shares it through shared memory (one L2 request per block, not per warp).
-__device__ __forceinline__ unsigned long long block_read(const unsigned long long* p, unsigned long long* sh) {
-  if (threadIdx.x == 0) *sh = ld_acquire_u64(p);
-  __syncthreads();
-  const unsigned long long v = *sh;
-  __syncthreads();
-  return v;
-}
-
 __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
-  __shared__ unsigned long long sh;
+  __shared__ unsigned long long sh[4];
   __shared__ uint64_t woff[kBigBatch + 1];
   __shared__ uint64_t wtmp[33];
   const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
@@ -720,18 +716,22 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
     }
     mn = warp_min(mn);
     if (lane_id() == 0 && mn != 0xffffffffu) atomicMin(mc, (unsigned long long)mn);
-    if (!grid_barrier(A.words, A.timeout_ns)) return;
+    {
+      const unsigned long long* const src[4] = {lc, mc, cc, &A.cnt[(i + 1) % 3]};
+      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+    }
     if (full) {
-      nl = block_read(lc, &sh);
+      nl = sh[0];
       li ^= 1;
     }
-    const unsigned long long dmin = block_read(mc, &sh);
+    const unsigned long long dmin = sh[1];
+    uint64_t nf = sh[3];
     ++ps;
     // The pass's frontier is round i + 1's; i advances even when it is empty,
     // so the next pass counts into a slot no slower block is still reading.
     ++i;
-    if (block_read(&A.cnt[i % 3], &sh) == 0) {
-      nc = block_read(cc, &sh);
+    if (nf == 0) {
+      nc = sh[2];
       ci ^= 1;
       if (full) {
         if (nl == 0) break;  // nothing alive
@@ -748,9 +748,7 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
     ++levels_run;
     // Frontier rounds of level k.
     DropRule R{k, top, nullptr, nullptr, cnext, cc};
-    while (true) {
-      const uint64_t nf = block_read(&A.cnt[i % 3], &sh);
-      if (nf == 0) break;
+    while (nf) {
       const uint32_t* fr = (i & 1) ? A.front[1] : A.front[0];
       R.next = (i & 1) ? A.front[0] : A.front[1];
       R.ncnt = &A.cnt[(i + 1) % 3];
@@ -774,17 +772,19 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
         A.cnt[(i + 2) % 3] = 0;
         A.cnt[3 + ((i + 1) & 1)] = 0;
       }
-      if (!grid_barrier(A.words, A.timeout_ns)) return;
-      const uint64_t nbig = block_read(bc, &sh);
+      const unsigned long long* const src[3] = {R.ncnt, bc, cc};
+      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+      const uint64_t nbig = sh[1];
       if (nbig) {
         deal_big_windows<32>(A.big, nbig, A.off, woff, wtmp,
                              [&](uint64_t b, uint64_t e) { drop_neighbours_core(A, b, e, R); });
-        if (!grid_barrier(A.words, A.timeout_ns)) return;
+        if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       }
+      nf = sh[0];
       ++i;
     }
     // Every candidate push of this pass is in (rounds end with a barrier).
-    nc = block_read(cc, &sh);
+    nc = sh[2];
     ci ^= 1;
     ++k;  // every survivor now has degree >= k
     full = k > top;

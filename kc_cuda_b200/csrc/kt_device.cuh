@@ -20,10 +20,10 @@ enum : uint32_t {
 
 // One block of device words per context (kept zeroed between launches).
 struct DevWords {
-  uint32_t err;
-  uint32_t bar_count;
-  uint32_t bar_gen;
+  uint32_t err;  // err and bar are polled as one 64-bit word
+  uint32_t bar;  // grid barrier: arrivals in the low bits, the phase in bit 31
   uint32_t pad0;
+  uint32_t pad1;
   unsigned long long bad_line;
   unsigned long long counters[16];
 };
@@ -130,40 +130,69 @@ __device__ __forceinline__ T block_sum(T v, T* tmp) {
   return r;
 }
 
+__device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Bounded grid barrier for kernels launched with cudaLaunchCooperativeKernel
 // (which guarantees that every block is resident).  Every block must call it
 // the same number of times.  A wait longer than `timeout_ns` sets
 // kDevErrBarrier and returns; callers test the returned flag and leave the
 // kernel, so a mismatch can never hang the device.  Returns true when no
 // error is flagged.
-__device__ __forceinline__ bool grid_barrier(DevWords* w, unsigned long long timeout_ns) {
+//
+// One thread per block arrives with one atomic -- block 0 adds what flips bit
+// 31 once the others' ones are in, so the word needs no reset and no second
+// atomic -- and polls (error, phase) as one 64-bit word.  Only that thread
+// touches the barrier's words: what every thread needs after it (the flag, and
+// with grid_barrier_read up to N device counters) comes from it through
+// __syncthreads_and and shared memory.  Several thousand warps loading one
+// counter are served one after another by the L2 slice that holds it: with
+// such loads after each barrier the core decomposition of an R-MAT graph of
+// 400,009 ids and 8M records (about 1,100 barriers, 592 blocks) took 8.4 ms,
+// without them 6.75 ms.
+template <int N>
+__device__ __forceinline__ bool grid_barrier_read(DevWords* w, unsigned long long timeout_ns,
+                                                  const unsigned long long* const (&src)[N],
+                                                  unsigned long long* sh) {
   __syncthreads();
+  bool ok = true;
   if (threadIdx.x == 0) {
-    const uint32_t gen = ld_acquire_u32(&w->bar_gen);
+    const uint32_t nb = gridDim.x * gridDim.y * gridDim.z;
     __threadfence();
-    const uint32_t arrived = atomicAdd(&w->bar_count, 1u);
-    if (arrived == gridDim.x * gridDim.y * gridDim.z - 1) {
-      atomicExch(&w->bar_count, 0u);
-      __threadfence();
-      atomicAdd(&w->bar_gen, 1u);
-    } else {
-      const unsigned long long t0 = globaltimer_ns();
-      unsigned spins = 0;
-      while (ld_acquire_u32(&w->bar_gen) == gen) {
-        if (++spins > 32) __nanosleep(spins > 1024 ? 256 : 32);
-        // The bound is checked on the first spin and every 64th after it, so
-        // a bound of 0 gives up at once.
-        if ((spins & 63) == 1 && globaltimer_ns() - t0 >= timeout_ns) {
+    const uint32_t old = atomicAdd(&w->bar, blockIdx.x == 0 ? 0x80000000u - (nb - 1) : 1u);
+    unsigned long long t0 = 0;
+    for (unsigned spins = 0;; ++spins) {
+      const unsigned long long v = ld_acquire_u64(reinterpret_cast<const unsigned long long*>(&w->err));
+      ok = (uint32_t)v == 0;
+      if (!ok || (((uint32_t)(v >> 32) ^ old) & 0x80000000u)) break;
+      // The bound is checked on the first spin and every 64th after it, so
+      // a bound of 0 gives up at once.
+      if ((spins & 63) == 0) {
+        if (spins == 0) t0 = globaltimer_ns();
+        if (globaltimer_ns() - t0 >= timeout_ns) {
           atomicOr(&w->err, kDevErrBarrier);
+          ok = false;
           break;
         }
-        if ((spins & 255) == 0 && ld_volatile_u32(&w->err) != 0) break;
       }
+      if (spins > 64) __nanosleep(spins > 1024 ? 256 : 32);
     }
-    __threadfence();
+    unsigned long long val[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) val[i] = src[i] ? ld_relaxed_u64(src[i]) : 0ULL;
+#pragma unroll
+    for (int i = 0; i < N; ++i) sh[i] = val[i];
   }
-  __syncthreads();
-  return ld_volatile_u32(&w->err) == 0;
+  return __syncthreads_and(ok) != 0;
+}
+
+__device__ __forceinline__ bool grid_barrier(DevWords* w, unsigned long long timeout_ns) {
+  __shared__ unsigned long long none[1];
+  const unsigned long long* const src[1] = {nullptr};
+  return grid_barrier_read<1>(w, timeout_ns, src, none);
 }
 
 // One bulk copy by the TMA engine (cp.async.bulk, no multicast) of `bytes`

@@ -92,9 +92,11 @@ __global__ void __launch_bounds__(kThreads) k_kcore_noalloc(View S, const uint64
     if (want) S.rem[v] = 1;
     push(want, (uint32_t)v, S.front[0], &S.cnt[0], err);
   }
-  if (!grid_barrier(S.words, timeout_ns)) return;
+  __shared__ unsigned long long sh[1];
+  const unsigned long long* src[1] = {&S.cnt[0]};
+  if (!grid_barrier_read(S.words, timeout_ns, src, sh)) return;
   for (uint32_t i = 0;; ++i) {
-    const uint64_t nf = ld_acquire_u64(&S.cnt[i % 3]);
+    const uint64_t nf = sh[0];
     if (nf == 0) break;
     const uint32_t* fr = S.front[i & 1];
     uint32_t* nx = S.front[(i + 1) & 1];
@@ -116,7 +118,8 @@ __global__ void __launch_bounds__(kThreads) k_kcore_noalloc(View S, const uint64
       }
     }
     if (gtid == 0) S.cnt[(i + 2) % 3] = 0;  // read at the start of round i-1
-    if (!grid_barrier(S.words, timeout_ns)) return;
+    src[0] = nc;
+    if (!grid_barrier_read(S.words, timeout_ns, src, sh)) return;
   }
   for (uint64_t v = gtid; v < n; v += gthreads) member[v] = S.rem[v] == kAlive;
 }

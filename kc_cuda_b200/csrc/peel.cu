@@ -431,8 +431,10 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_cascade(Pe
   uint32_t* su = dense_smem + warp_id() * A.R.W;
   const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ unsigned long long sh[1];
+  const unsigned long long* src[1] = {&A.cnt[0]};
   level_frontier(A, A.r0, gtid, gthreads);
-  if (!grid_barrier(A.words, A.timeout_ns)) return;
+  if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
   const uint64_t gwarps = gthreads >> 5, gwarp = gtid >> 5;
   uint64_t tdeg = 0, tdec = 0, trec = 0;
   uint64_t alive = A.na;
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_cascade(Pe
   bool ok = true;
   bool gave_up = false;
   while (true) {
-    const uint64_t nf = ld_acquire_u64(&A.cnt[i % 3]);
+    const uint64_t nf = sh[0];
     if (nf == 0) break;
     // Every block reads the same counts, so all of them give up together.
     if (alive - nf < A.fail_below) {
@@ -489,7 +491,8 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_cascade(Pe
         for (uint64_t f = gwarp; f < nf; f += gwarps) peel_edge(A, fr[f], r, nx, nc, tdeg, tdec);
     }
     if (gtid == 0) A.cnt[(i + 2) % 3] = 0;  // read at the start of round i-1, next written in round i+1
-    if (!grid_barrier(A.words, A.timeout_ns)) {
+    src[0] = nc;
+    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) {
       ok = false;
       break;
     }
