@@ -5,8 +5,8 @@
 // decrements the degrees of its surviving neighbours; a neighbour whose
 // degree steps from k to k-1 (atomicSub returns k) joins the next frontier,
 // so every vertex enters a frontier at most once.  Rows of more than
-// kcore_big_row (option, 512) entries are cut into 32-entry windows dealt to
-// every warp of the grid, so hub rows do not serialise on one warp.
+// kcore_big_row (option, 512) entries are cut into windows dealt to every
+// warp of the grid, so hub rows do not serialise on one warp.
 //
 // The search for the maximum core (the reference steps k by a fixed stride
 // with host backups, src/kc.cu:770-884) ramps k geometrically from the
@@ -24,11 +24,10 @@
 
 #include "compact.cuh"
 #include "kcore.h"
+#include "rows.cuh"
 
 namespace kt {
 namespace {
-
-constexpr unsigned kBigRow = 2048;
 
 struct AliveF {
   const uint32_t* rem;
@@ -60,64 +59,6 @@ __device__ __forceinline__ void push_warp(bool want, uint32_t item, uint32_t* li
       list[p] = item;
     else
       atomicOr(err, kDevErrCapacity);
-  }
-}
-
-constexpr unsigned kBigBatch = 1024;  // big rows per batch of dealt windows
-
-// Deals the kWin-entry windows of the big rows big[0..nbig) to every warp of
-// the grid, so one long row is spread over the whole GPU instead of one
-// block: each block lists the rows' first window numbers (the same block scan
-// in every block, kBigBatch rows at a time) and warp w takes windows w,
-// w + warps, ...; `drop(b, e)` handles entries [b, e) (at most kWin) of a
-// row.  Every thread of the block must call it (it synchronises the block);
-// blocks have 256 threads.
-template <unsigned kWin, class Drop>
-__device__ __forceinline__ void deal_big_windows(const uint32_t* __restrict__ big, uint64_t nbig,
-                                                 const uint64_t* __restrict__ off, uint64_t* woff, uint64_t* tmp,
-                                                 Drop drop) {
-  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
-  constexpr unsigned per = kBigBatch / 256;  // rows per thread
-  for (uint64_t base = 0; base < nbig; base += kBigBatch) {
-    const uint64_t left = nbig - base;
-    const uint32_t cnt = left < kBigBatch ? (uint32_t)left : kBigBatch;
-    uint64_t w[per];
-    uint64_t sum = 0;
-#pragma unroll
-    for (unsigned j = 0; j < per; ++j) {
-      const uint32_t r = threadIdx.x * per + j;
-      w[j] = 0;
-      if (r < cnt) {
-        const uint32_t v = big[base + r];
-        w[j] = (off[v + 1] - off[v] + kWin - 1) / kWin;
-      }
-      sum += w[j];
-    }
-    uint64_t total;
-    uint64_t pre = block_excl_scan<uint64_t>(sum, tmp, &total);
-#pragma unroll
-    for (unsigned j = 0; j < per; ++j) {
-      const uint32_t r = threadIdx.x * per + j;
-      if (r < cnt) woff[r] = pre;
-      pre += w[j];
-    }
-    if (threadIdx.x == 0) woff[cnt] = total;
-    __syncthreads();
-    for (uint64_t x = gwarp; x < total; x += gwarps) {
-      uint32_t lo = 0, hi = cnt;  // last row with woff <= x
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (woff[mid] <= x)
-          lo = mid;
-        else
-          hi = mid;
-      }
-      const uint32_t v = big[base + lo];
-      const uint64_t b = off[v] + (x - woff[lo]) * kWin, e = min(off[v + 1], b + kWin);
-      drop(b, e);
-    }
-    __syncthreads();
   }
 }
 
@@ -234,20 +175,28 @@ __global__ void k_recount(const uint32_t* __restrict__ alive, uint64_t n_alive, 
   }
 }
 
-// Big rows of the recount: one block per row, a warp-level count and one
-// atomic per warp per row.
-__global__ void k_recount_big(const uint32_t* __restrict__ big, const unsigned long long* nbig_p,
-                              const uint64_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                              const uint32_t* __restrict__ rem, uint32_t* __restrict__ deg) {
-  const uint64_t nbig = *nbig_p;
-  for (uint64_t bi = blockIdx.x; bi < nbig; bi += gridDim.x) {
-    const uint32_t v = big[bi];
-    const uint64_t b = off[v], e = off[v + 1];
-    uint32_t c = 0;
-    for (uint64_t j = b + threadIdx.x; j < e; j += blockDim.x) c += rem[adj[j]] == kAlive;
-    c = warp_sum(c);
-    if (lane_id() == 0 && c) atomicAdd(&deg[v], c);
-  }
+// Big rows of the recount: their 256-entry windows dealt to every warp, 8
+// entries per lane in flight, one atomic per window.
+__global__ void __launch_bounds__(256) k_recount_big(const uint32_t* __restrict__ big,
+                                                     const unsigned long long* nbig_p,
+                                                     const uint64_t* __restrict__ off,
+                                                     const uint32_t* __restrict__ adj,
+                                                     const uint32_t* __restrict__ rem, uint32_t* __restrict__ deg) {
+  __shared__ uint64_t woff[kBigBatch + 1];
+  __shared__ uint64_t tmp[33];
+  constexpr unsigned kPer = 8;
+  deal_windows<32 * kPer>(
+      *nbig_p, [&](uint64_t x) { return big[x]; }, off, woff, tmp, [&](uint64_t x, uint64_t b, uint64_t e) {
+        const uint64_t j0 = b + lane_id();
+        uint32_t w[kPer];
+#pragma unroll
+        for (unsigned k = 0; k < kPer; ++k) w[k] = j0 + 32 * k < e ? adj[j0 + 32 * k] : 0u;
+        uint32_t n = 0;
+#pragma unroll
+        for (unsigned k = 0; k < kPer; ++k) n += j0 + 32 * k < e && rem[w[k]] == kAlive;
+        n = warp_sum(n);
+        if (lane_id() == 0 && n) atomicAdd(&deg[big[x]], n);
+      });
 }
 
 __global__ void k_revive(uint32_t* __restrict__ rem, uint64_t n, uint32_t newer_than) {
@@ -292,140 +241,6 @@ __global__ void k_core_from_tags(const uint32_t* __restrict__ rem, uint64_t n, c
   }
 }
 
-
-// Compacted copy of the alive part: row i of the new graph is alive[i] with
-// only its alive neighbours, renumbered.
-__global__ void k_compact_rows(const uint32_t* __restrict__ alive, uint64_t na, const uint64_t* __restrict__ off,
-                               const uint32_t* __restrict__ adj, const uint32_t* __restrict__ rem,
-                               const uint32_t* __restrict__ newid, const uint64_t* __restrict__ noff,
-                               uint32_t* __restrict__ nadj) {
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  for (uint64_t i = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id(); i < na; i += warps) {
-    const uint32_t v = alive[i];
-    const uint64_t b = off[v], e = off[v + 1];
-    if (e - b > kBigRow) continue;  // k_compact_big_rows
-    uint64_t pos = noff[i];
-    const uint64_t end = noff[i + 1];
-    for (uint64_t j = b + lane_id(); j < b + ((e - b + 31) & ~31ULL); j += 32) {
-      bool keep = false;
-      uint32_t w = 0;
-      if (j < e) {
-        w = adj[j];
-        keep = rem[w] == kAlive;
-      }
-      const unsigned bal = __ballot_sync(kFull, keep);
-      const uint64_t p = pos + __popc(bal & lanemask_lt());
-      if (keep && p < end) nadj[p] = newid[w];
-      pos += __popc(bal);
-    }
-  }
-}
-
-// Alive-list indices whose rows are longer than kBigRow (compacted apart).
-struct BigAliveRow {
-  const uint32_t* alive;
-  const uint64_t* off;
-  __device__ bool keep(uint64_t i) const {
-    const uint32_t v = alive[i];
-    return off[v + 1] - off[v] > kBigRow;
-  }
-  __device__ uint32_t value(uint64_t i) const { return (uint32_t)i; }
-};
-
-// Rows longer than kBigRow in the compaction: their 256-entry chunks are
-// dealt to every warp of the grid (each block lists the rows' first chunk
-// numbers with the same block scan, kBigBatch rows at a time); a warp loads
-// its chunk's 8 entries per lane, their alive flags and new ids before it
-// uses any of them (so 8 loads of each kind are in flight per lane), and
-// the chunk's kept entries go to the row's next free positions (a per-row
-// cursor, one atomic per chunk), so a hub row is spread over the whole GPU.
-// Entry order within these rows is not kept; nothing downstream needs it.
-constexpr unsigned kCompactChunk = 256;  // entries per warp step (8 per lane)
-
-__global__ void __launch_bounds__(256) k_compact_big_rows(const uint32_t* __restrict__ rows, uint64_t nrows,
-                                                          const uint32_t* __restrict__ alive,
-                                                          const uint64_t* __restrict__ off,
-                                                          const uint32_t* __restrict__ adj,
-                                                          const uint32_t* __restrict__ rem,
-                                                          const uint32_t* __restrict__ newid,
-                                                          const uint64_t* __restrict__ noff,
-                                                          uint32_t* __restrict__ cursor, uint32_t* __restrict__ nadj) {
-  __shared__ uint64_t woff[kBigBatch + 1];
-  __shared__ uint64_t tmp[33];
-  constexpr unsigned kPer = kCompactChunk / 32;
-  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
-  const unsigned l = lane_id();
-  constexpr unsigned per = kBigBatch / 256;  // rows per thread
-  for (uint64_t base = 0; base < nrows; base += kBigBatch) {
-    const uint64_t left = nrows - base;
-    const uint32_t cnt = left < kBigBatch ? (uint32_t)left : kBigBatch;
-    uint64_t w[per];
-    uint64_t sum = 0;
-#pragma unroll
-    for (unsigned j = 0; j < per; ++j) {
-      const uint32_t r = threadIdx.x * per + j;
-      w[j] = 0;
-      if (r < cnt) {
-        const uint32_t v = alive[rows[base + r]];
-        w[j] = (off[v + 1] - off[v] + kCompactChunk - 1) / kCompactChunk;
-      }
-      sum += w[j];
-    }
-    uint64_t total;
-    uint64_t pre = block_excl_scan<uint64_t>(sum, tmp, &total);
-#pragma unroll
-    for (unsigned j = 0; j < per; ++j) {
-      const uint32_t r = threadIdx.x * per + j;
-      if (r < cnt) woff[r] = pre;
-      pre += w[j];
-    }
-    if (threadIdx.x == 0) woff[cnt] = total;
-    __syncthreads();
-    for (uint64_t x = gwarp; x < total; x += gwarps) {
-      uint32_t lo = 0, hi = cnt;  // last row with woff <= x
-      while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (woff[mid] <= x)
-          lo = mid;
-        else
-          hi = mid;
-      }
-      const uint32_t i = rows[base + lo];
-      const uint32_t v = alive[i];
-      const uint64_t e = off[v + 1];
-      const uint64_t j0 = off[v] + (x - woff[lo]) * kCompactChunk + l;
-      uint32_t u[kPer];
-#pragma unroll
-      for (unsigned k = 0; k < kPer; ++k) u[k] = j0 + 32 * k < e ? adj[j0 + 32 * k] : 0u;
-      bool keep[kPer];
-#pragma unroll
-      for (unsigned k = 0; k < kPer; ++k) keep[k] = j0 + 32 * k < e && rem[u[k]] == kAlive;
-#pragma unroll
-      for (unsigned k = 0; k < kPer; ++k) u[k] = keep[k] ? newid[u[k]] : 0u;
-      unsigned bal[kPer];
-      uint32_t kept = 0;
-#pragma unroll
-      for (unsigned k = 0; k < kPer; ++k) {
-        bal[k] = __ballot_sync(kFull, keep[k]);
-        kept += __popc(bal[k]);
-      }
-      if (!kept) continue;
-      uint32_t at = 0;
-      if (l == 0) at = atomicAdd(&cursor[base + lo], kept);
-      at = __shfl_sync(kFull, at, 0);
-      const uint64_t row0 = noff[i], row1 = noff[i + 1];
-      uint64_t p0 = row0 + at;
-#pragma unroll
-      for (unsigned k = 0; k < kPer; ++k) {
-        const uint64_t p = p0 + __popc(bal[k] & lanemask_lt());
-        if (keep[k] && p < row1) nadj[p] = u[k];
-        p0 += __popc(bal[k]);
-      }
-    }
-    __syncthreads();
-  }
-}
 
 __global__ void k_compact_meta(const uint32_t* __restrict__ alive, uint64_t na, const uint32_t* __restrict__ deg,
                                const uint32_t* __restrict__ oldmap, uint32_t* __restrict__ newid,
@@ -572,8 +387,9 @@ __global__ void __launch_bounds__(256, 4) k_probe(ProbeArgs A) {
     const uint64_t nbig = sh[1];
     if (nbig) {
       // Rows longer than big_row: their 256-entry windows dealt to every warp.
-      deal_big_windows<256>(A.big, nbig, A.off, woff, wtmp,
-                            [&](uint64_t b, uint64_t e) { drop_neighbours_wide(A, b, e, nx, nc); });
+      deal_windows<256>(
+          nbig, [&](uint64_t x) { return A.big[x]; }, A.off, woff, wtmp,
+          [&](uint64_t, uint64_t b, uint64_t e) { drop_neighbours_wide(A, b, e, nx, nc); });
       if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
     }
     ++i;
@@ -776,8 +592,9 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
       if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       const uint64_t nbig = sh[1];
       if (nbig) {
-        deal_big_windows<32>(A.big, nbig, A.off, woff, wtmp,
-                             [&](uint64_t b, uint64_t e) { drop_neighbours_core(A, b, e, R); });
+        deal_windows<32>(
+            nbig, [&](uint64_t x) { return A.big[x]; }, A.off, woff, wtmp,
+            [&](uint64_t, uint64_t b, uint64_t e) { drop_neighbours_core(A, b, e, R); });
         if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       }
       nf = sh[0];
@@ -852,24 +669,8 @@ void KCore::compact_to_alive(Ctx* c, uint32_t level) {
   const uint64_t n2 = read_word<uint64_t>(c, L.off.as<uint64_t>() + na);
   L.m = n2 / 2;
   L.adj.alloc(c, (n2 ? n2 : 1) * sizeof(uint32_t));
-  k_compact_rows<<<grid_for(na * 32, 256, c->num_sms * 16), 256, 0, c->stream>>>(
-      alive.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem.as<uint32_t>(),
-      newid.as<uint32_t>(), L.off.as<uint64_t>(), L.adj.as<uint32_t>());
-  KT_LAUNCHED(c);
-  {
-    DBuf rows(c, (na ? na : 1) * sizeof(uint32_t));
-    const uint64_t nbig = compact(c, na, BigAliveRow{alive.as<uint32_t>(), g.off.as<uint64_t>()},
-                                  rows.as<uint32_t>());
-    if (nbig) {
-      DBuf cursor(c, nbig * sizeof(uint32_t));
-      zero(c, cursor.get(), cursor.bytes());
-      k_compact_big_rows<<<c->num_sms * 8, 256, 0, c->stream>>>(
-          rows.as<uint32_t>(), nbig, alive.as<uint32_t>(), g.off.as<uint64_t>(), g.adj.as<uint32_t>(),
-          rem.as<uint32_t>(), newid.as<uint32_t>(), L.off.as<uint64_t>(), cursor.as<uint32_t>(),
-          L.adj.as<uint32_t>());
-      KT_LAUNCHED(c);
-    }
-  }
+  copy_rows(c, alive.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem.as<uint32_t>(),
+            newid.as<uint32_t>(), L.off.as<uint64_t>(), g.max_deg, OutColumn{L.adj.as<uint32_t>()});
   L.max_deg = g.max_deg;  // an upper bound is enough here
   newid.release();
   // Install; the previous compaction, if any, is kept for restores.
@@ -905,7 +706,7 @@ void KCore::recount(Ctx* c) {
       alive.as<uint32_t>(), n_alive, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem.as<uint32_t>(),
       deg.as<uint32_t>(), big.as<uint32_t>(), nbig, n, &dev_words(c)->err, big_row(c));
   KT_LAUNCHED(c);
-  k_recount_big<<<c->num_sms * 4, 256, 0, c->stream>>>(big.as<uint32_t>(), nbig, g.off.as<uint64_t>(),
+  k_recount_big<<<c->num_sms * 8, 256, 0, c->stream>>>(big.as<uint32_t>(), nbig, g.off.as<uint64_t>(),
                                                        g.adj.as<uint32_t>(), rem.as<uint32_t>(),
                                                        deg.as<uint32_t>());
   KT_LAUNCHED(c);

@@ -17,6 +17,7 @@
 
 #include "compact.cuh"
 #include "dense.cuh"
+#include "rows.cuh"
 #include "subgraph.h"
 
 namespace kt {
@@ -61,60 +62,6 @@ __global__ void k_order_apply(const uint64_t* __restrict__ keys, uint64_t na, ui
     orig[i] = v;  // ids of the graph being read; mapped below if it is a compacted copy
     newid[v] = (uint32_t)i;
     sdeg[i] = grouped ? deg[v] : (uint32_t)(k >> 32);
-  }
-}
-
-// Emits (r << 32 | newid[w]) for every alive neighbour w of orig[r], at
-// off[r] + rank.  Warp per row.
-__global__ void k_emit(const uint32_t* __restrict__ orig, uint64_t na, const uint64_t* __restrict__ goff,
-                       const uint32_t* __restrict__ gadj, const uint32_t* __restrict__ rem,
-                       const uint32_t* __restrict__ newid, const uint64_t* __restrict__ soff,
-                       uint64_t* __restrict__ keys) {
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  for (uint64_t r = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id(); r < na; r += warps) {
-    const uint32_t v = orig[r];
-    const uint64_t b = goff[v], e = goff[v + 1];
-    uint64_t pos = soff[r];
-    const uint64_t row_end = soff[r + 1];  // a degree mismatch must not spill into the next row
-    for (uint64_t j = b + lane_id(); j < b + ((e - b + 31) & ~31ULL); j += 32) {
-      bool keep = false;
-      uint32_t w = 0;
-      if (j < e) {
-        w = gadj[j];
-        keep = rem == nullptr || rem[w] == kAlive;
-      }
-      const unsigned bal = __ballot_sync(kFull, keep);
-      const uint64_t p = pos + __popc(bal & lanemask_lt());
-      if (keep && p < row_end) keys[p] = ((uint64_t)r << 32) | newid[w];
-      pos += __popc(bal);
-    }
-  }
-}
-
-// As k_emit, but the entries are the new column ids alone, written into the
-// rows of adj (unsorted within a row).
-__global__ void k_emit_cols(const uint32_t* __restrict__ orig, uint64_t na, const uint64_t* __restrict__ goff,
-                            const uint32_t* __restrict__ gadj, const uint32_t* __restrict__ rem,
-                            const uint32_t* __restrict__ newid, const uint64_t* __restrict__ soff,
-                            uint32_t* __restrict__ adj) {
-  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  for (uint64_t r = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id(); r < na; r += warps) {
-    const uint32_t v = orig[r];
-    const uint64_t b = goff[v], e = goff[v + 1];
-    uint64_t pos = soff[r];
-    const uint64_t row_end = soff[r + 1];  // a degree mismatch must not spill into the next row
-    for (uint64_t j = b + lane_id(); j < b + ((e - b + 31) & ~31ULL); j += 32) {
-      bool keep = false;
-      uint32_t w = 0;
-      if (j < e) {
-        w = gadj[j];
-        keep = rem == nullptr || rem[w] == kAlive;
-      }
-      const unsigned bal = __ballot_sync(kFull, keep);
-      const uint64_t p = pos + __popc(bal & lanemask_lt());
-      if (keep && p < row_end) adj[p] = newid[w];
-      pos += __popc(bal);
-    }
   }
 }
 
@@ -318,10 +265,8 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
   const bool bitmap_rows = n2 && max_range <= kMaxBitmapRange && bitmap_words <= 4 * n2;
   s.adj.alloc(c, (n2 ? n2 : 1) * sizeof(uint32_t));
   if (bitmap_rows) {
-    k_emit_cols<<<grid_for(na * 32, 256, c->num_sms * 16), 256, 0, c->stream>>>(
-        s.orig.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem, newid.as<uint32_t>(),
-        s.off.as<uint64_t>(), s.adj.as<uint32_t>());
-    KT_LAUNCHED(c);
+    copy_rows(c, s.orig.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem, newid.as<uint32_t>(),
+              s.off.as<uint64_t>(), g.max_deg, OutColumn{s.adj.as<uint32_t>()});
     newid.release();
     const size_t smem = (size_t)((max_range + 31) / 32) * sizeof(uint32_t);
     if (smem > 48 * 1024)
@@ -332,10 +277,8 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
     KT_LAUNCHED(c);
   } else {
     DBuf keys(c, (n2 ? n2 : 1) * sizeof(uint64_t));
-    k_emit<<<grid_for(na * 32, 256, c->num_sms * 16), 256, 0, c->stream>>>(
-        s.orig.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem, newid.as<uint32_t>(),
-        s.off.as<uint64_t>(), keys.as<uint64_t>());
-    KT_LAUNCHED(c);
+    copy_rows(c, s.orig.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem, newid.as<uint32_t>(),
+              s.off.as<uint64_t>(), g.max_deg, OutKey{keys.as<uint64_t>()});
     newid.release();
     // Row in bits 32.., column in bits 0..: constant digits are skipped.
     radix_sort_u64(c, keys.as<uint64_t>(), nullptr, n2, 64);
