@@ -43,9 +43,28 @@ void reset_words(Ctx* c) {
   KT_CUDA(cudaMemsetAsync(&dev_words(c)->bad_line, 0xff, sizeof(unsigned long long), c->stream));
 }
 
+static void throw_words(Ctx* c, const DevWords& w, const char* stage);
+
 void check_words(Ctx* c, const char* stage) {
   DevWords w;
-  copy_d2h(c, &w, c->words.get(), sizeof(DevWords));
+  read_checked(c, &w, c->words.get(), sizeof(DevWords), stage);
+}
+
+void read_checked(Ctx* c, void* dst, const void* src, size_t bytes, const char* stage) {
+  char* host = reinterpret_cast<char*>(c->pinned);
+  static_assert(sizeof(DevWords) <= 1024, "beside the result in the pinned words");
+  if (bytes > 3072) throw Error(KT_ERR_CUDA, "result larger than the pinned words");
+  c->d2h_bytes += bytes + sizeof(DevWords);
+  KT_CUDA(cudaMemcpyAsync(host, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+  KT_CUDA(cudaMemcpyAsync(host + 3072, c->words.get(), sizeof(DevWords), cudaMemcpyDeviceToHost, c->stream));
+  sync(c);
+  std::memcpy(dst, host, bytes);
+  DevWords w;
+  std::memcpy(&w, host + 3072, sizeof(w));
+  throw_words(c, w, stage);
+}
+
+static void throw_words(Ctx* c, const DevWords& w, const char* stage) {
   if (!w.err) return;
   char buf[256];
   kt_status s = KT_ERR_CUDA;

@@ -4,7 +4,9 @@
 // < k form the first frontier, and each round removes the frontier and
 // decrements the degrees of its surviving neighbours; a neighbour whose
 // degree steps from k to k-1 (atomicSub returns k) joins the next frontier,
-// so every vertex enters a frontier at most once.  Rows of more than
+// so every vertex enters a frontier at most once.  The whole search runs in
+// one cooperative launch (k_core_search), which ends early only for a
+// compaction.  Rows of more than
 // kcore_big_row (option, 512) entries are cut into windows dealt to every
 // warp of the grid, so hub rows do not serialise on one warp.
 //
@@ -260,144 +262,317 @@ __global__ void k_members_mapped(const uint32_t* __restrict__ rem, uint64_t n, c
 }
 
 
-struct ProbeArgs {
+// Rows of a frontier, 32 entries a step and kWide steps in flight, handed to
+// `drop(w, ok)`: lane l of step t gets neighbour w[t] where ok[t].  A warp
+// takes up to 32 vertices (fewer when the frontier is small for the grid) and
+// walks their rows end to end, so short rows fill its lanes: a warp per vertex
+// left most of them idle and waited for one entry after another (core
+// decomposition of an R-MAT graph of 400,009 ids and 8M records: 5.3 -> 4.7 ms
+// with this walk).  Rows longer than big_row go to big[0..*nbig).
+constexpr unsigned kWide = 4;
+
+template <class Drop>
+__device__ __forceinline__ void walk_rows(const uint32_t* __restrict__ front, uint64_t nf,
+                                          const uint64_t* __restrict__ off, const uint32_t* __restrict__ adj,
+                                          uint32_t big_row, uint32_t* __restrict__ big, unsigned long long* nbig,
+                                          uint64_t cap, uint32_t* err, Drop drop) {
+  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
+  const unsigned lane = lane_id();
+  const uint64_t share = (nf + gwarps - 1) / gwarps;
+  const uint32_t per = share < 32 ? (uint32_t)share : 32u;
+  for (uint64_t f0 = gwarp * per; f0 < nf; f0 += gwarps * per) {
+    uint64_t start = 0;
+    uint32_t len = 0, v = 0;
+    if (lane < per && f0 + lane < nf) {
+      v = front[f0 + lane];
+      start = off[v];
+      const uint64_t l = off[v + 1] - start;
+      len = l > big_row ? 0xffffffffu : (uint32_t)l;
+    }
+    push_warp(len == 0xffffffffu, v, big, nbig, cap, err);
+    if (len == 0xffffffffu) len = 0;
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(kFull, incl, 31), excl = incl - len;
+    start -= excl;  // entry p of the walk is adj[start + p] of its row's lane
+    for (uint32_t base = 0; base < total; base += 32 * kWide) {
+      uint32_t w[kWide];
+      bool ok[kWide];
+#pragma unroll
+      for (unsigned t = 0; t < kWide; ++t) {
+        const uint32_t p = base + 32 * t + lane;
+        uint32_t from = 0;  // the last row starting at or before p
+        if (per > 1) {
+#pragma unroll
+          for (uint32_t st = 16; st >= 1; st >>= 1) {
+            const uint32_t x = __shfl_sync(kFull, excl, from + st);
+            if (x <= p) from += st;
+          }
+        }
+        const uint64_t s = __shfl_sync(kFull, start, from);
+        ok[t] = p < total;
+        w[t] = ok[t] ? adj[s + p] : 0u;
+      }
+      drop(w, ok);
+    }
+  }
+}
+
+// What the search leaves for the host.
+constexpr uint32_t kMaxProbes = 64;  // probes of one launch
+struct SearchOut {
+  uint64_t n_alive, rounds;
+  uint32_t lo, hi;       // the lo-core is not empty, the hi-core is
+  uint32_t ramp;         // still doubling
+  uint32_t list;         // alive list in use (0 or 1)
+  uint32_t probes;
+  uint32_t compact;      // ended for a compaction (to the last probe's level)
+  uint32_t k[kMaxProbes];
+  uint32_t left[kMaxProbes];  // 0: the probe failed and was undone
+};
+static_assert(sizeof(SearchOut) <= 1024, "read through the context's pinned words");
+
+struct SearchArgs {
   const uint64_t* off;
   const uint32_t* adj;
   uint32_t* deg;
   uint32_t* rem;
-  const uint32_t* alive;
+  uint32_t* snap;       // degrees before the probe, of the alive vertices
+  uint32_t* alive[2];   // the list in use, and the one the next is written to
   uint64_t n_alive;
   uint32_t* front[2];
   uint32_t* big;
-  unsigned long long* cnt;  // [0..2] frontier sizes, [3..4] big-row counts, [5] rounds, [6] removed, [7] stopped
+  // [0..2] frontier sizes, [3..4] big-row counts, [5] least degree, [6] sum of
+  // degrees; then one kept count per block
+  unsigned long long* cnt;
   uint64_t cap;
-  uint32_t k, tag;
-  bool may_stop;     // stop once fewer than k+1 vertices can remain (the k-core is then empty)
-  uint32_t big_row;  // rows longer than this are dealt to all warps in windows
+  uint32_t lo, hi, ramp;  // search (lo, hi); hi = lo + 1 with fixed: one probe at level lo
+  uint32_t fixed;
+  uint32_t tag;           // of the first probe
+  uint64_t compact_below; // end when the core's degrees add up to less than this
+  uint32_t big_row;       // rows longer than this are dealt to all warps in windows
+  SearchOut* out;
   DevWords* words;
   unsigned long long timeout_ns;
 };
 
-__device__ __forceinline__ void drop_neighbours(const ProbeArgs& A, uint64_t b, uint64_t e, uint32_t* next,
-                                                unsigned long long* ncnt) {
-  for (uint64_t j = b + lane_id(); j < b + ((e - b + 31) & ~31ULL); j += 32) {
-    bool want = false;
-    uint32_t w = 0;
-    if (j < e) {
-      w = A.adj[j];
-      if (A.rem[w] == kAlive) {
-        const uint32_t old = atomicSub(&A.deg[w], 1u);
-        if (old == A.k) {
-          A.rem[w] = A.tag;
+// Decrements the degrees of N neighbours per lane; the lanes' loads and
+// atomics of all N are in flight before any result is used.
+template <unsigned N>
+__device__ __forceinline__ void drop_entries(const SearchArgs& A, const uint32_t (&w)[N], const bool (&ok)[N],
+                                             uint32_t k, uint32_t tag, uint32_t* next, unsigned long long* ncnt) {
+  bool live[N];
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) live[t] = ok[t] && A.rem[w[t]] == kAlive;
+  uint32_t old[N];
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) old[t] = live[t] ? atomicSub(&A.deg[w[t]], 1u) : 0u;
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) {
+    const bool want = live[t] && old[t] == k;
+    if (want) A.rem[w[t]] = tag;
+    push_warp(want, w[t], next, ncnt, A.cap, &A.words->err);
+  }
+}
+
+// The maximum-core search in one cooperative launch.  Each probe starts with a
+// pass over the alive list, which undoes a failed probe (degrees from the
+// snapshot) or takes the snapshot, and picks the first frontier; then the
+// rounds; a probe that leaves vertices ends with an ordered compaction of the
+// alive list (each block counts and writes its own stretch of it) that also
+// finds the least degree and the sum of the degrees.  With a launch per probe
+// the host's reads and the launches between two probes cost 70 us of the 100
+// us that a probe took on graphs of up to a million edges.
+__global__ void __launch_bounds__(256, 4) k_core_search(SearchArgs A) {
+  __shared__ uint64_t woff[kBigBatch + 1];
+  __shared__ uint64_t wtmp[33];
+  __shared__ unsigned long long sh[2];
+  const unsigned long long* src[2] = {nullptr, nullptr};
+  const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
+  const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long* kept = A.cnt + 7;
+  uint32_t lo = A.lo, hi = A.hi, ramp = A.ramp;
+  uint64_t na = A.n_alive, rounds = 0;
+  uint32_t list = 0, probes = 0, tag = A.tag, compact = 0;
+  uint32_t i = 0;  // round index, continued across probes (it picks the counters)
+  bool undo = false;
+  while ((hi - lo > 1 || A.fixed) && na && probes < kMaxProbes) {
+    uint32_t k;
+    if (A.fixed) {
+      k = lo;
+    } else {
+      k = ramp ? (2ull * lo < hi - 1 ? 2 * lo : hi - 1) : lo + (hi - lo) / 2;
+      if (k <= lo) k = lo + 1;
+    }
+    // Slot (i + 1) % 3 is zero, and slot (i + 2) % 3 and the next round's big
+    // count were read before the barriers of the rounds before.
+    if (gtid == 0) {
+      A.cnt[(i + 2) % 3] = 0;
+      A.cnt[3 + ((i + 1) & 1)] = 0;
+      A.cnt[5] = ~0ULL;
+      A.cnt[6] = 0;
+    }
+    const uint32_t* alive = A.alive[list];
+    for (uint64_t j = gtid; j < ((na + 31) & ~31ULL); j += gthreads) {
+      bool want = false;
+      uint32_t v = 0;
+      if (j < na) {
+        v = alive[j];
+        uint32_t d;
+        if (undo) {
+          d = A.snap[v];
+          A.deg[v] = d;
+          A.rem[v] = kAlive;
+        } else {
+          d = A.deg[v];
+          A.snap[v] = d;
+        }
+        if (d < k) {
+          A.rem[v] = tag;
           want = true;
         }
       }
+      push_warp(want, v, (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap, &A.words->err);
     }
-    push_warp(want, w, next, ncnt, A.cap, &A.words->err);
-  }
-}
-
-// drop_neighbours for up to 256 entries [b, e): each lane loads its 8
-// entries, their alive flags, then decrements their degrees, before it uses
-// any result, so 8 loads and 8 atomics of each lane are in flight at once
-// (the big rows' windows in a probe).
-__device__ __forceinline__ void drop_neighbours_wide(const ProbeArgs& A, uint64_t b, uint64_t e, uint32_t* next,
-                                                     unsigned long long* ncnt) {
-  constexpr unsigned kPer = 8;
-  const uint64_t j0 = b + lane_id();
-  uint32_t w[kPer];
-#pragma unroll
-  for (unsigned k = 0; k < kPer; ++k) w[k] = j0 + 32 * k < e ? A.adj[j0 + 32 * k] : 0u;
-  bool live[kPer];
-#pragma unroll
-  for (unsigned k = 0; k < kPer; ++k) live[k] = j0 + 32 * k < e && A.rem[w[k]] == kAlive;
-  uint32_t old[kPer];
-#pragma unroll
-  for (unsigned k = 0; k < kPer; ++k) old[k] = live[k] ? atomicSub(&A.deg[w[k]], 1u) : 0u;
-#pragma unroll
-  for (unsigned k = 0; k < kPer; ++k) {
-    const bool want = live[k] && old[k] == A.k;
-    if (want) A.rem[w[k]] = A.tag;
-    push_warp(want, w[k], next, ncnt, A.cap, &A.words->err);
-  }
-}
-
-// A whole probe (frontier init and every round) in one cooperative launch.
-__global__ void __launch_bounds__(256, 4) k_probe(ProbeArgs A) {
-  __shared__ uint64_t woff[kBigBatch + 1];
-  __shared__ uint64_t wtmp[33];
-  const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t gwarps = gthreads >> 5, gwarp = gtid >> 5;
-  for (uint64_t i = gtid; i < ((A.n_alive + 31) & ~31ULL); i += gthreads) {
-    bool want = false;
-    uint32_t v = 0;
-    if (i < A.n_alive) {
-      v = A.alive[i];
-      if (A.rem[v] == kAlive && A.deg[v] < A.k) {
-        A.rem[v] = A.tag;
-        want = true;
+    undo = false;
+    ++i;
+    src[0] = &A.cnt[i % 3];
+    src[1] = nullptr;
+    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+    uint64_t removed = 0;
+    bool empty = false;
+    while (true) {
+      const uint64_t nf = sh[0];
+      if (nf == 0) break;
+      removed += nf;
+      // Every block reads the same counts, so all of them stop together: fewer
+      // than k+1 vertices can remain, so the k-core is empty.
+      if (!A.fixed && na - removed < (uint64_t)k + 1) {
+        empty = true;
+        break;
       }
+      const uint32_t* fr = A.front[i & 1];
+      uint32_t* nx = A.front[(i + 1) & 1];
+      unsigned long long* nc = &A.cnt[(i + 1) % 3];
+      unsigned long long* bc = &A.cnt[3 + (i & 1)];
+      walk_rows(fr, nf, A.off, A.adj, A.big_row, A.big, bc, A.cap, &A.words->err,
+                [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) {
+                  drop_entries<kWide>(A, w, ok, k, tag, nx, nc);
+                });
+      if (gtid == 0) {
+        A.cnt[(i + 2) % 3] = 0;        // read at the start of round i-1
+        A.cnt[3 + ((i + 1) & 1)] = 0;  // big count of round i-1, read before the barrier ending it
+      }
+      // sh[0]: the next frontier's size so far (final when there are no big
+      // rows, whose windows add to it); sh[1]: this round's big rows.
+      src[0] = nc;
+      src[1] = bc;
+      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+      const uint64_t nbig = sh[1];
+      if (nbig) {
+        deal_windows<256>(
+            nbig, [&](uint64_t x) { return A.big[x]; }, A.off, woff, wtmp, [&](uint64_t, uint64_t b, uint64_t e) {
+              uint32_t w[8];
+              bool ok[8];
+#pragma unroll
+              for (unsigned t = 0; t < 8; ++t) {
+                const uint64_t j = b + lane_id() + 32 * t;
+                ok[t] = j < e;
+                w[t] = ok[t] ? A.adj[j] : 0u;
+              }
+              drop_entries<8>(A, w, ok, k, tag, nx, nc);
+            });
+        if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+      }
+      ++i;
+      ++rounds;
     }
-    push_warp(want, v, A.front[0], &A.cnt[0], A.cap, &A.words->err);
-  }
-  __shared__ unsigned long long sh[2];
-  const unsigned long long* src[2] = {&A.cnt[0], nullptr};
-  if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
-  uint32_t i = 0;
-  uint64_t removed = 0;
-  bool stopped = false;
-  while (true) {
-    const uint64_t nf = sh[0];
-    if (nf == 0) break;
-    removed += nf;
-    // Every block reads the same counts, so all of them stop together.
-    if (A.may_stop && A.n_alive - removed < (uint64_t)A.k + 1) {
-      stopped = true;
+    const uint64_t left = empty ? 0 : na - removed;
+    if (gtid == 0) {
+      A.out->k[probes] = k;
+      A.out->left[probes] = (uint32_t)left;
+    }
+    ++probes;
+    if (!left) {
+      if (A.fixed) {
+        na = 0;
+        break;
+      }
+      hi = k;
+      ramp = 0;
+      undo = true;
+      continue;
+    }
+    ++tag;
+    // Ordered compaction: block b owns [b, b + 1) * stretch of the list.
+    const uint64_t stretch = (na + gridDim.x - 1) / gridDim.x;
+    const uint64_t s0 = min(na, blockIdx.x * stretch), s1 = min(na, s0 + stretch);
+    uint64_t n = 0, sum = 0;
+    uint32_t mn = 0xffffffffu;
+    for (uint64_t j = s0 + threadIdx.x; j < s1; j += blockDim.x) {
+      const uint32_t v = alive[j];
+      if (A.rem[v] != kAlive) continue;
+      const uint32_t d = A.deg[v];
+      ++n;
+      sum += d;
+      mn = min(mn, d);
+    }
+    n = block_sum<uint64_t>(n, wtmp);
+    mn = warp_min(mn);
+    sum = warp_sum(sum);
+    if (lane_id() == 0 && mn != 0xffffffffu) {
+      atomicMin(&A.cnt[5], (unsigned long long)mn);
+      atomicAdd(&A.cnt[6], (unsigned long long)sum);
+    }
+    if (threadIdx.x == 0) kept[blockIdx.x] = n;
+    src[0] = &A.cnt[5];
+    src[1] = &A.cnt[6];
+    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+    const uint64_t dmin = sh[0], dsum = sh[1];
+    uint64_t at = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += blockDim.x) at += ld_relaxed_u64(&kept[b]);
+    at = block_sum<uint64_t>(at, wtmp);
+    uint32_t* to = A.alive[list ^ 1];
+    for (uint64_t j0 = s0; j0 < s1; j0 += blockDim.x) {
+      const uint64_t j = j0 + threadIdx.x;
+      const uint32_t v = j < s1 ? alive[j] : 0u;
+      const bool keep = j < s1 && A.rem[v] == kAlive;
+      uint64_t total;
+      const uint64_t p = at + block_excl_scan<uint64_t>(keep ? 1 : 0, wtmp, &total);
+      if (keep) to[p] = v;
+      at += total;
+    }
+    list ^= 1;
+    na = left;
+    // The k-core left is the core of its least degree too, so every level up
+    // to that is known to be non-empty.
+    lo = k;
+    if (dmin > lo) lo = dmin < hi - 1 ? (uint32_t)dmin : hi - 1;
+    if (A.fixed) break;
+    if (dsum < A.compact_below) {
+      compact = 1;
       break;
     }
-    const uint32_t* fr = A.front[i & 1];
-    uint32_t* nx = A.front[(i + 1) & 1];
-    unsigned long long* nc = &A.cnt[(i + 1) % 3];
-    unsigned long long* bc = &A.cnt[3 + (i & 1)];
-    for (uint64_t f = gwarp; f < nf; f += gwarps) {
-      const uint32_t v = fr[f];
-      const uint64_t b = A.off[v], e = A.off[v + 1];
-      if (e - b > A.big_row) {
-        if (lane_id() == 0) {
-          const unsigned long long p = atomicAdd(bc, 1ULL);
-          if (p < A.cap)
-            A.big[p] = v;
-          else
-            atomicOr(&A.words->err, kDevErrCapacity);
-        }
-        continue;
-      }
-      drop_neighbours(A, b, e, nx, nc);
+    if (!grid_barrier(A.words, A.timeout_ns)) return;
+  }
+  if (undo) {  // the last probe failed
+    const uint32_t* alive = A.alive[list];
+    for (uint64_t j = gtid; j < na; j += gthreads) {
+      const uint32_t v = alive[j];
+      A.deg[v] = A.snap[v];
+      A.rem[v] = kAlive;
     }
-    if (gtid == 0) {
-      A.cnt[(i + 2) % 3] = 0;        // read at the start of round i-1
-      A.cnt[3 + ((i + 1) & 1)] = 0;  // big count of round i-1, read before the barrier ending it
-    }
-    // sh[0]: the next frontier's size so far (final when there are no big
-    // rows, whose windows add to it); sh[1]: this round's big rows.
-    src[0] = nc;
-    src[1] = bc;
-    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
-    const uint64_t nbig = sh[1];
-    if (nbig) {
-      // Rows longer than big_row: their 256-entry windows dealt to every warp.
-      deal_windows<256>(
-          nbig, [&](uint64_t x) { return A.big[x]; }, A.off, woff, wtmp,
-          [&](uint64_t, uint64_t b, uint64_t e) { drop_neighbours_wide(A, b, e, nx, nc); });
-      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
-    }
-    ++i;
   }
   if (gtid == 0) {
-    A.cnt[5] = i;
-    A.cnt[6] = removed;
-    A.cnt[7] = stopped;
+    SearchOut* o = A.out;
+    o->n_alive = na;
+    o->rounds = rounds;
+    o->lo = lo;
+    o->hi = hi;
+    o->ramp = ramp;
+    o->list = list;
+    o->probes = probes;
+    o->compact = compact;
   }
 }
 
@@ -407,7 +582,7 @@ __global__ void __launch_bounds__(256, 4) k_probe(ProbeArgs A) {
 //
 // Level k removes every alive vertex of degree <= k (core number k): a pass
 // over a vertex list takes the vertices of degree <= k as the first frontier,
-// and the frontier rounds then run as in k_probe (a neighbour stepping from
+// and the frontier rounds then run as in k_core_search (a neighbour stepping from
 // k+1 to k joins the next frontier).  Passes are windowed: a full pass over
 // the compact alive list opens a window of `window` levels [k, top] and
 // lists the candidates, the alive vertices of degree <= top; within the
@@ -446,25 +621,25 @@ struct DropRule {
   unsigned long long* ccnt;
 };
 
-__device__ __forceinline__ void drop_neighbours_core(const DecompArgs& A, uint64_t b, uint64_t e, const DropRule& R) {
-  for (uint64_t j = b + lane_id(); j < b + ((e - b + 31) & ~31ULL); j += 32) {
-    bool want = false, join = false;
-    uint32_t w = 0;
-    if (j < e) {
-      w = A.adj[j];
-      if (A.rem[w] == kAlive) {
-        const uint32_t old = atomicSub(&A.deg[w], 1u);
-        if (old == R.k + 1) {
-          A.rem[w] = 0u;
-          A.core[w] = R.k;
-          want = true;
-        } else if (old == R.top + 1) {
-          join = true;  // its degree entered the window
-        }
-      }
+template <unsigned N>
+__device__ __forceinline__ void drop_entries_core(const DecompArgs& A, const uint32_t (&w)[N], const bool (&ok)[N],
+                                                  const DropRule& R) {
+  bool live[N];
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) live[t] = ok[t] && A.rem[w[t]] == kAlive;
+  uint32_t old[N];
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) old[t] = live[t] ? atomicSub(&A.deg[w[t]], 1u) : 0u;
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) {
+    const bool want = live[t] && old[t] == R.k + 1;
+    const bool join = live[t] && !want && old[t] == R.top + 1;  // its degree entered the window
+    if (want) {
+      A.rem[w[t]] = 0u;
+      A.core[w[t]] = R.k;
     }
-    push_warp(want, w, R.next, R.ncnt, A.cap, &A.words->err);
-    push_warp(join, w, R.cand, R.ccnt, A.cap, &A.words->err);
+    push_warp(want, w[t], R.next, R.ncnt, A.cap, &A.words->err);
+    push_warp(join, w[t], R.cand, R.ccnt, A.cap, &A.words->err);
   }
 }
 
@@ -474,7 +649,6 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
   __shared__ uint64_t wtmp[33];
   const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t gwarps = gthreads >> 5, gwarp = gtid >> 5;
   uint64_t nl = A.n_list;  // entries of the current alive list
   uint64_t nc = 0;         // entries of the current candidate list
   uint32_t k = 1;          // every alive vertex has degree >= k
@@ -569,21 +743,8 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
       R.next = (i & 1) ? A.front[0] : A.front[1];
       R.ncnt = &A.cnt[(i + 1) % 3];
       unsigned long long* bc = &A.cnt[3 + (i & 1)];
-      for (uint64_t f = gwarp; f < nf; f += gwarps) {
-        const uint32_t v = fr[f];
-        const uint64_t b = A.off[v], e = A.off[v + 1];
-        if (e - b > A.big_row) {
-          if (lane_id() == 0) {
-            const unsigned long long p = atomicAdd(bc, 1ULL);
-            if (p < A.cap)
-              A.big[p] = v;
-            else
-              atomicOr(&A.words->err, kDevErrCapacity);
-          }
-          continue;
-        }
-        drop_neighbours_core(A, b, e, R);
-      }
+      walk_rows(fr, nf, A.off, A.adj, A.big_row, A.big, bc, A.cap, &A.words->err,
+                [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) { drop_entries_core<kWide>(A, w, ok, R); });
       if (gtid == 0) {
         A.cnt[(i + 2) % 3] = 0;
         A.cnt[3 + ((i + 1) & 1)] = 0;
@@ -592,9 +753,18 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
       if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       const uint64_t nbig = sh[1];
       if (nbig) {
-        deal_windows<32>(
-            nbig, [&](uint64_t x) { return A.big[x]; }, A.off, woff, wtmp,
-            [&](uint64_t, uint64_t b, uint64_t e) { drop_neighbours_core(A, b, e, R); });
+        deal_windows<128>(
+            nbig, [&](uint64_t x) { return A.big[x]; }, A.off, woff, wtmp, [&](uint64_t, uint64_t b, uint64_t e) {
+              uint32_t w[4];
+              bool ok[4];
+#pragma unroll
+              for (unsigned t = 0; t < 4; ++t) {
+                const uint64_t j = b + lane_id() + 32 * t;
+                ok[t] = j < e;
+                w[t] = ok[t] ? A.adj[j] : 0u;
+              }
+              drop_entries_core<4>(A, w, ok, R);
+            });
         if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       }
       nf = sh[0];
@@ -615,8 +785,17 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
   }
 }
 
+// Blocks of a cooperative launch here at most (one count per block is kept).
+constexpr unsigned kMaxGrid = 4096;
+// Graphs with fewer edges (32 MB of adjacency) are searched without compaction:
+// the copy cost more than the probes it sped up (R-MAT scale 18, 3.4M edges:
+// membership of one core 1.26 ms with copies, 1.09 ms without; a 49M-edge
+// Chung-Lu solve 21.8 ms with, 22.3 ms without).
+constexpr uint64_t kCompactMinEdges = 1u << 22;
+
 uint32_t big_row(const Ctx* c) {
-  return (uint32_t)std::min<int64_t>(std::max<int64_t>(32, c->opt.kcore_big_row), 1 << 30);
+  // At most 2^26: a warp adds up the lengths of 32 rows in 32 bits.
+  return (uint32_t)std::min<int64_t>(std::max<int64_t>(32, c->opt.kcore_big_row), 1 << 26);
 }
 
 }  // namespace
@@ -629,7 +808,7 @@ void KCore::reset_state(Ctx* c, const Graph& gr) {
   front[0].ensure(c, (n ? n : 1) * sizeof(uint32_t));
   front[1].ensure(c, (n ? n : 1) * sizeof(uint32_t));
   big.ensure(c, (n ? n : 1) * sizeof(uint32_t));
-  cnt.ensure(c, 8 * sizeof(unsigned long long));
+  cnt.ensure(c, (7 + kMaxGrid) * sizeof(unsigned long long));
   if (n) {
     k_init_state<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(gr.deg.as<uint32_t>(), n,
                                                                              deg.as<uint32_t>(), rem.as<uint32_t>());
@@ -712,51 +891,85 @@ void KCore::recount(Ctx* c) {
   KT_LAUNCHED(c);
 }
 
+// One launch of k_core_search from the current alive set: the search of
+// (lo, hi), or with fixed one probe at level lo.  Successful probes get their
+// tags, and the alive list and n_alive are the last one's.
+void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixed, uint64_t compact_below,
+                          void* result) {
+  const Graph& g = cur();
+  snap.ensure(c, (n ? n : 1) * sizeof(uint32_t));
+  alive2.ensure(c, (n ? n : 1) * sizeof(uint32_t));
+  out.ensure(c, sizeof(SearchOut));
+  if (!coop_grid) {
+    int per_sm = 0;
+    KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_search, 256, 0));
+    coop_grid = std::min(coop_blocks(c, per_sm), kMaxGrid);
+  }
+  SearchArgs A;
+  A.off = g.off.as<uint64_t>();
+  A.adj = g.adj.as<uint32_t>();
+  A.deg = deg.as<uint32_t>();
+  A.rem = rem.as<uint32_t>();
+  A.snap = snap.as<uint32_t>();
+  A.alive[0] = alive.as<uint32_t>();
+  A.alive[1] = alive2.as<uint32_t>();
+  A.n_alive = n_alive;
+  A.front[0] = front[0].as<uint32_t>();
+  A.front[1] = front[1].as<uint32_t>();
+  A.big = big.as<uint32_t>();
+  A.cnt = cnt.as<unsigned long long>();
+  A.cap = n;
+  A.lo = lo;
+  A.hi = hi;
+  A.ramp = ramp;
+  A.fixed = fixed;
+  A.tag = (uint32_t)levels.size();
+  A.compact_below = compact_below;
+  A.big_row = big_row(c);
+  A.out = out.as<SearchOut>();
+  A.words = dev_words(c);
+  A.timeout_ns = (unsigned long long)c->opt.timeout_ms * 1000000ULL;
+  if (A.tag >= 0xfffffff0u - kMaxProbes) throw Error(KT_ERR_LIMIT, "k-core: too many probes");
+  zero(c, cnt.get(), 7 * sizeof(unsigned long long));
+  void* p[] = {&A};
+  SearchOut& h = *static_cast<SearchOut*>(result);
+  {
+    CoopLock coop(c);
+    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_search, dim3(coop_grid), dim3(256), p, 0, c->stream));
+    KT_LAUNCHED(c);
+    read_checked(c, &h, out.get(), sizeof(SearchOut), "k-core probe");
+  }
+  rounds += h.rounds;
+  probes += h.probes;
+  n_alive = h.n_alive;
+  if (h.list) std::swap(alive, alive2);
+  for (uint32_t i = 0; i < h.probes; ++i) {
+    KT_LOG(c, "kt: k-core probe %u: %u vertices left\n", h.k[i], h.left[i]);
+    if (!h.left[i] && !fixed) continue;
+    if (!fixed) succ.push_back((uint32_t)levels.size());
+    levels.push_back(h.k[i]);
+  }
+}
+
 uint64_t KCore::probe(Ctx* c, uint32_t k, bool may_stop) {
+  if (!n_alive) {
+    levels.push_back(k);
+    return 0;
+  }
+  if (c->opt.persistent) {
+    SearchOut h;
+    search_launch(c, k, k + 1, false, true, 0, &h);
+    return n_alive;
+  }
   const uint32_t tag = (uint32_t)levels.size();
   if (tag >= 0xfffffff0u) throw Error(KT_ERR_LIMIT, "k-core: too many probes");
   levels.push_back(k);
-  if (!n_alive) return 0;
   const Graph& g = cur();
   unsigned long long* cn = cnt.as<unsigned long long>();
-  zero(c, cnt.get(), cnt.bytes());
+  zero(c, cnt.get(), 7 * sizeof(unsigned long long));
   uint32_t* err = &dev_words(c)->err;
   uint64_t removed = 0;
-  if (c->opt.persistent) {
-    ProbeArgs A;
-    A.off = g.off.as<uint64_t>();
-    A.adj = g.adj.as<uint32_t>();
-    A.deg = deg.as<uint32_t>();
-    A.rem = rem.as<uint32_t>();
-    A.alive = alive.as<uint32_t>();
-    A.n_alive = n_alive;
-    A.front[0] = front[0].as<uint32_t>();
-    A.front[1] = front[1].as<uint32_t>();
-    A.big = big.as<uint32_t>();
-    A.cnt = cn;
-    A.cap = n;
-    A.k = k;
-    A.tag = tag;
-    A.may_stop = may_stop;
-    A.big_row = big_row(c);
-    A.words = dev_words(c);
-    A.timeout_ns = (unsigned long long)c->opt.timeout_ms * 1000000ULL;
-    if (!coop_grid) {
-      int per_sm = 0;
-      KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_probe, 256, 0));
-      coop_grid = coop_blocks(c, per_sm);
-    }
-    void* p[] = {&A};
-    uint64_t h[3];
-    {
-      CoopLock coop(c);
-      KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_probe, dim3(coop_grid), dim3(256), p, 0, c->stream));
-      KT_LAUNCHED(c);
-      copy_d2h(c, h, cn + 5, 24);
-    }
-    rounds += h[0];
-    removed = h[2] ? n_alive : h[1];  // stopped: the k-core is empty (the state is partial)
-  } else {
+  {
     k_frontier_init<<<grid_for(n_alive, 256, c->num_sms * 16), 256, 0, c->stream>>>(
         alive.as<uint32_t>(), n_alive, deg.as<uint32_t>(), rem.as<uint32_t>(), k, tag, front[0].as<uint32_t>(),
         cn + 0, n, err);
@@ -788,7 +1001,9 @@ uint64_t KCore::probe(Ctx* c, uint32_t k, bool may_stop) {
   }
   ++probes;
   check_words(c, "k-core probe");
-  return n_alive - removed;
+  const uint64_t left = n_alive - removed;
+  if (left) rebuild_alive(c);
+  return left;
 }
 
 uint32_t KCore::find_max_core(Ctx* c) {
@@ -802,6 +1017,32 @@ uint32_t KCore::find_max_core(Ctx* c) {
   ub = std::min<uint64_t>(ub, base->max_deg);
   uint64_t lo = 1, hi = ub + 1;  // the 1-core (non-isolated vertices) is non-empty
   bool ramp = true;
+  if (c->opt.persistent) {
+    while (hi - lo > 1) {
+      // Work on a compacted copy once the core's edges are a small part of
+      // the current graph's: a copy that keeps most of them costs more than
+      // the probes it would speed up.  (The copy holds the k-core, which
+      // every level from k up can be restored from.)  A graph below
+      // kCompactMinEdges stays as it is: it is read from L2 either way.
+      const uint64_t m2 = 2 * cur().m;
+      const uint64_t below = c->opt.kcore_compact > 0 && cur().m >= kCompactMinEdges
+                                 ? (m2 + c->opt.kcore_compact - 1) / (uint64_t)c->opt.kcore_compact
+                                 : 0;
+      SearchOut h;
+      search_launch(c, (uint32_t)lo, (uint32_t)hi, ramp, false, below, &h);
+      lo = h.lo;
+      hi = h.hi;
+      ramp = h.ramp;
+      if (h.compact) {
+        const uint32_t k = h.k[h.probes - 1];
+        compact_to_alive(c, k);
+        KT_LOG(c, "kt: k-core compacted copy of the %u-core: %llu vertices, %llu edges\n", k,
+               (unsigned long long)n, (unsigned long long)local.m);
+      }
+    }
+    cmax = (uint32_t)lo;
+    return cmax;
+  }
   DBuf mn(c, 16), snap;
   while (hi - lo > 1) {
     uint64_t k = ramp ? std::min<uint64_t>(lo * 2, hi - 1) : lo + (hi - lo) / 2;
@@ -820,7 +1061,6 @@ uint32_t KCore::find_max_core(Ctx* c) {
     if (left) {
       lo = k;
       succ.push_back(tag);
-      rebuild_alive(c);
       // The probe left the k-core; its minimum degree d >= k makes it the
       // d-core too, so every level up to d is known to be non-empty.
       // mn: [0] the minimum alive degree, [2..3] the sum of alive degrees.
@@ -900,7 +1140,6 @@ void KCore::restore_core(Ctx* c, uint32_t k) {
   recount(c);
   const uint32_t tag = (uint32_t)levels.size();
   if (probe(c, k)) succ.push_back(tag);
-  rebuild_alive(c);
 }
 
 void KCore::members(Ctx* c, uint8_t* dout) {
@@ -933,8 +1172,7 @@ void KCore::core_numbers(Ctx* c, uint32_t* dcore) {
         alive.as<uint32_t>(), n_alive, deg.as<uint32_t>(), rem.as<uint32_t>(), mn.as<uint32_t>());
     KT_LAUNCHED(c);
     const uint32_t d = read_word<uint32_t>(c, mn.as<uint32_t>());
-    probe(c, d + 1);
-    rebuild_alive(c);
+    n_alive = probe(c, d + 1);
   }
   DBuf lv(c, levels.size() * sizeof(uint32_t));
   copy_h2d(c, lv.get(), levels.data(), levels.size() * sizeof(uint32_t));

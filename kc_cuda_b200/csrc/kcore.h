@@ -16,6 +16,9 @@ struct KCore {
   DBuf deg;        // uint32[n]: alive degree of alive vertices
   DBuf rem;        // uint32[n]: kAlive, or the tag of the probe that removed it
   DBuf alive;      // uint32[n]: compact list of alive vertices (ascending)
+  DBuf alive2;     // the list the search writes next
+  DBuf snap;       // uint32[n]: degrees before a probe of the search
+  DBuf out;        // the search's result
   DBuf front[2];   // frontiers
   DBuf big;        // rows handled by whole blocks
   DBuf cnt;        // counters
@@ -42,9 +45,10 @@ struct KCore {
   void init(Ctx* c, const Graph& gr);
   void rebuild_alive(Ctx* c);
   void recount(Ctx* c);
-  // Peels the alive set to its k-core; returns the vertices left.  may_stop:
-  // the peel may stop once fewer than k+1 vertices can remain, returning 0
-  // with the state partial (the caller then undoes the probe).
+  // Peels the alive set to its k-core and makes the alive list its vertices;
+  // returns how many.  may_stop (host-stepped rounds): the peel may stop once
+  // fewer than k+1 vertices can remain, returning 0 with the state partial
+  // (the caller then undoes the probe).
   uint64_t probe(Ctx* c, uint32_t k, bool may_stop = false);
   // Leaves the alive set at the maximum core; returns its k.
   uint32_t find_max_core(Ctx* c);
@@ -58,6 +62,7 @@ struct KCore {
   void core_numbers_persistent(Ctx* c, uint32_t* dcore);
 
  private:
+  void search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixed, uint64_t compact_below, void* result);
   void reset_state(Ctx* c, const Graph& gr);
   void compact_to_alive(Ctx* c, uint32_t level);
 };

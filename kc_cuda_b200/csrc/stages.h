@@ -37,5 +37,8 @@ DevWords* dev_words(Ctx* c);
 void reset_words(Ctx* c);
 // Throws the error a kernel flagged in the device words (if any).
 void check_words(Ctx* c, const char* stage);
+// Reads a kernel's result (at most 3072 bytes) and the device words in one
+// wait, and throws as check_words does.
+void read_checked(Ctx* c, void* dst, const void* src, size_t bytes, const char* stage);
 
 }  // namespace kt
