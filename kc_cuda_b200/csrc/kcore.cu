@@ -272,9 +272,9 @@ __global__ void k_members_mapped(const uint32_t* __restrict__ rem, uint64_t n, c
 constexpr unsigned kWide = 4;
 
 template <class Drop>
-__device__ __forceinline__ void walk_rows(const uint32_t* __restrict__ front, uint64_t nf,
+__device__ __forceinline__ void walk_rows(const uint32_t* front, uint64_t nf,
                                           const uint64_t* __restrict__ off, const uint32_t* __restrict__ adj,
-                                          uint32_t big_row, uint32_t* __restrict__ big, unsigned long long* nbig,
+                                          uint32_t big_row, uint32_t* big, unsigned long long* nbig,
                                           uint64_t cap, uint32_t* err, Drop drop) {
   const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();

@@ -311,6 +311,25 @@ __global__ void __launch_bounds__(256, 4) k_dense_support(uint64_t m, const uint
   if (lane_id() == 0 && wr) atomicAdd(row_words, wr);
 }
 
+// Exact counts over rows of at most kShortRow words, from 8-entry groups (a
+// warp works on eight edges at once).
+__global__ void __launch_bounds__(256) k_dense_support_short(uint64_t m, const uint32_t* __restrict__ order,
+                                                             const uint64_t* __restrict__ ends, DenseRows R,
+                                                             uint32_t* __restrict__ sup,
+                                                             unsigned long long* __restrict__ row_words) {
+  const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint32_t size = m / warps >= 32 ? 32u : 8u;
+  unsigned long long wr = 0;
+  for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * size < m; g += warps) {
+    uint32_t e, s;
+    bool ok;
+    dense_group_short(order, g * size, min(m, (g + 1) * size), ends, R, nullptr, e, s, ok, &wr);
+    if (ok) sup[e] = s;
+  }
+  wr = warp_sum(wr);
+  if (lane_id() == 0 && wr) atomicAdd(row_words, wr);
+}
+
 // Capped counts (search phase): threshold `cap`, or gcap[vgid[u]] per graph
 // of a grouped union.
 __global__ void __launch_bounds__(256) k_dense_support_capped(uint64_t m, const uint32_t* __restrict__ order,
@@ -370,7 +389,11 @@ void launch_exact(Ctx* c, const Sub& s, uint32_t* sup, unsigned long long* row_w
 // side, one per half of the warp.
 void launch_dense_support(Ctx* c, const Sub& s, uint32_t* sup, bool capped, uint32_t cap, const uint32_t* gcap,
                           unsigned long long* row_words, unsigned long long* cursor) {
-  if (capped) {
+  if (s.W <= kShortRow) {  // (exact also where a cap is given: there is little to abandon)
+    k_dense_support_short<<<grid_for((s.m + 7) / 8 * 32, 256, c->num_sms * 8), 256, 0, c->stream>>>(
+        s.m, s.order.as<uint32_t>(), s.ends.as<uint64_t>(), dense_rows(s), sup, row_words);
+    KT_LAUNCHED(c);
+  } else if (capped) {
     const size_t smem = dense_smem_bytes(s.W, 256);
     const unsigned grid = dense_grid(c, (const void*)k_dense_support_capped, s, smem);
     k_dense_support_capped<<<grid, 256, smem, c->stream>>>(s.m, s.order.as<uint32_t>(), s.ends.as<uint64_t>(),
