@@ -7,8 +7,11 @@
 // recorded level when no edge is left is kmax.
 //
 // Rounds: the frontier edges of round r carry state r; deleted edges keep
-// their round, alive edges kAlive.  A warp takes a frontier edge (x, y) and
-// intersects the two sorted rows: 32-wide tiles of both rows are compared
+// their round, alive edges kAlive.  Without bitsets, the entries w of the
+// shorter row of a frontier edge (x, y) are looked up as edges to its other
+// end in a hash table of the edges (list_round).  With bitsets, a warp takes a
+// frontier edge and ANDs the two rows, or where the sorted rows are shorter
+// (and in list mode without a table) merges them: 32-wide tiles of both rows are compared
 // with a 5-step shuffle search, and whichever tile ends lower is retired
 // (both when the ends tie), so every common neighbour is met exactly once;
 // when one row is more than peel_search_ratio (16) times longer the lanes
@@ -39,6 +42,7 @@
 
 #include "compact.cuh"
 #include "dense.cuh"
+#include "rows.cuh"
 #include "subgraph.h"
 
 namespace kt {
@@ -59,7 +63,8 @@ struct PeelArgs {
   const uint32_t* alive;
   uint64_t na;
   uint32_t* front[2];
-  // [0..2] rotating frontier counters, [6..7] recount cursors, [8..10] and
+  // [0..2] rotating frontier counters, [3..4] long rows of a list-mode round,
+  // [6..7] recount cursors, [8..10] and
   // [12..14] a level's figures (k_levels, by level parity: 2^32 - 1 - the least
   // support left, the largest, the edges left), [16...] one kept count per block
   unsigned long long* cnt;
@@ -82,6 +87,11 @@ struct PeelArgs {
   const uint32_t* gthr;
   const uint32_t* egr;
   const uint32_t* gthr_max;  // batched: the largest running threshold (recount cost model)
+  // List mode: the edges in a hash table (null: none), tag << 32 | edge id per
+  // slot, and the frontier edges whose shorter row is long.
+  const unsigned long long* table;
+  uint32_t table_bits;  // 2^table_bits slots
+  uint32_t* big;
   // A level tried from a snapshot: give up (the level's truss is empty) as
   // soon as fewer than this many edges can remain, t(t-1)/2 for level t
   // (0: peel to the end).  The state is then partial; the caller undoes it.
@@ -251,6 +261,172 @@ __device__ __forceinline__ void peel_edge(const PeelArgs& A, const Level& V, uin
     if (alast <= blast) i += ta;
     if (blast <= alast) j += tb;
   }
+  tdec += ndec;
+}
+
+// ---- list mode: triangles of a frontier edge through an edge hash table.
+
+__device__ __forceinline__ uint32_t edge_hash(uint32_t u, uint32_t v) {
+  uint32_t h = (u * 0x9E3779B1u) ^ __funnelshift_l(v * 0x85EBCA77u, v * 0x85EBCA77u, 15);
+  h ^= h >> 15;
+  return h * 0xC2B2AE3Du;
+}
+__device__ __forceinline__ uint32_t edge_tag(uint32_t u, uint32_t v) { return (u * 0x27D4EB2Fu) ^ (v + (v << 13)); }
+constexpr unsigned long long kNoEdge = ~0ULL;
+
+__global__ void k_table_build(uint64_t m, const uint64_t* __restrict__ ends, unsigned long long* table,
+                              uint32_t bits) {
+  const uint64_t mask = (1ULL << bits) - 1;
+  for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = ends[e];
+    const uint32_t u = (uint32_t)(k >> 32), v = (uint32_t)k;
+    const unsigned long long ent = ((unsigned long long)edge_tag(u, v) << 32) | (uint32_t)e;
+    uint64_t at = edge_hash(u, v) >> (32 - bits);
+    while (atomicCAS(&table[at], kNoEdge, ent) != kNoEdge) at = (at + 1) & mask;  // at most 2/5 of the slots fill
+  }
+}
+
+// Id of the edge (a, b), or 0xffffffff.
+__device__ __forceinline__ uint32_t find_edge(const PeelArgs& A, uint32_t a, uint32_t b) {
+  const uint32_t u = min(a, b), v = max(a, b), tag = edge_tag(u, v);
+  const uint64_t key = ((uint64_t)u << 32) | v, mask = (1ULL << A.table_bits) - 1;
+  for (uint64_t at = edge_hash(u, v) >> (32 - A.table_bits);; at = (at + 1) & mask) {
+    const unsigned long long ent = A.table[at];
+    if (ent == kNoEdge) return 0xffffffffu;
+    if ((uint32_t)(ent >> 32) == tag && A.ends[(uint32_t)ent] == key) return (uint32_t)ent;
+  }
+}
+
+// The end of edge (x, y) with the shorter row.
+__device__ __forceinline__ void shorter_row(const PeelArgs& A, uint32_t e, uint32_t& s, uint32_t& other) {
+  const uint64_t k = A.ends[e];
+  s = (uint32_t)(k >> 32);
+  other = (uint32_t)k;
+  if (A.off[s + 1] - A.off[s] > A.off[other + 1] - A.off[other]) {
+    const uint32_t t = s;
+    s = other;
+    other = t;
+  }
+}
+
+// N row entries per lane (row positions j[t], where ok[t]) of the shorter rows
+// of frontier edges e[t], whose other ends are o[t].
+template <unsigned N>
+__device__ __forceinline__ void close_entries(const PeelArgs& A, const Level& V, const uint32_t (&e)[N],
+                                              const uint32_t (&o)[N], const uint64_t (&j)[N], const bool (&ok)[N],
+                                              uint32_t r, uint32_t* next, unsigned long long* ncnt, uint32_t& ndec) {
+  uint32_t a[N], w[N], b[N];
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) {
+    a[t] = ok[t] ? A.eid[j[t]] : 0u;
+    w[t] = ok[t] ? A.adj[j[t]] : 0u;
+  }
+  bool live[N];
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) live[t] = ok[t] && a[t] != e[t] && A.state[a[t]] >= r;
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) b[t] = live[t] ? find_edge(A, o[t], w[t]) : 0xffffffffu;
+#pragma unroll
+  for (unsigned t = 0; t < N; ++t) {
+    bool pa = false, pb = false;
+    if (b[t] != 0xffffffffu) close_triangle(A, V, e[t], a[t], b[t], r, edge_thr(A, V, e[t]), pa, pb, ndec);
+    __syncwarp();
+    push_warp_full(pa, a[t], next, ncnt, A.cap, &A.words->err);
+    push_warp_full(pb, b[t], next, ncnt, A.cap, &A.words->err);
+  }
+}
+
+// A round over the frontier's shorter rows: a warp takes up to 32 edges (fewer
+// when the frontier is small for the grid) and walks their rows end to end;
+// rows of more than kLongJob entries go to A.big[0..*nbig), whose windows are
+// dealt to every warp after a barrier.  An entry costs its edge's state and,
+// if that is alive, one table slot or two, all independent of its neighbours';
+// the merge of the two sorted rows by one warp was a chain of as many dependent
+// steps as the rows have tiles of 32 entries (truss numbers of an R-MAT scale 16
+// graph, 850,000 edges, 828 rounds: levels 52.2 -> 15.9 ms).
+constexpr uint32_t kLongJob = 256;
+constexpr unsigned kJobWide = 2;
+
+__device__ __forceinline__ void list_round(const PeelArgs& A, const Level& V, const uint32_t* fr, uint64_t nf,
+                                           uint32_t r, uint32_t* next, unsigned long long* ncnt,
+                                           unsigned long long* nbig, uint64_t& tdeg, uint64_t& tdec) {
+  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
+  const unsigned lane = lane_id();
+  const uint64_t share = (nf + gwarps - 1) / gwarps;
+  const uint32_t per = share < 32 ? (uint32_t)share : 32u;
+  uint32_t ndec = 0;
+  for (uint64_t f0 = gwarp * per; f0 < nf; f0 += gwarps * per) {
+    uint64_t start = 0;
+    uint32_t len = 0, e = 0, o = 0;
+    bool is_long = false;
+    if (lane < per && f0 + lane < nf) {
+      e = fr[f0 + lane];
+      uint32_t s;
+      shorter_row(A, e, s, o);
+      tdeg += (uint64_t)atomicSub(&A.adeg[s], 1u) + atomicSub(&A.adeg[o], 1u);
+      start = A.off[s];
+      const uint64_t l = A.off[s + 1] - start;
+      is_long = l > kLongJob;
+      len = is_long ? 0u : (uint32_t)l;
+    }
+    push_warp_full(is_long, e, A.big, nbig, A.cap, &A.words->err);
+    const uint32_t incl = warp_incl_scan(len);
+    const uint32_t total = __shfl_sync(kFull, incl, 31), excl = incl - len;
+    start -= excl;  // entry p of the walk is at start + p of its row's lane
+    for (uint32_t base = 0; base < total; base += 32 * kJobWide) {
+      uint32_t ee[kJobWide], oo[kJobWide];
+      uint64_t j[kJobWide];
+      bool ok[kJobWide];
+#pragma unroll
+      for (unsigned t = 0; t < kJobWide; ++t) {
+        const uint32_t p = base + 32 * t + lane;
+        uint32_t from = 0;  // the last row starting at or before p
+        if (per > 1) {
+#pragma unroll
+          for (uint32_t st = 16; st >= 1; st >>= 1) {
+            const uint32_t x = __shfl_sync(kFull, excl, from + st);
+            if (x <= p) from += st;
+          }
+        }
+        ee[t] = __shfl_sync(kFull, e, from);
+        oo[t] = __shfl_sync(kFull, o, from);
+        j[t] = __shfl_sync(kFull, start, from) + p;
+        ok[t] = p < total;
+      }
+      close_entries<kJobWide>(A, V, ee, oo, j, ok, r, next, ncnt, ndec);
+    }
+  }
+  tdec += ndec;
+}
+
+__device__ __forceinline__ void list_round_long(const PeelArgs& A, const Level& V, uint64_t nbig, uint32_t r,
+                                                uint32_t* next, unsigned long long* ncnt, uint64_t* woff,
+                                                uint64_t* tmp, uint64_t& tdec) {
+  uint32_t ndec = 0;
+  deal_windows<32 * kJobWide>(
+      nbig,
+      [&](uint64_t x) {
+        uint32_t s, o;
+        shorter_row(A, A.big[x], s, o);
+        return s;
+      },
+      A.off, woff, tmp, [&](uint64_t x, uint64_t b, uint64_t e) {
+        const uint32_t f = A.big[x];
+        uint32_t s, o;
+        shorter_row(A, f, s, o);
+        uint32_t ee[kJobWide], oo[kJobWide];
+        uint64_t j[kJobWide];
+        bool ok[kJobWide];
+#pragma unroll
+        for (unsigned t = 0; t < kJobWide; ++t) {
+          ee[t] = f;
+          oo[t] = o;
+          j[t] = b + 32 * t + lane_id();
+          ok[t] = j[t] < e;
+        }
+        close_entries<kJobWide>(A, V, ee, oo, j, ok, r, next, ncnt, ndec);
+      });
   tdec += ndec;
 }
 
@@ -519,11 +695,13 @@ __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcn
 #ifndef KT_PEEL_MIN_BLOCKS
 #define KT_PEEL_MIN_BLOCKS 4
 #endif
+template <bool kLists>
 __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(PeelArgs A, LevelsArgs L) {
   extern __shared__ __align__(16) uint32_t dense_smem[];
+  __shared__ uint64_t woff[kLists ? kBigBatch + 1 : 1];
   __shared__ unsigned long long sh[3];
   __shared__ uint64_t wtmp[33];
-  uint32_t* su = dense_smem + warp_id() * A.R.W;
+  uint32_t* su = dense_smem + warp_id() * (kLists ? 0 : A.R.W);
   const unsigned long long* src[3] = {nullptr, nullptr, nullptr};
   const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -537,9 +715,12 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(Pee
   bool gave_up = false;
   uint64_t left = V.na;  // edges alive (the list may hold dead ones too)
   while (true) {
-    // Slot (i + 1) % 3 is zero, and slot (i + 2) % 3 was read before the
-    // barrier of the last round.
-    if (gtid == 0) A.cnt[(i + 2) % 3] = 0;
+    // Slot (i + 1) % 3 is zero; slot (i + 2) % 3, and the long rows' count
+    // that the next round uses, were read before the barrier of the last round.
+    if (gtid == 0) {
+      A.cnt[(i + 2) % 3] = 0;
+      A.cnt[3 + ((i + 1) & 1)] = 0;
+    }
     scanned += V.na;
     const uint64_t before = left;
     level_frontier(A, V, A.r0 + i + 1, (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], gtid, gthreads);
@@ -565,6 +746,26 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(Pee
       uint32_t* fr = (i & 1) ? A.front[1] : A.front[0];
       uint32_t* nx = (i & 1) ? A.front[0] : A.front[1];
       unsigned long long* nc = &A.cnt[(i + 1) % 3];
+      if (kLists) {
+        unsigned long long* bc = &A.cnt[3 + (i & 1)];
+        list_round(A, V, fr, nf, r, nx, nc, bc, tdeg, tdec);
+        if (gtid == 0) {
+          A.cnt[(i + 2) % 3] = 0;        // read at the start of round i-1
+          A.cnt[3 + ((i + 1) & 1)] = 0;  // long rows of round i-1, read before the barrier ending it
+        }
+        src[0] = nc;
+        src[1] = bc;
+        if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+        const uint64_t nbig = sh[1];
+        if (nbig) {
+          list_round_long(A, V, nbig, r, nx, nc, woff, wtmp, tdec);
+          if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+        }
+        alive -= nf;
+        ++i;
+        ++rounds;
+        continue;
+      }
       const uint32_t thr = A.gthr_max ? __ldcg(A.gthr_max) : V.thr;
       const bool recount = A.R.bits && (double)nf * (double)(thr > 0 ? thr : 1) * (double)A.gamma >
                                            (double)alive * (double)A.wavg;
@@ -604,7 +805,7 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(Pee
     ++levels;
     if (gave_up || alive == 0) break;
     // Bring the bitsets up to date with this cascade's remaining deletions.
-    if (A.R.bits && pending) {
+    if (!kLists && A.R.bits && pending) {
       if (pending > alive) {
         zero_bits(A, gtid, gthreads);
         if (!grid_barrier(A.words, A.timeout_ns)) return;
@@ -871,7 +1072,8 @@ struct Peeler {
   const Sub* s;
   uint32_t* sup;
   uint32_t* truss;
-  DBuf state, alive[2], front[2], cnt, out, mm, adeg, acct;
+  DBuf state, alive[2], front[2], cnt, out, mm, adeg, acct, table, big;
+  uint32_t table_bits = 0;
   uint64_t scanned = 0;  // alive-list entries scanned by level frontiers
   int ai = 0;
   uint64_t na = 0;
@@ -907,12 +1109,35 @@ struct Peeler {
     na = m;
     smem = s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, kPeelThreads);
     coop_grid = 0;
+    build_table();
     if (c->opt.persistent || s->W) {
-      allow_max_dynamic_smem((const void*)k_levels);
+      allow_max_dynamic_smem(kernel());
       int per_sm = 0;
-      KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_levels, kPeelThreads, smem));
+      KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(), kPeelThreads, smem));
       coop_grid = std::min(coop_blocks(c, per_sm), kMaxGrid);
     }
+  }
+
+  const void* kernel() const {
+    return table.get() ? (const void*)k_levels<true> : (const void*)k_levels<false>;
+  }
+
+  // List mode: the edge hash table, 8 to 20 bytes an edge, when the budget
+  // has room for it (else, and in host-stepped rounds, rows are merged).
+  void build_table() {
+    table.release();
+    big.release();
+    if (s->W || !c->opt.persistent) return;
+    table_bits = 10;
+    while (table_bits < 32 && (2ull << table_bits) < 5 * s->m) ++table_bits;
+    const uint64_t bytes = (8ull << table_bits) + s->m * sizeof(uint32_t);
+    if ((2ull << table_bits) < 5 * s->m || (c->budget && c->in_use + bytes + (1u << 20) > c->budget)) return;
+    table.alloc(c, 8ull << table_bits);
+    big.alloc(c, s->m * sizeof(uint32_t));
+    KT_CUDA(cudaMemsetAsync(table.get(), 0xff, 8ull << table_bits, c->stream));
+    k_table_build<<<grid_for(s->m, 256, c->num_sms * 16), 256, 0, c->stream>>>(
+        s->m, s->ends.as<uint64_t>(), table.as<unsigned long long>(), table_bits);
+    KT_LAUNCHED(c);
   }
 
   PeelArgs args(uint32_t t) {
@@ -947,6 +1172,9 @@ struct Peeler {
     A.gthr = track ? gthr.as<uint32_t>() : nullptr;
     A.egr = track ? egr.as<uint32_t>() : nullptr;
     A.gthr_max = track ? tmax.as<uint32_t>() : nullptr;
+    A.table = table.as<unsigned long long>();
+    A.table_bits = table_bits;
+    A.big = big.as<uint32_t>();
     A.fail_below = fail_below;
     return A;
   }
@@ -990,7 +1218,7 @@ struct Peeler {
     {
       CoopLock coop(c);
       void* p[] = {&A, &L};
-      KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_levels, dim3(coop_grid), dim3(kPeelThreads), p, smem,
+      KT_CUDA(cudaLaunchCooperativeKernel(kernel(), dim3(coop_grid), dim3(kPeelThreads), p, smem,
                                           c->stream));
       KT_LAUNCHED(c);
       c->timer.end(c->stream, e0, &c->stats.ms_peel_kernel);
