@@ -97,8 +97,10 @@ const char* kt_status_string(kt_status s);
  *                               only requests whose estimated footprint is at most
  *                               this many MB, the other lanes any (0: every lane any)
  *   serve_small_coop (0)        the small lane's k-core and peel rounds: 0 = host-
- *                               stepped (no cooperative launch, so it never waits for
- *                               another lane's), 1 = cooperative launches taking turns
+ *                               stepped while another lane has a wave in flight (no
+ *                               cooperative launch, so it never waits for another
+ *                               lane's; with the other lanes idle, cooperative),
+ *                               1 = cooperative launches taking turns
  *                               with the other lanes'
  *   serve_partition (0)         1: the other lanes admit only requests above
  *                               serve_small_mb (0: any request)

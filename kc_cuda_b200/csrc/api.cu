@@ -112,25 +112,26 @@ float event_ms(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
-// Device bytes (padded) -> Graph.
+// Device bytes (padded) -> Graph.  The stage times (ms_parse, ms_csr) are
+// added when the call's timers are resolved.
 void graph_from_device_bytes(Ctx* c, const uint8_t* dbuf, uint64_t len, Graph& g) {
   reset_words(c);
-  KT_CUDA(cudaEventRecord(c->ev[4], c->stream));
+  c->stats.ms_parse = c->stats.ms_csr = 0;
+  Timer tm(c);
+  tm.start();
   DBuf block_off;
   const uint64_t lines = parse_count_lines(c, dbuf, len, block_off);
   DBuf keys(c, (lines ? lines : 1) * sizeof(uint64_t));
   parse_lines(c, dbuf, len, block_off, keys.as<uint64_t>(), dev_words(c));
-  check_words(c, "parse");
   DevWords w;
-  copy_d2h(c, &w, c->words.get(), sizeof(DevWords));
+  read_checked(c, &w, c->words.get(), sizeof(DevWords), "parse");
   const uint64_t n = (w.counters[1] & 1) ? (uint64_t)(uint32_t)w.counters[0] + 1 : 0;
   reset_words(c);
   block_off.release();
-  KT_CUDA(cudaEventRecord(c->ev[5], c->stream));
+  tm.stop(&c->stats.ms_parse);
+  tm.start();
   build_graph(c, keys.as<uint64_t>(), lines, n, g, true);
-  KT_CUDA(cudaEventRecord(c->ev[6], c->stream));
-  c->stats.ms_parse = event_ms(c->ev[4], c->ev[5]);
-  c->stats.ms_csr = event_ms(c->ev[5], c->ev[6]);
+  tm.stop(&c->stats.ms_csr);
 }
 
 // Host TSV bytes -> Graph with the host-to-device copy overlapped with the
@@ -170,7 +171,9 @@ static void load_tsv_pipelined(Ctx* c, const char* bytes, uint64_t len, uint64_t
     KT_CUDA(cudaEventRecord(landed[i], c->copy_stream));
     c->h2d_bytes += n;
   }
-  KT_CUDA(cudaEventRecord(c->ev[4], c->stream));
+  c->stats.ms_parse = c->stats.ms_csr = 0;
+  Timer tm(c);
+  tm.start();
   std::vector<DBuf> part(nch);
   std::vector<uint64_t> plines(nch, 0);
   uint64_t lines = 0;
@@ -204,11 +207,10 @@ static void load_tsv_pipelined(Ctx* c, const char* bytes, uint64_t len, uint64_t
   }
   const uint64_t n = (w.counters[1] & 1) ? (uint64_t)(uint32_t)w.counters[0] + 1 : 0;
   reset_words(c);
-  KT_CUDA(cudaEventRecord(c->ev[5], c->stream));
+  tm.stop(&c->stats.ms_parse);  // copy and parse, overlapped
+  tm.start();
   build_graph(c, keys.as<uint64_t>(), lines, n, g, true);
-  KT_CUDA(cudaEventRecord(c->ev[6], c->stream));
-  c->stats.ms_parse = event_ms(c->ev[4], c->ev[5]);  // copy and parse, overlapped
-  c->stats.ms_csr = event_ms(c->ev[5], c->ev[6]);
+  tm.stop(&c->stats.ms_csr);
 }
 
 void load_tsv(Ctx* c, const char* bytes, uint64_t len, Graph& g) {
@@ -372,7 +374,7 @@ kt_status kt_init(int device, uint64_t budget, kt_ctx** out) {
     c.budget = budget ? budget : (uint64_t)((fr + (reserved > used ? reserved - used : 0)) * 0.9);
     live_contexts(device, +1);
     h->counted = true;
-    KT_CUDA(cudaHostAlloc(&c.pinned, 4096, cudaHostAllocDefault));
+    KT_CUDA(cudaHostAlloc(&c.pinned, kt::kPinnedBytes, cudaHostAllocDefault));
     for (auto& e : c.ev) KT_CUDA(cudaEventCreate(&e));
     c.words.alloc(&c, sizeof(kt::DevWords));
     kt::reset_words(&c);
@@ -399,6 +401,9 @@ void kt_destroy(kt_ctx* h) {
     for (auto& e : h->c.ev)
       if (e) cudaEventDestroy(e);
     if (h->c.pinned) cudaFreeHost(h->c.pinned);
+    for (auto& e : h->c.slot_done)
+      if (e) cudaEventDestroy(e);
+    if (h->c.slots) cudaFreeHost(h->c.slots);
     if (h->c.stream) cudaStreamDestroy(h->c.stream);
     if (h->c.copy_stream) cudaStreamDestroy(h->c.copy_stream);
     // The last context on the device hands the pool's cached memory back,
@@ -502,6 +507,7 @@ kt_status kt_load_tsv(kt_ctx* h, const char* bytes, uint64_t len, kt_graph** out
   KT_API_BEGIN(h)
   kt_graph* g = new kt_graph;
   try {
+    kt::ResolveTimers resolve{&h->c};
     kt::load_tsv(&h->c, bytes, len, g->g);
   } catch (...) {
     delete g;
@@ -517,6 +523,7 @@ kt_status kt_load_tsv_file(kt_ctx* h, const char* path, kt_graph** out) {
   KT_API_BEGIN(h)
   kt_graph* g = new kt_graph;
   try {
+    kt::ResolveTimers resolve{&h->c};
     kt::load_tsv_file(&h->c, path, g->g);
   } catch (...) {
     delete g;
@@ -586,12 +593,10 @@ kt_status kt_solve_tsv(kt_ctx* h, const char* bytes, uint64_t len, uint32_t* kma
   kt::begin_solve_stats(c);
   KT_CUDA(cudaEventRecord(c->ev[0], c->stream));
   {
+    kt::ResolveTimers resolve{c};
     kt::Graph g;
     kt::load_tsv(c, bytes, len, g);
-    const double p = c->stats.ms_parse, q = c->stats.ms_csr;
     kt::solve_graph(c, g, kmax, edges);
-    c->stats.ms_parse = p;
-    c->stats.ms_csr = q;
   }
   KT_CUDA(cudaEventRecord(c->ev[1], c->stream));
   c->stats.ms_total = kt::event_ms(c->ev[0], c->ev[1]);
@@ -627,14 +632,11 @@ kt_status kt_solve_staged(kt_ctx* h, const kt_tsv* t, uint32_t* kmax, uint64_t* 
   auto host_ms = [&] { return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count(); };
   KT_CUDA(cudaEventRecord(c->ev[0], c->stream));
   {
+    kt::ResolveTimers resolve{c};
     kt::Graph g;
     kt::graph_from_device_bytes(c, t->bytes.as<uint8_t>(), t->len, g);
-    KT_LOG(c, "kt: +%.2f ms graph built (parse %.2f, build %.2f ms)\n", host_ms(), c->stats.ms_parse,
-           c->stats.ms_csr);
-    const double p = c->stats.ms_parse, q = c->stats.ms_csr;
+    KT_LOG(c, "kt: +%.2f ms graph built\n", host_ms());
     kt::solve_graph(c, g, kmax, edges);
-    c->stats.ms_parse = p;
-    c->stats.ms_csr = q;
     KT_LOG(c, "kt: +%.2f ms solved\n", host_ms());
   }
   KT_CUDA(cudaEventRecord(c->ev[1], c->stream));

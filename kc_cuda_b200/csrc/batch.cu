@@ -182,7 +182,7 @@ __global__ void k_alive_degree(const uint32_t* __restrict__ list, uint64_t na, c
 }
 
 // Clique keys (local canonical u << 32 | v) of a planted clique.
-void clique_keys(const std::vector<uint32_t>& vs, std::vector<uint64_t>& out) {
+void clique_keys(const std::vector<uint32_t>& vs, Records& out) {
   for (size_t i = 0; i < vs.size(); ++i)
     for (size_t j = i + 1; j < vs.size(); ++j) {
       const uint64_t a = vs[i], b = vs[j];
@@ -212,14 +212,18 @@ void BatchItem::from_mix(uint64_t index, uint64_t base_seed) {
 
 void BatchItem::from_pairs(const uint64_t* xy, uint64_t count) {
   generated = false;
-  extra.assign(xy, xy + count);
-  uint64_t mx = 0;
-  bool any = false;
-  for (uint64_t i = 0; i < count; ++i) {
-    mx = std::max<uint64_t>(mx, std::max<uint64_t>(xy[i] >> 32, (uint32_t)xy[i]));
-    any = true;
+  // Copied and scanned for the largest id in one pass, by several threads
+  // where that pays (30M records: 137 -> 14 ms, most of it first-touched pages).
+  extra.resize(count);
+  uint64_t* to = extra.data();
+  uint32_t mx = 0;
+#pragma omp parallel for schedule(static) num_threads(8) reduction(max : mx) if (count >= (1u << 16))
+  for (int64_t i = 0; i < (int64_t)count; ++i) {
+    const uint64_t k = xy[i];
+    to[i] = k;
+    mx = std::max(mx, std::max((uint32_t)(k >> 32), (uint32_t)k));
   }
-  n = any ? mx + 1 : 0;
+  n = count ? (uint64_t)mx + 1 : 0;
   draws = 0;
   nkeys = count;
 }
@@ -266,7 +270,11 @@ static uint64_t wave_keys(Ctx* c, const std::vector<BatchItem*>& items, DBuf& ke
   }
   // Clique keys of generated graphs and records of host graphs (canonical,
   // self-loops -> ~0), in union ids, through one staging copy.
-  std::vector<uint64_t> stage_h, src, dst;
+  uint64_t extras = 0;
+  for (const BatchItem* it : items) extras += it->extra.size();
+  Records stage_h;
+  stage_h.reserve(extras);
+  std::vector<uint64_t> src, dst;
   for (uint32_t g = 0; g < G; ++g) {
     const BatchItem& it = *items[g];
     if (it.extra.empty()) continue;
@@ -439,16 +447,15 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
   uint64_t nkeys = 0;
   std::vector<uint64_t> vbase;
   // Input: generation (or upload) of the wave's edge keys, timed apart.
-  KT_CUDA(cudaEventRecord(c->ev[4], c->stream));
-  const uint64_t nv = wave_keys(c, items, keys, nkeys, vbase);
-  KT_CUDA(cudaEventRecord(c->ev[5], c->stream));
-  st.ms_parse += event_ms(c->ev[4], c->ev[5]);
   Timer tm(c);
+  tm.start();
+  const uint64_t nv = wave_keys(c, items, keys, nkeys, vbase);
+  tm.stop(&st.ms_parse);
   tm.start();
   Graph U;
   build_graph(c, keys.as<uint64_t>(), nkeys, nv, U);
   keys.release();
-  st.ms_csr += tm.stop();
+  tm.stop(&st.ms_csr);
   if (G == 1) {
     // A wave of one graph takes the single-graph driver: k-core probes
     // instead of the union's full decomposition, and none of the per-graph
@@ -504,7 +511,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
   }
   std::vector<char> single(G, 0);
   for (uint32_t g = 0; g < G; ++g) single[g] = in_max[g] * 4 >= with_edge[g];
-  st.ms_kcore += tm.stop();
+  tm.stop(&st.ms_kcore);
 
   // The graphs of a wave are split in two classes for each phase: those
   // whose working core fits the bitset limit (dense_max_n vertices) and the
@@ -539,12 +546,12 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
     union_sub(c, U, dcore.as<uint32_t>(), dgid.as<uint32_t>(), G, need, s1);
     st.predict_vertices += s1.n;
     st.predict_edges += s1.m;
-    st.ms_subgraph += tm.stop();
+    tm.stop(&st.ms_subgraph);
     tm.start();
     DBuf sup1(c, (s1.m ? s1.m : 1) * sizeof(uint32_t));
     edge_support(c, s1, sup1.as<uint32_t>());
     const std::vector<uint32_t> ub = group_bounds(c, s1, sup1.as<uint32_t>(), cap);
-    st.ms_support += tm.stop();
+    tm.stop(&st.ms_support);
     tm.start();
     std::vector<uint32_t> level(G, 0);
     bool pending = false;
@@ -587,7 +594,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
         }
       }
     }
-    st.ms_peel += tm.stop();
+    tm.stop(&st.ms_peel);
   }
 
   // Phase 2.
@@ -622,7 +629,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
         dcore.as<uint32_t>(), dgid.as<uint32_t>(), nv, dneed.as<uint32_t>(), dcnt.as<unsigned long long>());
     KT_LAUNCHED(c);
     copy_d2h(c, n2.data(), dcnt.get(), G * 8ull);
-    st.ms_subgraph += tm.stop();
+    tm.stop(&st.ms_subgraph);
   }
   for (int cls = 0; cls < 2; ++cls) {
     std::vector<uint32_t> need(G, 0);
@@ -638,7 +645,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
     union_sub(c, U, dcore.as<uint32_t>(), dgid.as<uint32_t>(), G, need, s2);
     st.core_vertices += s2.n;
     st.core_edges += s2.m;
-    st.ms_subgraph += tm.stop();
+    tm.stop(&st.ms_subgraph);
     tm.start();
     DBuf sup2(c, (s2.m ? s2.m : 1) * sizeof(uint32_t));
     std::vector<uint32_t> thr(G, 0);
@@ -659,7 +666,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
     Sub s3;
     DBuf sup3;
     const bool rebuilt = survivors(c, s2, sup2.as<uint32_t>(), thr, true, s3, sup3);
-    st.ms_support += tm.stop();
+    tm.stop(&st.ms_support);
     tm.start();
     const auto t_p = std::chrono::steady_clock::now();
     const uint32_t lv0 = st.levels, rd0 = st.rounds;
@@ -676,7 +683,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
       tracked_peel(c, s3, sup3.as<uint32_t>(), t0c, stopc, km, cn);
     else
       tracked_peel(c, s2, sup2.as<uint32_t>(), t0c, stopc, km, cn);
-    st.ms_peel += tm.stop();
+    tm.stop(&st.ms_peel);
     KT_LOG(c, "kt: wave phase 2 class %d: %llu edges (%s), tracked peel %u levels %u rounds in %.2f ms\n", cls,
            (unsigned long long)(rebuilt ? s3.m : s2.m), rebuilt ? "survivors" : "whole cores", st.levels - lv0,
            st.rounds - rd0, std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_p).count());
@@ -771,6 +778,7 @@ void run_batch(Ctx* c, std::vector<BatchItem>& items, BatchRun& out) {
     const kt_stats before = lc->stats;
     solve_wave(lc, wave);
     if (lc->opt.verbose) {
+      lc->timer.resolve();
       const kt_stats& a = lc->stats;
       uint64_t keys = 0, verts_w = 0;
       for (const BatchItem* it : wave) keys += it->nkeys, verts_w += it->n;

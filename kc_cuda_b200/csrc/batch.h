@@ -1,10 +1,30 @@
 // Batched solving (batch.cu).
 #pragma once
+#include <memory>
 #include <vector>
 
 #include "stages.h"
 
 namespace kt {
+
+// Vectors whose elements are written before they are read: resize() leaves
+// them uninitialised, so their pages are first touched by who fills them.
+template <class T>
+struct UninitAllocator : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = UninitAllocator<U>;
+  };
+  template <class U>
+  void construct(U* p) noexcept {
+    ::new (static_cast<void*>(p)) U;
+  }
+  template <class U, class A, class... R>
+  void construct(U* p, A&& a, R&&... r) {
+    ::new (static_cast<void*>(p)) U(std::forward<A>(a), std::forward<R>(r)...);
+  }
+};
+using Records = std::vector<uint64_t, UninitAllocator<uint64_t>>;
 
 // One graph of a batch: generated on the device from a mix spec, or host
 // records x << 32 | y.
@@ -15,7 +35,7 @@ struct BatchItem {
   uint64_t draws = 0;  // generated draws
   uint64_t seed = 0;
   uint64_t nkeys = 0;  // draws + extra
-  std::vector<uint64_t> extra;  // clique keys (generated) or the records (host)
+  Records extra;       // clique keys (generated) or the records (host)
   uint32_t kmax = 0;
   uint64_t count = 0;
   void from_mix(uint64_t index, uint64_t base_seed);

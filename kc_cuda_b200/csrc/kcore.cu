@@ -935,7 +935,8 @@ void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixe
   SearchOut& h = *static_cast<SearchOut*>(result);
   {
     CoopLock coop(c);
-    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_search, dim3(coop_grid), dim3(256), p, 0, c->stream));
+    const unsigned grid = coop_blocks_for(coop_grid, 2 * g.m, 8 * 32 * kWide);
+    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_search, dim3(grid), dim3(256), p, 0, c->stream));
     KT_LAUNCHED(c);
     read_checked(c, &h, out.get(), sizeof(SearchOut), "k-core probe");
   }
@@ -1220,7 +1221,7 @@ void KCore::core_numbers_persistent(Ctx* c, uint32_t* dcore) {
   int per_sm = 0;
   KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_levels, 256, 0));
   if (c->opt.kcore_blocks_per_sm > 0) per_sm = (int)std::min<int64_t>(per_sm, c->opt.kcore_blocks_per_sm);
-  const unsigned grid = coop_blocks(c, per_sm);
+  const unsigned grid = coop_blocks_for(coop_blocks(c, per_sm), 2 * g.m, 8 * 32 * kWide);
   void* p[] = {&A};
   uint64_t h[5];
   {

@@ -159,8 +159,12 @@ __device__ __forceinline__ bool grid_barrier_read(DevWords* w, unsigned long lon
                                                   unsigned long long* sh) {
   __syncthreads();
   bool ok = true;
-  if (threadIdx.x == 0) {
-    const uint32_t nb = gridDim.x * gridDim.y * gridDim.z;
+  const uint32_t nb = gridDim.x * gridDim.y * gridDim.z;
+  if (nb == 1 && threadIdx.x == 0) {  // nobody to wait for
+    __threadfence();
+    if (timeout_ns == 0) atomicOr(&w->err, kDevErrBarrier);
+    ok = ld_acquire_u32(&w->err) == 0;
+  } else if (threadIdx.x == 0) {
     __threadfence();
     const uint32_t old = atomicAdd(&w->bar, blockIdx.x == 0 ? 0x80000000u - (nb - 1) : 1u);
     unsigned long long t0 = 0;
@@ -180,6 +184,8 @@ __device__ __forceinline__ bool grid_barrier_read(DevWords* w, unsigned long lon
       }
       if (spins > 64) __nanosleep(spins > 1024 ? 256 : 32);
     }
+  }
+  if (threadIdx.x == 0) {
     unsigned long long val[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) val[i] = src[i] ? ld_relaxed_u64(src[i]) : 0ULL;

@@ -1114,7 +1114,8 @@ struct Peeler {
       allow_max_dynamic_smem(kernel());
       int per_sm = 0;
       KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(), kPeelThreads, smem));
-      coop_grid = std::min(coop_blocks(c, per_sm), kMaxGrid);
+      // A warp counts eight edges at once, or looks up kJobWide entries a lane.
+      coop_grid = coop_blocks_for(std::min(coop_blocks(c, per_sm), kMaxGrid), s->m, 64);
     }
   }
 

@@ -1,5 +1,6 @@
 // Context plumbing: device buffers charged to the HBM budget, small copies,
 // and the CUDA error -> kt::Error conversion.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -68,9 +69,72 @@ void allow_max_dynamic_smem(const void* func) {
 
 void sync(Ctx* c) { KT_CUDA(cudaStreamSynchronize(c->stream)); }
 
+namespace {
+
+// Whether a copy of `bytes` at host address p goes through the pinned slots:
+// large, and to or from pageable memory, which the driver would stage with one
+// thread (loading and solving 48 MB of records 5.6 -> 3.7 ms, 32 MB of supports
+// counted and returned 6.8 -> 4.9 ms).
+bool through_slots(Ctx* c, const void* p, size_t bytes) {
+  if (bytes < (1 << 20)) return false;
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (a.type != cudaMemoryTypeUnregistered) return false;
+  if (c->slots) return true;
+  if (cudaHostAlloc(reinterpret_cast<void**>(&c->slots), kSlotBytes * kCopySlots, cudaHostAllocDefault) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    c->slots = nullptr;  // no pinned memory to be had: the driver's staging
+    return false;
+  }
+  for (cudaEvent_t& e : c->slot_done)
+    if (!e) KT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return true;
+}
+
+void parallel_memcpy(char* dst, const char* src, size_t n) {
+  constexpr int kParts = 8;
+#pragma omp parallel for schedule(static) num_threads(kParts)
+  for (int t = 0; t < kParts; ++t) {
+    const size_t a = n * t / kParts, b = n * (t + 1) / kParts;
+    std::memcpy(dst + a, src + a, b - a);
+  }
+}
+
+}  // namespace
+
 void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
   c->d2h_bytes += bytes;
+  if (bytes <= kPinnedBytes) {
+    // Small results through the context's pinned words: a copy to pageable
+    // memory is staged by the driver.
+    KT_CUDA(cudaMemcpyAsync(c->pinned, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+    sync(c);
+    std::memcpy(dst, c->pinned, bytes);
+    return;
+  }
+  if (through_slots(c, dst, bytes)) {
+    const size_t n = (bytes + kSlotBytes - 1) / kSlotBytes;
+    auto size = [&](size_t i) { return std::min(kSlotBytes, bytes - i * kSlotBytes); };
+    for (size_t i = 0; i < n + kCopySlots - 1; ++i) {
+      if (i < n) {
+        const int s = (int)(i % kCopySlots);
+        KT_CUDA(cudaMemcpyAsync(c->slots + s * kSlotBytes, static_cast<const char*>(src) + i * kSlotBytes, size(i),
+                                cudaMemcpyDeviceToHost, c->stream));
+        KT_CUDA(cudaEventRecord(c->slot_done[s], c->stream));
+      }
+      if (i + 1 < kCopySlots) continue;  // keep kCopySlots - 1 copies ahead
+      const size_t k = i + 1 - kCopySlots;
+      const int s = (int)(k % kCopySlots);
+      KT_CUDA(cudaEventSynchronize(c->slot_done[s]));
+      parallel_memcpy(static_cast<char*>(dst) + k * kSlotBytes, c->slots + s * kSlotBytes, size(k));
+    }
+    return;
+  }
   KT_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
   sync(c);
 }
@@ -78,6 +142,18 @@ void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
 void copy_h2d(Ctx* c, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
   c->h2d_bytes += bytes;
+  if (through_slots(c, src, bytes)) {
+    for (size_t at = 0, i = 0; at < bytes; at += kSlotBytes, ++i) {
+      const int s = (int)(i % kCopySlots);
+      const size_t n = std::min(kSlotBytes, bytes - at);
+      KT_CUDA(cudaEventSynchronize(c->slot_done[s]));
+      parallel_memcpy(c->slots + s * kSlotBytes, static_cast<const char*>(src) + at, n);
+      KT_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + at, c->slots + s * kSlotBytes, n, cudaMemcpyHostToDevice,
+                              c->stream));
+      KT_CUDA(cudaEventRecord(c->slot_done[s], c->stream));
+    }
+    return;
+  }
   KT_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, c->stream));
 }
 

@@ -9,9 +9,11 @@
 // footprint fits the lane's share of the budget (and up to a graph cap) --
 // with two or more lanes, the last lane admits only small requests
 // (footprint up to serve_small_mb), so they never queue behind a wave of
-// large graphs; it launches nothing cooperative, and the other lanes'
-// cooperative grids take 75% of the resident blocks, so its waves run beside
-// theirs -- and
+// large graphs; while another lane has a wave in flight it launches nothing
+// cooperative, and the other lanes' cooperative grids take 75% of the resident
+// blocks, so its waves run beside theirs (with the other lanes idle it holds
+// the cooperative launches for its wave, which is then solved as theirs are) --
+// and
 // solves the admitted set as one wave -- one disjoint union through every
 // stage, each graph on its own peel levels (batch.cu).  So while one wave is
 // on the device, requests that arrive meanwhile start in the next free lane
@@ -71,6 +73,9 @@ struct kt_server {
   uint64_t small_bytes = 0;  // the small lane (the last) admits only requests this small (0: any)
   bool partition = false;    // ... and the other lanes only larger ones
   int64_t lane0_coop_pct = 100;  // the server's context's coop_occupancy_pct, restored at the end
+  bool stepped = false;          // the small lane's launches are host-stepped (unless the others are idle)
+  kt::Options full;              // its options with cooperative launches
+  int in_flight = 0;             // waves in flight
   // Whether a lane admits a request: the small lane only small ones; with
   // the partition the other lanes only the others.
   bool admits(bool small_lane, const Request* r) const {
@@ -108,6 +113,7 @@ struct kt_server {
     cudaSetDevice(c->device);
     while (true) {
       std::vector<Request*> wave;
+      std::unique_lock<std::mutex> turn;  // the cooperative launches, for this wave
       {
         std::unique_lock<std::mutex> lk(m);
         work_cv.wait(lk, [&] { return stopping || !queue.empty(); });
@@ -138,6 +144,8 @@ struct kt_server {
         }
         // Others still queued: wake the other free lanes for them.
         if (!queue.empty()) work_cv.notify_all();
+        if (small_lane && stepped && in_flight == 0) turn = std::unique_lock<std::mutex>(coop, std::try_to_lock);
+        ++in_flight;
       }
       const Clock::time_point t_admit = Clock::now();
       std::vector<kt::BatchItem*> items;
@@ -150,6 +158,11 @@ struct kt_server {
       uint64_t peak = 0;
       {
         std::lock_guard<std::recursive_mutex> lk(c->mu);
+        const kt::Options own = c->opt;
+        if (turn) {
+          c->coop_mu = nullptr;  // held already
+          c->opt = full;
+        }
         try {
           kt::reset_words(c);
           kt::solve_wave(c, items);
@@ -169,9 +182,15 @@ struct kt_server {
         } catch (...) {
         }
         peak = c->peak;
+        if (turn) {
+          c->coop_mu = &coop;
+          c->opt = own;
+          turn.unlock();
+        }
       }
       const Clock::time_point t_done = Clock::now();
       std::lock_guard<std::mutex> lk(m);
+      --in_flight;
       const uint32_t wave_no = (uint32_t)st.waves++;
       st.ms_busy += ms_between(t_admit, t_done);
       if (wave.size() > st.max_wave_graphs) st.max_wave_graphs = wave.size();
@@ -270,9 +289,11 @@ kt_status kt_server_create(kt_ctx* ctx, uint32_t max_wave_graphs, kt_server** ou
       lc.coop_mu = &s->coop;
       if (!s->small_bytes || opt.serve_small_coop) continue;
       if (i + 1 == s->lanes.size()) {
-        // The small lane launches nothing cooperative (host-stepped rounds,
-        // list-mode support), so it never waits for another lane's
+        // The small lane launches nothing cooperative beside another lane's
+        // wave (host-stepped rounds, list-mode support), so it never waits for another lane's
         // cooperative grid to end ...
+        s->stepped = true;
+        s->full = lc.opt;
         lc.opt.persistent = 0;
         lc.opt.dense_max_n = 0;
       } else {

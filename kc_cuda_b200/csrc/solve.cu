@@ -92,15 +92,7 @@ void begin_solve_stats(Ctx* c) {
 }
 
 void solve_graph(Ctx* c, const Graph& g, uint32_t* kmax, uint64_t* count) {
-  struct Resolve {
-    Ctx* c;
-    ~Resolve() {
-      try {
-        c->timer.resolve();
-      } catch (...) {
-      }
-    }
-  } resolve{c};
+  ResolveTimers resolve{c};
   solve_graph_inner(c, g, kmax, count);
 }
 
@@ -170,7 +162,7 @@ void solve_graph_inner(Ctx* c, const Graph& g, uint32_t* kmax, uint64_t* count) 
   const uint64_t n_edge_vertices = kc.n_alive;  // vertices with an edge
   const uint32_t cmax = kc.find_max_core(c);
   st.cmax = cmax;
-  st.ms_kcore += tm.stop();
+  tm.stop(&st.ms_kcore);
   mark("maximum core found");
   if (g.m == 0 || cmax < 2) return;  // a triangle needs three vertices of degree >= 2
 
@@ -180,20 +172,20 @@ void solve_graph_inner(Ctx* c, const Graph& g, uint32_t* kmax, uint64_t* count) 
   if (!c->opt.predict || kc.n_alive * 4 >= n_edge_vertices) {
     tm.start();
     kc.restore_core(c, 2);
-    st.ms_kcore += tm.stop();
+    tm.stop(&st.ms_kcore);
     tm.start();
     Sub s;
     build_sub(c, g, kc, s);
     st.core_vertices = s.n;
     st.core_edges = s.m;
-    st.ms_subgraph += tm.stop();
+    tm.stop(&st.ms_subgraph);
     tm.start();
     DBuf sup(c, (s.m ? s.m : 1) * sizeof(uint32_t));
     edge_support(c, s, sup.as<uint32_t>());
-    st.ms_support += tm.stop();
+    tm.stop(&st.ms_support);
     tm.start();
     const PeelResult p = predict_peel(c, s, sup.as<uint32_t>(), cmax);
-    st.ms_peel += tm.stop();
+    tm.stop(&st.ms_peel);
     st.levels += p.levels;
     st.rounds += (uint32_t)p.rounds;
     *kmax = p.kmax;
@@ -210,16 +202,16 @@ void solve_graph_inner(Ctx* c, const Graph& g, uint32_t* kmax, uint64_t* count) 
     build_sub(c, g, kc, s1);
     st.predict_vertices = s1.n;
     st.predict_edges = s1.m;
-    st.ms_subgraph += tm.stop();
+    tm.stop(&st.ms_subgraph);
     mark("prediction subgraph built");
     tm.start();
     DBuf sup1(c, (s1.m ? s1.m : 1) * sizeof(uint32_t));
     edge_support(c, s1, sup1.as<uint32_t>());
-    st.ms_support += tm.stop();
+    tm.stop(&st.ms_support);
     mark("prediction support counted");
     tm.start();
     const PeelResult p1 = predict_peel(c, s1, sup1.as<uint32_t>(), cmax);
-    st.ms_peel += tm.stop();
+    tm.stop(&st.ms_peel);
     mark("prediction peeled");
     st.levels += p1.levels;
     st.rounds += (uint32_t)p1.rounds;
@@ -235,14 +227,14 @@ void solve_graph_inner(Ctx* c, const Graph& g, uint32_t* kmax, uint64_t* count) 
   st.kmax_lower_bound = L;
   tm.start();
   kc.restore_core(c, L >= 3 ? L - 1 : 2);
-  st.ms_kcore += tm.stop();
+  tm.stop(&st.ms_kcore);
   mark("search core restored");
   tm.start();
   Sub s2;
   build_sub(c, g, kc, s2);
   st.core_vertices = s2.n;
   st.core_edges = s2.m;
-  st.ms_subgraph += tm.stop();
+  tm.stop(&st.ms_subgraph);
   mark("search subgraph built");
   tm.start();
   DBuf sup2(c, (s2.m ? s2.m : 1) * sizeof(uint32_t));
@@ -275,28 +267,17 @@ void solve_graph_inner(Ctx* c, const Graph& g, uint32_t* kmax, uint64_t* count) 
       supp = sup3.as<uint32_t>();
     }
   }
-  st.ms_support += tm.stop();
+  tm.stop(&st.ms_support);
   mark("search support counted");
   tm.start();
   const PeelResult p2 = truss_peel(c, *sp, supp, t2, L >= 3 ? C : 0, nullptr);
-  st.ms_peel += tm.stop();
+  tm.stop(&st.ms_peel);
   mark("search peeled");
   st.levels += p2.levels;
   st.rounds += (uint32_t)p2.rounds;
   *kmax = p2.kmax;
   *count = p2.count;
 }
-
-// Resolves the context's kernel timers when a stage-output call ends.
-struct ResolveTimers {
-  Ctx* c;
-  ~ResolveTimers() {
-    try {
-      c->timer.resolve();
-    } catch (...) {
-    }
-  }
-};
 
 void graph_support(Ctx* c, const Graph& g, uint32_t* dout) {
   begin_solve_stats(c);

@@ -4,25 +4,24 @@
 
 namespace kt {
 
-// Stream-ordered stage timer: stop() waits for the stage and returns its ms.
+// Stage timer: the span between start() and stop() is added to *acc when the
+// call's timers are resolved (a stage does not wait for the one before it).
 struct Timer {
   Ctx* c;
-  cudaEvent_t a, b;
-  explicit Timer(Ctx* cx) : c(cx) {
-    KT_CUDA(cudaEventCreate(&a));
-    KT_CUDA(cudaEventCreate(&b));
-  }
-  ~Timer() {
-    cudaEventDestroy(a);
-    cudaEventDestroy(b);
-  }
-  void start() { KT_CUDA(cudaEventRecord(a, c->stream)); }
-  double stop() {
-    KT_CUDA(cudaEventRecord(b, c->stream));
-    KT_CUDA(cudaEventSynchronize(b));
-    float ms = 0;
-    KT_CUDA(cudaEventElapsedTime(&ms, a, b));
-    return ms;
+  cudaEvent_t a = nullptr;
+  explicit Timer(Ctx* cx) : c(cx) {}
+  void start() { c->timer.begin(c->stream, nullptr, &a); }
+  void stop(double* acc) { c->timer.end(c->stream, a, acc); }
+};
+
+// Resolves the context's timers when a call ends, by an error too.
+struct ResolveTimers {
+  Ctx* c;
+  ~ResolveTimers() {
+    try {
+      c->timer.resolve();
+    } catch (...) {
+    }
   }
 };
 
