@@ -163,6 +163,65 @@ __device__ __forceinline__ void close_triangle(const PeelArgs& A, const Level& V
   }
 }
 
+// Position of the r-th (from 0) set bit of m.
+__device__ __forceinline__ uint32_t select_bit(uint32_t m, uint32_t r) {
+  uint32_t pos = 0;
+#pragma unroll
+  for (uint32_t s = 16; s >= 1; s >>= 1) {
+    const uint32_t low = __popc(m & ((1u << s) - 1u));
+    if (r >= low) {
+      r -= low;
+      m >>= s;
+      pos += s;
+    }
+  }
+  return pos;
+}
+
+// Words [w0, w0 + cw) (cw at most 32) of frontier edge e's two bitset rows:
+// the common neighbours found there are dealt one per lane (a warp scan of the
+// words' popcounts, then a search for each task's word and a select of its
+// bit), each closing its triangle.  Each common neighbour's edge ids come from
+// its position in the sorted rows, a popcount of the rows as built.  Bits of
+// edges deleted in earlier cascades are clear; deletions of this cascade are
+// caught by close_triangle's state test.  (With each lane closing the set bits
+// of its own word, a step of 32 words took as many iterations as the fullest
+// word has bits: 64 mix graphs, 741 decrement rounds, 23.7 ms; dealt 15.2 ms.)
+__device__ __forceinline__ void close_common(const PeelArgs& A, const Level& V, uint32_t e, uint32_t x, uint32_t y,
+                                             uint32_t thr, uint32_t W, uint32_t w0, uint32_t cw, uint32_t r,
+                                             uint32_t* next, unsigned long long* ncnt, uint32_t& ndec) {
+  const unsigned lane = lane_id();
+  const uint32_t i = w0 + lane;
+  uint32_t m = 0;
+  if (lane < cw && i < W) m = __ldcg(A.R.bits + A.R.off(x) + i) & __ldcg(A.R.bits + A.R.off(y) + i);
+  const uint32_t c = __popc(m);
+  const uint32_t incl = warp_incl_scan(c);
+  const uint32_t T = __shfl_sync(kFull, incl, 31);
+  if (T == 0) return;
+  const uint32_t excl = incl - c;
+  const uint64_t ox = A.off[x], oy = A.off[y];
+  for (uint32_t base = 0; base < T; base += 32) {
+    const uint32_t t = base + lane;
+    uint32_t lo = 0;  // the last word whose first task is at or before t
+#pragma unroll
+    for (uint32_t st = 16; st >= 1; st >>= 1) {
+      const uint32_t ec = __shfl_sync(kFull, excl, lo + st);
+      if (ec <= t) lo += st;
+    }
+    const uint32_t oexcl = __shfl_sync(kFull, excl, lo), om = __shfl_sync(kFull, m, lo);
+    bool pa = false, pb = false;
+    uint32_t a = 0, b = 0;
+    if (t < T) {
+      const uint32_t col = (w0 + lo) * 32 + select_bit(om, t - oexcl);
+      a = A.eid[ox + A.R.rank(x, col)];
+      b = A.eid[oy + A.R.rank(y, col)];
+      close_triangle(A, V, e, a, b, r, thr, pa, pb, ndec);
+    }
+    push_warp_full(pa, a, next, ncnt, A.cap, &A.words->err);
+    push_warp_full(pb, b, next, ncnt, A.cap, &A.words->err);
+  }
+}
+
 // One frontier edge, one warp.  Pushes into next / ncnt; adds the edge's
 // alive degrees and its decrements to the per-thread tallies.
 __device__ __forceinline__ void peel_edge(const PeelArgs& A, const Level& V, uint32_t e, uint32_t r, uint32_t* next,
@@ -185,32 +244,10 @@ __device__ __forceinline__ void peel_edge(const PeelArgs& A, const Level& V, uin
   uint32_t* err = &A.words->err;
   const unsigned lane = lane_id();
   if (A.R.sbits && (uint64_t)A.R.words(x) <= na + nb) {
-    // Dense rows shorter than the two lists: AND the two bitset rows (32
-    // words a step, one per lane); each common neighbour's edge ids come from
-    // its position in the sorted rows, a popcount of the rows as built.  Bits
-    // of edges deleted in earlier cascades are clear; deletions of this
-    // cascade are caught by close_triangle's state test, as in the merge.
-    const uint32_t* rx = A.R.bits + A.R.off(x);
-    const uint32_t* ry = A.R.bits + A.R.off(y);
+    // Dense rows shorter than the two lists: AND the two bitset rows, 32
+    // words a step.
     const uint32_t W = A.R.words(x);
-    const uint64_t ox = A.off[x], oy = A.off[y];
-    for (uint32_t i0 = 0; i0 < W; i0 += 32) {
-      const uint32_t i = i0 + lane;
-      uint32_t mset = i < W ? __ldcg(rx + i) & __ldcg(ry + i) : 0u;
-      while (__any_sync(kFull, mset != 0)) {
-        bool pa = false, pb = false;
-        uint32_t a = 0, b = 0;
-        if (mset) {
-          const uint32_t col = i * 32 + (uint32_t)(__ffs(mset) - 1);
-          mset &= mset - 1;
-          a = A.eid[ox + A.R.rank(x, col)];
-          b = A.eid[oy + A.R.rank(y, col)];
-          close_triangle(A, V, e, a, b, r, thr, pa, pb, ndec);
-        }
-        push_warp_full(pa, a, next, ncnt, A.cap, err);
-        push_warp_full(pb, b, next, ncnt, A.cap, err);
-      }
-    }
+    for (uint32_t w0 = 0; w0 < W; w0 += 32) close_common(A, V, e, x, y, thr, W, w0, 32, r, next, ncnt, ndec);
     tdec += ndec;
     return;
   }
@@ -430,75 +467,21 @@ __device__ __forceinline__ void list_round_long(const PeelArgs& A, const Level& 
   tdec += ndec;
 }
 
-// Rounds with few frontier edges split each edge's bitset intersection into
-// chunks of kSplitWords words, one warp per (edge, chunk), so a small
-// frontier of edges with many triangles keeps the whole grid busy.
-constexpr uint32_t kSplitWords = 8;
+// A decrement round over (frontier edge, chunk of cw words) units, a warp
+// each, so a small frontier of edges with many triangles keeps the whole grid
+// busy (a round of one edge in a core of 1,311 vertices: 13.2 us in chunks of 8
+// words, 5.4 us in the shortest that fill the grid); edges that use the sorted-list merge go whole to the warp of their
+// first chunk.
+constexpr uint32_t kSplitWords = 8;  // words of a chunk at most
 
-// Position of the r-th (from 0) set bit of m.
-__device__ __forceinline__ uint32_t select_bit(uint32_t m, uint32_t r) {
-  uint32_t pos = 0;
-#pragma unroll
-  for (uint32_t s = 16; s >= 1; s >>= 1) {
-    const uint32_t low = __popc(m & ((1u << s) - 1u));
-    if (r >= low) {
-      r -= low;
-      m >>= s;
-      pos += s;
-    }
-  }
-  return pos;
-}
-
-// Words [w0, w0 + kSplitWords) of frontier edge e's two bitset rows: the
-// common neighbours found there are dealt one per lane (a warp scan of the
-// words' popcounts, then a 3-step search for each task's word and a select of
-// its bit), each closing its triangle as in peel_edge.
-__device__ __forceinline__ void peel_edge_chunk(const PeelArgs& A, const Level& V, uint32_t e, uint32_t x, uint32_t y, uint32_t thr,
-                                                uint32_t W, uint32_t w0, uint32_t r, uint32_t* next,
-                                                unsigned long long* ncnt, uint64_t& tdec) {
-  const unsigned lane = lane_id();
-  const uint32_t i = w0 + lane;
-  uint32_t m = 0;
-  if (lane < kSplitWords && i < W) m = __ldcg(A.R.bits + A.R.off(x) + i) & __ldcg(A.R.bits + A.R.off(y) + i);
-  const uint32_t c = __popc(m);
-  const uint32_t incl = warp_incl_scan(c);
-  const uint32_t T = __shfl_sync(kFull, incl, 31);
-  const uint32_t excl = incl - c;
-  const uint64_t ox = A.off[x], oy = A.off[y];
+__device__ __forceinline__ void split_round(const PeelArgs& A, const Level& V, const uint32_t* fr, uint32_t nf,
+                                            uint32_t cw, uint32_t chunks, uint32_t r, uint32_t* next,
+                                            unsigned long long* ncnt, uint32_t gwarp, uint32_t gwarps,
+                                            uint64_t& tdeg, uint64_t& tdec) {
   uint32_t ndec = 0;
-  for (uint32_t base = 0; base < T; base += 32) {
-    const uint32_t t = base + lane;
-    uint32_t lo = 0;  // the last word (lane < kSplitWords) whose first task is <= t
-#pragma unroll
-    for (uint32_t st = kSplitWords / 2; st >= 1; st >>= 1) {
-      const uint32_t cand = lo + st;
-      const uint32_t ec = __shfl_sync(kFull, excl, cand & 31);
-      if (cand < kSplitWords && ec <= t) lo = cand;
-    }
-    const uint32_t oexcl = __shfl_sync(kFull, excl, lo), om = __shfl_sync(kFull, m, lo);
-    bool pa = false, pb = false;
-    uint32_t a = 0, b = 0;
-    if (t < T) {
-      const uint32_t col = (w0 + lo) * 32 + select_bit(om, t - oexcl);
-      a = A.eid[ox + A.R.rank(x, col)];
-      b = A.eid[oy + A.R.rank(y, col)];
-      close_triangle(A, V, e, a, b, r, thr, pa, pb, ndec);
-    }
-    push_warp_full(pa, a, next, ncnt, A.cap, &A.words->err);
-    push_warp_full(pb, b, next, ncnt, A.cap, &A.words->err);
-  }
-  tdec += ndec;
-}
-
-// A decrement round over (frontier edge, chunk) units; edges that use the
-// sorted-list merge go whole to the warp of their first chunk.
-__device__ __forceinline__ void split_round(const PeelArgs& A, const Level& V, const uint32_t* fr, uint64_t nf, uint64_t chunks,
-                                            uint32_t r, uint32_t* next, unsigned long long* ncnt, uint64_t gwarp,
-                                            uint64_t gwarps, uint64_t& tdeg, uint64_t& tdec) {
-  for (uint64_t u = gwarp; u < nf * chunks; u += gwarps) {
-    const uint64_t f = u / chunks;
-    const uint32_t ch = (uint32_t)(u - f * chunks);
+  for (uint32_t u = gwarp; u < nf * chunks; u += gwarps) {
+    const uint32_t f = u / chunks;
+    const uint32_t ch = u - f * chunks;
     const uint32_t e = fr[f];
     const uint64_t k = A.ends[e];
     const uint32_t x = (uint32_t)(k >> 32), y = (uint32_t)k;
@@ -508,10 +491,11 @@ __device__ __forceinline__ void split_round(const PeelArgs& A, const Level& V, c
       if (ch == 0) peel_edge(A, V, e, r, next, ncnt, tdeg, tdec);
       continue;
     }
-    if (ch * kSplitWords >= W) continue;
+    if (ch * cw >= W) continue;
     if (ch == 0 && lane_id() == 0) tdeg += (uint64_t)atomicSub(&A.adeg[x], 1u) + atomicSub(&A.adeg[y], 1u);
-    peel_edge_chunk(A, V, e, x, y, edge_thr(A, V, e), W, ch * kSplitWords, r, next, ncnt, tdec);
+    close_common(A, V, e, x, y, edge_thr(A, V, e), W, ch * cw, cw, r, next, ncnt, ndec);
   }
+  tdec += ndec;
 }
 
 __device__ __forceinline__ void flush_tallies(const PeelArgs& A, uint64_t tdeg, uint64_t tdec) {
@@ -591,25 +575,36 @@ __device__ __forceinline__ void clear_deleted(const PeelArgs& A, const Level& V,
   }
 }
 
+constexpr uint64_t kRowsInL2 = 64u << 20;  // bytes of bitset rows that stay in L2 beside the rest
+
 // Dense recount round r: every surviving edge gets its exact support in the
 // graph without this round's frontier; those below the threshold form the
 // next frontier.  Replaces per-triangle decrements when the frontier is a
 // large part of the graph.
-// Warps take the next group of the alive list from `cursor` (zero at the
-// start of the round), so the groups in flight stay a narrow window of the
-// tile-ordered list and the rows they read stay in L2.  A group is 32 entries,
-// or fewer (8 at least) where that leaves warps of the grid without one: its
-// edges are counted one after another.
+// A group is 32 entries of the alive list, or fewer (8 at least) where that
+// leaves warps of the grid without one: its edges are counted one after
+// another.  Rows that fit in L2 together are read in any order, so warps
+// stride over the groups; of more rows, warps take the next group from
+// `cursor` (zero at the start of the round), so that the groups in flight stay
+// a narrow window of the tile-ordered list -- the cursor is one word that every
+// group waits for, 10 us of a 25 us round of 230,000 edges.
 __device__ __forceinline__ void recount_round(const PeelArgs& A, const Level& V, uint32_t r, uint32_t* next,
                                               unsigned long long* ncnt, unsigned long long* cursor,
                                               uint64_t& trec, uint32_t* su) {
-  const uint64_t share = V.na / ((uint64_t)gridDim.x * (blockDim.x >> 5));
-  const uint32_t size = share >= 32 ? 32u : share >= 16 ? 16u : 8u;
+  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+  const uint64_t share = V.na / gwarps;
+  const uint32_t size = share >= 128 ? 32u : share >= 64 ? 16u : 8u;
   const uint64_t groups = (V.na + size - 1) / size;
+  const bool in_l2 = A.bit_words <= kRowsInL2 / 4;
+  uint64_t mine = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
   for (;;) {
-    unsigned long long g = 0;
-    if (lane_id() == 0) g = atomicAdd(cursor, 1ULL);
-    g = __shfl_sync(kFull, g, 0);
+    unsigned long long g = mine;
+    if (in_l2) {
+      mine += gwarps;
+    } else {
+      if (lane_id() == 0) g = atomicAdd(cursor, 1ULL);
+      g = __shfl_sync(kFull, g, 0);
+    }
     if (g >= groups) break;
     uint32_t e, sc;
     bool ok;
@@ -767,8 +762,13 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(Pee
         continue;
       }
       const uint32_t thr = A.gthr_max ? __ldcg(A.gthr_max) : V.thr;
+      // (Beyond short rows a factor of 2: decrements dealt one per lane cost
+      // half of what the option's scale was set for; 64 mix graphs in a batch
+      // 167.9 ms without it, 163.9 with 2, 165.4 with 5.  Counts over short rows
+      // are cheaper too: the Chung-Lu solve 18.0 ms without it, 18.2 with 2.)
+      const double scale = A.R.W <= kShortRow ? 1.0 : 2.0;
       const bool recount = A.R.bits && (double)nf * (double)(thr > 0 ? thr : 1) * (double)A.gamma >
-                                           (double)alive * (double)A.wavg;
+                                           scale * (double)alive * (double)A.wavg;
       pending += nf;
       if (recount) {
         ++nrec;
@@ -780,6 +780,8 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(Pee
           zero_bits(A, gtid, gthreads);
           if (!grid_barrier(A.words, A.timeout_ns)) return;
           set_alive_bits(A, V, gtid, gthreads);
+        } else if (cleared + 1 == r) {  // only this round's frontier to clear
+          for (uint64_t f = gtid; f < nf; f += gthreads) clear_edge_bits(A, fr[f]);
         } else {
           clear_deleted(A, V, cleared, r, gtid, gthreads);
         }
@@ -788,11 +790,16 @@ __global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(Pee
         if (!grid_barrier(A.words, A.timeout_ns)) return;
         recount_round(A, V, r, nx, nc, &A.cnt[6 + (nrec & 1)], trec, su);
       } else {
-        // Few frontier edges for the grid: deal (edge, chunk) units instead.
+        // Few frontier edges for the grid: deal (edge, chunk) units instead,
+        // in the shortest chunks that give every warp one unit at most (a
+        // chunk's common neighbours, up to 32 a word, are closed 32 at a time).
         const uint64_t chunks = A.R.sbits ? (A.R.W + kSplitWords - 1) / kSplitWords : 1;
-        if (chunks >= 2 && nf * chunks <= (uint64_t)A.split * gwarps)
-          split_round(A, V, fr, nf, chunks, r, nx, nc, gwarp, gwarps, tdeg, tdec);
-        else
+        if (A.R.sbits && A.R.W >= 2 && nf * chunks <= (uint64_t)A.split * gwarps) {
+          uint32_t cw = 1;
+          while (cw < kSplitWords && nf * ((A.R.W + cw - 1) / cw) > gwarps) cw *= 2;
+          split_round(A, V, fr, (uint32_t)nf, cw, (A.R.W + cw - 1) / cw, r, nx, nc, (uint32_t)gwarp,
+                      (uint32_t)gwarps, tdeg, tdec);
+        } else
           for (uint64_t f = gwarp; f < nf; f += gwarps) peel_edge(A, V, fr[f], r, nx, nc, tdeg, tdec);
       }
       if (gtid == 0) A.cnt[(i + 2) % 3] = 0;  // read at the start of round i-1, next written in round i+1
@@ -1167,7 +1174,7 @@ struct Peeler {
     A.bit_words = s->W ? s->bit_words : 0;
     A.gamma = (uint32_t)std::max<int64_t>(1, c->opt.recount_gamma);
     A.search_ratio = (uint32_t)std::min<int64_t>(std::max<int64_t>(1, c->opt.peel_search_ratio), 1 << 20);
-    A.split = (uint32_t)std::min<int64_t>(std::max<int64_t>(0, c->opt.peel_split), 1 << 20);
+    A.split = (uint32_t)std::min<int64_t>(std::max<int64_t>(0, c->opt.peel_split), 1 << 14);  // units fit 32 bits
     A.words = dev_words(c);
     A.timeout_ns = (unsigned long long)c->opt.timeout_ms * 1000000ULL;
     A.gthr = track ? gthr.as<uint32_t>() : nullptr;
