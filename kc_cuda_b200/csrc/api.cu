@@ -397,6 +397,8 @@ void kt_destroy(kt_ctx* h) {
     std::lock_guard<std::recursive_mutex> lk(h->c.mu);
     cudaSetDevice(h->c.device);
     h->c.words.release();
+    h->c.lb_status.release();
+    h->c.lb_ticket.release();
     if (h->c.stream) cudaStreamSynchronize(h->c.stream);
     for (auto& e : h->c.ev)
       if (e) cudaEventDestroy(e);

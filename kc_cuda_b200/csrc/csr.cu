@@ -219,12 +219,6 @@ __global__ void k_unpack(uint64_t* __restrict__ keys, uint64_t n, int vb) {
   }
 }
 
-int bits_for(uint64_t n) {
-  int b = 0;
-  while ((1ULL << b) < n) ++b;
-  return b;
-}
-
 // The grouped-input route; false (g and keys untouched) when the records
 // are not in that form.
 bool build_graph_grouped(Ctx* c, const uint64_t* keys, uint64_t nk, uint64_t n, Graph& g) {
@@ -263,7 +257,7 @@ bool build_graph_grouped(Ctx* c, const uint64_t* keys, uint64_t nk, uint64_t n, 
   up.release();
   eoff.release();
   // Sorted by x, the high half (stable: y stays ascending within each x).
-  radix_sort_u64(c, low.as<uint64_t>(), nullptr, m, 32 + bits_for(n), 32);
+  radix_sort_u64(c, low.as<uint64_t>(), nullptr, m, {{32, 32 + bits_for(n)}});
   k_equal_u64<<<grid_for(m, 256, c->num_sms * 16), 256, 0, c->stream>>>(low.as<uint64_t>(), edges.as<uint64_t>(),
                                                                           m, flags.as<uint32_t>());
   KT_LAUNCHED(c);
@@ -327,9 +321,8 @@ void build_graph_sorted(Ctx* c, uint64_t* keys, uint64_t nkeys, uint64_t n, Grap
     g.m = nkeys;
   } else {
     // Keys are min << 32 | max with both halves below 2^vb - 1; the radix sort
-    // skips digits shared by every key, so it runs 2 ceil(vb / 8) passes once
-    // the "no edge" key ~0 is rewritten to ((2^vb - 1) << 32) | (2^vb - 1)
-    // (still last).  When packing to min << vb | max saves a pass (2 vb bits,
+    // runs 2 ceil(vb / 8) passes over the two halves' bits once the "no edge"
+    // key ~0 is rewritten to ((2^vb - 1) << 32) | (2^vb - 1) (still last).  When packing to min << vb | max saves a pass (2 vb bits,
     // ceil(2 vb / 8) passes), the keys are packed instead.
     const int vb = bits_for(n + 1);
     const bool small = vb < 32 && nkeys;
@@ -344,7 +337,10 @@ void build_graph_sorted(Ctx* c, uint64_t* keys, uint64_t nkeys, uint64_t n, Grap
                                                                                    small ? sentinel : ~0ULL);
       KT_LAUNCHED(c);
     }
-    if (nkeys > 1) radix_sort_u64(c, keys, nullptr, nkeys, 64);
+    if (pack)
+      radix_sort_u64(c, keys, nullptr, nkeys, {{0, 2 * vb}});
+    else
+      radix_sort_u64(c, keys, nullptr, nkeys, {{0, vb}, {32, 32 + vb}});
     if (pack) {
       k_unpack<<<grid_for(nkeys, 256, c->num_sms * 16), 256, 0, c->stream>>>(keys, nkeys, vb);
       KT_LAUNCHED(c);

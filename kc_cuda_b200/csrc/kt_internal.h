@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -181,6 +182,11 @@ struct Ctx {
   // Pinned host words (kPinnedBytes) for small device-to-host reads.
   uint64_t* pinned = nullptr;
   cudaEvent_t ev[8] = {};
+  // Look-back words of the scans and compactions (scan.cu): a status word per
+  // tile, the ticket (and a launch's total), the tiles and the launches so far.
+  DBuf lb_status, lb_ticket;
+  uint64_t lb_tickets = 0;
+  uint32_t lb_epoch = 0;
   // Device word block: bounded-wait error flag, barrier state, counters.
   DBuf words;
   EventTimer timer;
@@ -233,15 +239,24 @@ void zero(Ctx* c, void* dptr, size_t bytes);
 // Device-wide primitives (scan.cu, sort.cu).
 // Exclusive scan of n uint32 values into uint64 (out may not alias in).
 void scan_u32_to_u64(Ctx* c, const uint32_t* in, uint64_t* out, uint64_t n);
-// Exclusive scan of n uint32 values in place-safe form into uint32 (out may alias in).
+// Exclusive scan of n uint32 values into uint32 (out may alias in).
 void scan_u32(Ctx* c, const uint32_t* in, uint32_t* out, uint64_t n);
 // Sum of n uint32 values (device result in *dsum, also returned).
 uint64_t reduce_u32(Ctx* c, const uint32_t* in, uint64_t n);
-// Stable LSD radix sort of keys (and optional uint32 values) by their bits
-// [lo_bit, bits) (8-bit digits from lo_bit up; a digit may also read bits at
-// or above `bits`, which must then be equal in every key).  `keys`/`vals`
-// hold the input and receive the output.
-void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, int bits, int lo_bit = 0);
+// Bits [lo, hi) of a key.
+struct BitField {
+  int lo, hi;
+};
+// Stable LSD radix sort of keys (and optional uint32 values) by the given
+// fields (the least significant first); bits outside them do not count.
+// `keys`/`vals` hold the input and receive the output.
+void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::initializer_list<BitField> fields);
+// Bits that hold every value below n.
+inline int bits_for(uint64_t n) {
+  int b = 0;
+  while (b < 64 && (1ULL << b) < n) ++b;
+  return b;
+}
 // Sorted-unique compaction of keys (drops key == ~0).  Returns new count.
 uint64_t unique_sorted_u64(Ctx* c, const uint64_t* in, uint64_t* out, uint64_t n);
 

@@ -1,42 +1,49 @@
 // Device-wide scans, reductions and the sorted-unique compaction.
 //
-// Scans are reduce-then-scan over tiles of 2048 items (256 threads x 8): a
-// tile-sum kernel, a recursive scan of the tile sums, and a tile-scan kernel
-// that adds the tile's prefix.  Tiles are staged through shared memory so
-// every global access is coalesced.
+// Scans and compactions (compact.cuh) take one pass over the data in one
+// launch: tiles of 2048 items (256 threads x 8) find their prefix by decoupled
+// look-back.  (Tile sums, a recursive scan of those and a second pass over the
+// data took three to seven launches, most of the small kernels of a solve:
+// R-MAT scale 10, 1.65 -> 1.37 ms with one.)
+#include "compact.cuh"
 #include "kt_device.cuh"
 #include "kt_internal.h"
+#include "lookback.cuh"
 
 namespace kt {
+
+// The context's look-back words for one launch of `tiles` tiles.
+Lookback begin_lookback(Ctx* c, uint64_t tiles) {
+  if (!c->lb_ticket.get()) {
+    c->lb_ticket.alloc(c, 2 * sizeof(unsigned long long));  // the ticket, and a launch's total
+    zero(c, c->lb_ticket.get(), c->lb_ticket.bytes());
+    c->lb_tickets = 0;
+  }
+  if (c->lb_status.bytes() < tiles * sizeof(unsigned long long) || ++c->lb_epoch >= kEpochs) {
+    c->lb_status.ensure(c, std::max<uint64_t>(tiles, 1 << 12) * sizeof(unsigned long long));
+    zero(c, c->lb_status.get(), c->lb_status.bytes());
+    c->lb_epoch = 1;
+  }
+  return Lookback{c->lb_status.as<unsigned long long>(), c->lb_ticket.as<unsigned long long>(), c->lb_tickets,
+                  c->lb_epoch, &dev_words(c)->err};
+}
+void end_lookback(Ctx* c, uint64_t tiles) { c->lb_tickets += tiles; }
+
 namespace {
 
 constexpr unsigned kScanThreads = 256;
 constexpr unsigned kScanItems = 8;
 constexpr unsigned kScanTile = kScanThreads * kScanItems;
 
+// Exclusive scan.  In-place safe: a tile is read before any of it is written.
 template <typename Tin, typename Tout>
-__global__ void __launch_bounds__(kScanThreads) k_tile_sum(const Tin* __restrict__ in, uint64_t n,
-                                                           Tout* __restrict__ sums) {
-  __shared__ Tout tmp[33];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-  Tout s = 0;
-#pragma unroll
-  for (unsigned i = 0; i < kScanItems; ++i) {
-    const uint64_t j = base + i * kScanThreads + threadIdx.x;
-    if (j < n) s += (Tout)in[j];
-  }
-  s = block_sum<Tout>(s, tmp);
-  if (threadIdx.x == 0) sums[blockIdx.x] = s;
-}
-
-// Exclusive scan of one tile plus an optional per-tile prefix.  In-place safe:
-// the whole tile is read before any of it is written.
-template <typename Tin, typename Tout>
-__global__ void __launch_bounds__(kScanThreads) k_tile_scan(const Tin* in, Tout* out, uint64_t n,
-                                                            const Tout* __restrict__ prefix) {
+__global__ void __launch_bounds__(kScanThreads) k_scan(const Tin* in, Tout* out, uint64_t n, Lookback L) {
   __shared__ Tout stage[kScanTile];
   __shared__ Tout tmp[33];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
+  __shared__ unsigned long long sh[2];
+  const uint64_t tile = gridDim.x > 1 ? take_tile(L, &sh[0]) : 0;
+  if (tile >= gridDim.x) return;
+  const uint64_t base = tile * kScanTile;
 #pragma unroll
   for (unsigned i = 0; i < kScanItems; ++i) {
     const uint64_t j = base + i * kScanThreads + threadIdx.x;
@@ -52,7 +59,17 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const Tin* in, Tout*
   }
   Tout total;
   const Tout excl = block_excl_scan<Tout>(run, tmp, &total);
-  const Tout off = (prefix ? prefix[blockIdx.x] : Tout(0)) + excl;
+  bool ok = true;
+  if (gridDim.x > 1) {
+    if (warp_id() == 0) {
+      const unsigned long long p = tile_prefix(L, tile, (unsigned long long)total, &ok);
+      if (lane_id() == 0) sh[1] = p;
+    }
+  } else if (threadIdx.x == 0) {
+    sh[1] = 0;
+  }
+  if (!__syncthreads_and(ok)) return;
+  const Tout off = (Tout)sh[1] + excl;
 #pragma unroll
   for (unsigned i = 0; i < kScanItems; ++i) stage[threadIdx.x * kScanItems + i] = v[i] + off;
   __syncthreads();
@@ -68,17 +85,10 @@ void scan_impl(Ctx* c, const Tin* in, Tout* out, uint64_t n) {
   if (n == 0) return;
   const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
   if (tiles > 0x7fffffffULL) throw Error(KT_ERR_LIMIT, "scan: too many tiles");
-  if (tiles == 1) {
-    k_tile_scan<Tin, Tout><<<1, kScanThreads, 0, c->stream>>>(in, out, n, nullptr);
-    KT_LAUNCHED(c);
-    return;
-  }
-  DBuf sums(c, tiles * sizeof(Tout));
-  k_tile_sum<Tin, Tout><<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, n, sums.as<Tout>());
+  const Lookback L = tiles > 1 ? begin_lookback(c, tiles) : Lookback{};
+  k_scan<Tin, Tout><<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, out, n, L);
   KT_LAUNCHED(c);
-  scan_impl<Tout, Tout>(c, sums.as<Tout>(), sums.as<Tout>(), tiles);
-  k_tile_scan<Tin, Tout><<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, out, n, sums.as<Tout>());
-  KT_LAUNCHED(c);
+  if (tiles > 1) end_lookback(c, tiles);
 }
 
 __global__ void k_reduce_u32(const uint32_t* __restrict__ in, uint64_t n, unsigned long long* out) {
@@ -90,52 +100,20 @@ __global__ void k_reduce_u32(const uint32_t* __restrict__ in, uint64_t n, unsign
   if (threadIdx.x == 0 && s) atomicAdd(out, (unsigned long long)s);
 }
 
-// ---- sorted unique: count kept keys per tile, scan, then write them.
-__device__ __forceinline__ bool keep_key(const uint64_t* in, uint64_t j) {
-  const uint64_t k = in[j];
-  return k != ~0ULL && (j == 0 || in[j - 1] != k);
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_unique_count(const uint64_t* __restrict__ in, uint64_t n,
-                                                               uint64_t* __restrict__ counts) {
-  __shared__ uint64_t tmp[33];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-  uint64_t s = 0;
-#pragma unroll
-  for (unsigned i = 0; i < kScanItems; ++i) {
-    const uint64_t j = base + i * kScanThreads + threadIdx.x;
-    if (j < n) s += keep_key(in, j);
+// Distinct keys of a sorted list, ~0 dropped.
+struct DistinctKey {
+  const uint64_t* in;
+  __device__ bool keep(uint64_t j) const {
+    const uint64_t k = in[j];
+    return k != ~0ULL && (j == 0 || in[j - 1] != k);
   }
-  s = block_sum<uint64_t>(s, tmp);
-  if (threadIdx.x == 0) counts[blockIdx.x] = s;
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_unique_write(const uint64_t* __restrict__ in, uint64_t n,
-                                                               const uint64_t* __restrict__ offs,
-                                                               uint64_t* __restrict__ out) {
-  __shared__ uint64_t tmp[33];
-  const uint64_t base = (uint64_t)blockIdx.x * kScanTile;
-  // Blocked ownership keeps the output in input order.
-  uint32_t flags = 0;
-  uint64_t keys[kScanItems];
-#pragma unroll
-  for (unsigned i = 0; i < kScanItems; ++i) {
-    const uint64_t j = base + threadIdx.x * kScanItems + i;
-    keys[i] = j < n ? in[j] : ~0ULL;
-    if (j < n && keep_key(in, j)) flags |= 1u << i;
-  }
-  uint64_t total;
-  uint64_t pos = offs[blockIdx.x] + block_excl_scan<uint64_t>((uint64_t)__popc(flags), tmp, &total);
-#pragma unroll
-  for (unsigned i = 0; i < kScanItems; ++i)
-    if (flags & (1u << i)) out[pos++] = keys[i];
-}
+  __device__ uint64_t value(uint64_t j) const { return in[j]; }
+};
 
 }  // namespace
 
-void scan_u32_to_u64(Ctx* c, const uint32_t* in, uint64_t* out, uint64_t n) { scan_impl<uint32_t, uint64_t>(c, in, out, n); }
 void scan_u32(Ctx* c, const uint32_t* in, uint32_t* out, uint64_t n) { scan_impl<uint32_t, uint32_t>(c, in, out, n); }
-void scan_u64(Ctx* c, const uint64_t* in, uint64_t* out, uint64_t n) { scan_impl<uint64_t, uint64_t>(c, in, out, n); }
+void scan_u32_to_u64(Ctx* c, const uint32_t* in, uint64_t* out, uint64_t n) { scan_impl<uint32_t, uint64_t>(c, in, out, n); }
 
 uint64_t reduce_u32(Ctx* c, const uint32_t* in, uint64_t n) {
   DBuf acc(c, 8);
@@ -148,17 +126,7 @@ uint64_t reduce_u32(Ctx* c, const uint32_t* in, uint64_t n) {
 }
 
 uint64_t unique_sorted_u64(Ctx* c, const uint64_t* in, uint64_t* out, uint64_t n) {
-  if (n == 0) return 0;
-  const uint64_t tiles = (n + kScanTile - 1) / kScanTile;
-  DBuf counts(c, (tiles + 1) * sizeof(uint64_t));
-  k_unique_count<<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, n, counts.as<uint64_t>());
-  KT_LAUNCHED(c);
-  // counts[tiles] = 0 so the exclusive scan's last slot is the total.
-  zero(c, counts.as<uint64_t>() + tiles, sizeof(uint64_t));
-  scan_u64(c, counts.as<uint64_t>(), counts.as<uint64_t>(), tiles + 1);
-  k_unique_write<<<(unsigned)tiles, kScanThreads, 0, c->stream>>>(in, n, counts.as<uint64_t>(), out);
-  KT_LAUNCHED(c);
-  return read_word<uint64_t>(c, counts.as<uint64_t>() + tiles);
+  return compact(c, n, DistinctKey{in}, out);
 }
 
 }  // namespace kt

@@ -5,8 +5,6 @@
 
 namespace kt {
 
-void scan_u64(Ctx* c, const uint64_t* in, uint64_t* out, uint64_t n);
-
 // parse.cu -- stage (a)
 uint64_t parse_padded_bytes(uint64_t len);
 // Bytes per parse block; a chunk of the input for the pipelined ingest is a

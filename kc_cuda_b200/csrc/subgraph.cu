@@ -211,7 +211,14 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
   k_order_keys<<<grid_for(na, 256, c->num_sms * 16), 256, 0, c->stream>>>(alive, na, deg, group_of,
                                                                              okeys.as<uint64_t>());
   KT_LAUNCHED(c);
-  radix_sort_u64(c, okeys.as<uint64_t>(), nullptr, na, 64);
+  if (group_of)
+    radix_sort_u64(c, okeys.as<uint64_t>(), nullptr, na,
+                   {{0, bits_for(g.n)},
+                    {28, 28 + bits_for(std::min<uint64_t>((uint64_t)g.max_deg + 1, 1u << 20))},
+                    {48, 48 + bits_for(ngroups)}});
+  else
+    radix_sort_u64(c, okeys.as<uint64_t>(), nullptr, na,
+                   {{0, bits_for(g.n)}, {32, 32 + bits_for((uint64_t)g.max_deg + 1)}});
   DBuf newid(c, (g.n ? g.n : 1) * sizeof(uint32_t));
   DBuf sdeg(c, (na + 1) * sizeof(uint32_t));
   zero(c, sdeg.get(), (na + 1) * sizeof(uint32_t));
@@ -280,8 +287,9 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
     copy_rows(c, s.orig.as<uint32_t>(), na, g.off.as<uint64_t>(), g.adj.as<uint32_t>(), rem, newid.as<uint32_t>(),
               s.off.as<uint64_t>(), g.max_deg, OutKey{keys.as<uint64_t>()});
     newid.release();
-    // Row in bits 32.., column in bits 0..: constant digits are skipped.
-    radix_sort_u64(c, keys.as<uint64_t>(), nullptr, n2, 64);
+    // Row in bits 32.., column in bits 0...
+    const int vb = bits_for(na);
+    radix_sort_u64(c, keys.as<uint64_t>(), nullptr, n2, {{0, vb}, {32, 32 + vb}});
     if (n2) {
       k_rows_from_keys<<<grid_for(n2, 256, c->num_sms * 16), 256, 0, c->stream>>>(keys.as<uint64_t>(), n2,
                                                                                     s.adj.as<uint32_t>());

@@ -533,7 +533,8 @@ bool build_bits(Ctx* c, Sub& s) {
                                                                             keys.as<uint64_t>(),
                                                                             s.order.as<uint32_t>());
   KT_LAUNCHED(c);
-  radix_sort_u64(c, keys.as<uint64_t>(), s.order.as<uint32_t>(), s.m, 32);
+  const int blocks_bits = bits_for(((uint64_t)(s.n - 1) >> tb) + 1);
+  radix_sort_u64(c, keys.as<uint64_t>(), s.order.as<uint32_t>(), s.m, {{0, blocks_bits}, {16, 16 + blocks_bits}});
   return true;
 }
 
