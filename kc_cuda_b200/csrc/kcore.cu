@@ -318,6 +318,12 @@ __device__ __forceinline__ void walk_rows(const uint32_t* front, uint64_t nf,
   }
 }
 
+// Threads of the cooperative kernels here, two blocks per SM: a barrier of 296
+// blocks takes 1.6 us, of 592 blocks of 256 threads 2.3 (core decomposition of
+// a 400,009-id R-MAT graph 4.94 -> 4.75 ms; one block of 1024 threads, which
+// waits longer for its own warps, 5.10).
+constexpr unsigned kCoreThreads = 512;
+
 // What the search leaves for the host.
 constexpr uint32_t kMaxProbes = 64;  // probes of one launch
 struct SearchOut {
@@ -360,7 +366,7 @@ struct SearchArgs {
 // atomics of all N are in flight before any result is used.
 template <unsigned N>
 __device__ __forceinline__ void drop_entries(const SearchArgs& A, const uint32_t (&w)[N], const bool (&ok)[N],
-                                             uint32_t k, uint32_t tag, uint32_t* next, unsigned long long* ncnt) {
+                                             uint32_t k, uint32_t tag, WarpList& next) {
   bool live[N];
 #pragma unroll
   for (unsigned t = 0; t < N; ++t) live[t] = ok[t] && A.rem[w[t]] == kAlive;
@@ -371,7 +377,7 @@ __device__ __forceinline__ void drop_entries(const SearchArgs& A, const uint32_t
   for (unsigned t = 0; t < N; ++t) {
     const bool want = live[t] && old[t] == k;
     if (want) A.rem[w[t]] = tag;
-    push_warp(want, w[t], next, ncnt, A.cap, &A.words->err);
+    next.push(want, w[t]);
   }
 }
 
@@ -383,7 +389,8 @@ __device__ __forceinline__ void drop_entries(const SearchArgs& A, const uint32_t
 // finds the least degree and the sum of the degrees.  With a launch per probe
 // the host's reads and the launches between two probes cost 70 us of the 100
 // us that a probe took on graphs of up to a million edges.
-__global__ void __launch_bounds__(256, 4) k_core_search(SearchArgs A) {
+__global__ void __launch_bounds__(kCoreThreads, 2) k_core_search(SearchArgs A) {
+  __shared__ uint32_t items[kCoreThreads / 32][WarpList::kEntries];
   __shared__ uint64_t woff[kBigBatch + 1];
   __shared__ uint64_t wtmp[33];
   __shared__ unsigned long long sh[2];
@@ -413,6 +420,7 @@ __global__ void __launch_bounds__(256, 4) k_core_search(SearchArgs A) {
       A.cnt[6] = 0;
     }
     const uint32_t* alive = A.alive[list];
+    WarpList first(items[warp_id()], (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap, &A.words->err);
     for (uint64_t j = gtid; j < ((na + 31) & ~31ULL); j += gthreads) {
       bool want = false;
       uint32_t v = 0;
@@ -432,8 +440,9 @@ __global__ void __launch_bounds__(256, 4) k_core_search(SearchArgs A) {
           want = true;
         }
       }
-      push_warp(want, v, (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap, &A.words->err);
+      first.push(want, v);
     }
+    first.flush();
     undo = false;
     ++i;
     src[0] = &A.cnt[i % 3];
@@ -455,10 +464,11 @@ __global__ void __launch_bounds__(256, 4) k_core_search(SearchArgs A) {
       uint32_t* nx = A.front[(i + 1) & 1];
       unsigned long long* nc = &A.cnt[(i + 1) % 3];
       unsigned long long* bc = &A.cnt[3 + (i & 1)];
-      walk_rows(fr, nf, A.off, A.adj, A.big_row, A.big, bc, A.cap, &A.words->err,
-                [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) {
-                  drop_entries<kWide>(A, w, ok, k, tag, nx, nc);
-                });
+      WarpList next(items[warp_id()], nx, nc, A.cap, &A.words->err);
+      walk_rows(
+          fr, nf, A.off, A.adj, A.big_row, A.big, bc, A.cap, &A.words->err,
+          [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) { drop_entries<kWide>(A, w, ok, k, tag, next); });
+      next.flush();
       if (gtid == 0) {
         A.cnt[(i + 2) % 3] = 0;        // read at the start of round i-1
         A.cnt[3 + ((i + 1) & 1)] = 0;  // big count of round i-1, read before the barrier ending it
@@ -480,8 +490,9 @@ __global__ void __launch_bounds__(256, 4) k_core_search(SearchArgs A) {
                 ok[t] = j < e;
                 w[t] = ok[t] ? A.adj[j] : 0u;
               }
-              drop_entries<8>(A, w, ok, k, tag, nx, nc);
+              drop_entries<8>(A, w, ok, k, tag, next);
             });
+        next.flush();
         if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       }
       ++i;
@@ -613,17 +624,9 @@ struct DecompArgs {
   unsigned long long timeout_ns;
 };
 
-struct DropRule {
-  uint32_t k, top;
-  uint32_t* next;              // frontier of the next round
-  unsigned long long* ncnt;
-  uint32_t* cand;              // candidates of this pass
-  unsigned long long* ccnt;
-};
-
 template <unsigned N>
 __device__ __forceinline__ void drop_entries_core(const DecompArgs& A, const uint32_t (&w)[N], const bool (&ok)[N],
-                                                  const DropRule& R) {
+                                                  uint32_t k, uint32_t top, WarpList& next, WarpList& cand) {
   bool live[N];
 #pragma unroll
   for (unsigned t = 0; t < N; ++t) live[t] = ok[t] && A.rem[w[t]] == kAlive;
@@ -632,19 +635,20 @@ __device__ __forceinline__ void drop_entries_core(const DecompArgs& A, const uin
   for (unsigned t = 0; t < N; ++t) old[t] = live[t] ? atomicSub(&A.deg[w[t]], 1u) : 0u;
 #pragma unroll
   for (unsigned t = 0; t < N; ++t) {
-    const bool want = live[t] && old[t] == R.k + 1;
-    const bool join = live[t] && !want && old[t] == R.top + 1;  // its degree entered the window
+    const bool want = live[t] && old[t] == k + 1;
+    const bool join = live[t] && !want && old[t] == top + 1;  // its degree entered the window
     if (want) {
       A.rem[w[t]] = 0u;
-      A.core[w[t]] = R.k;
+      A.core[w[t]] = k;
     }
-    push_warp(want, w[t], R.next, R.ncnt, A.cap, &A.words->err);
-    push_warp(join, w[t], R.cand, R.ccnt, A.cap, &A.words->err);
+    next.push(want, w[t]);
+    cand.push(join, w[t]);
   }
 }
 
-__global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
+__global__ void __launch_bounds__(kCoreThreads, 2) k_core_levels(DecompArgs A) {
   __shared__ unsigned long long sh[4];
+  __shared__ uint32_t items[3][kCoreThreads / 32][WarpList::kEntries];
   __shared__ uint64_t woff[kBigBatch + 1];
   __shared__ uint64_t wtmp[33];
   const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
@@ -682,6 +686,10 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
     uint32_t* lnext = li ? A.list[0] : A.list[1];
     uint32_t* cnext = ci ? A.cand[0] : A.cand[1];
     uint32_t mn = 0xffffffffu;
+    WarpList cands(items[1][warp_id()], cnext, cc, A.cap, &A.words->err);
+    WarpList leaving(items[0][warp_id()], (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap,
+                     &A.words->err);
+    WarpList staying(items[2][warp_id()], lnext, lc, A.cap, &A.words->err);
     for (uint64_t j = gtid; j < ((nsrc + 31) & ~31ULL); j += gthreads) {
       bool out = false, keep = false, cand = false;
       uint32_t v = 0;
@@ -700,10 +708,13 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
           }
         }
       }
-      push_warp(out, v, (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap, &A.words->err);
-      if (full) push_warp(keep, v, lnext, lc, A.cap, &A.words->err);
-      push_warp(cand, v, cnext, cc, A.cap, &A.words->err);
+      leaving.push(out, v);
+      if (full) staying.push(keep, v);
+      cands.push(cand, v);
     }
+    leaving.flush();
+    staying.flush();
+    cands.flush();
     mn = warp_min(mn);
     if (lane_id() == 0 && mn != 0xffffffffu) atomicMin(mc, (unsigned long long)mn);
     {
@@ -737,19 +748,22 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
     }
     ++levels_run;
     // Frontier rounds of level k.
-    DropRule R{k, top, nullptr, nullptr, cnext, cc};
     while (nf) {
       const uint32_t* fr = (i & 1) ? A.front[1] : A.front[0];
-      R.next = (i & 1) ? A.front[0] : A.front[1];
-      R.ncnt = &A.cnt[(i + 1) % 3];
+      WarpList next(items[0][warp_id()], (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap,
+                    &A.words->err);
       unsigned long long* bc = &A.cnt[3 + (i & 1)];
       walk_rows(fr, nf, A.off, A.adj, A.big_row, A.big, bc, A.cap, &A.words->err,
-                [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) { drop_entries_core<kWide>(A, w, ok, R); });
+                [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) {
+                  drop_entries_core<kWide>(A, w, ok, k, top, next, cands);
+                });
+      next.flush();
+      cands.flush();
       if (gtid == 0) {
         A.cnt[(i + 2) % 3] = 0;
         A.cnt[3 + ((i + 1) & 1)] = 0;
       }
-      const unsigned long long* const src[3] = {R.ncnt, bc, cc};
+      const unsigned long long* const src[3] = {next.cnt, bc, cc};
       if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       const uint64_t nbig = sh[1];
       if (nbig) {
@@ -763,8 +777,10 @@ __global__ void __launch_bounds__(256, 4) k_core_levels(DecompArgs A) {
                 ok[t] = j < e;
                 w[t] = ok[t] ? A.adj[j] : 0u;
               }
-              drop_entries_core<4>(A, w, ok, R);
+              drop_entries_core<4>(A, w, ok, k, top, next, cands);
             });
+        next.flush();
+        cands.flush();
         if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
       }
       nf = sh[0];
@@ -902,7 +918,7 @@ void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixe
   out.ensure(c, sizeof(SearchOut));
   if (!coop_grid) {
     int per_sm = 0;
-    KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_search, 256, 0));
+    KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_search, kCoreThreads, 0));
     coop_grid = std::min(coop_blocks(c, per_sm), kMaxGrid);
   }
   SearchArgs A;
@@ -935,8 +951,8 @@ void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixe
   SearchOut& h = *static_cast<SearchOut*>(result);
   {
     CoopLock coop(c);
-    const unsigned grid = coop_blocks_for(coop_grid, 2 * g.m, 8 * 32 * kWide);
-    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_search, dim3(grid), dim3(256), p, 0, c->stream));
+    const unsigned grid = coop_blocks_for(coop_grid, 2 * g.m, kCoreThreads * kWide);
+    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_search, dim3(grid), dim3(kCoreThreads), p, 0, c->stream));
     KT_LAUNCHED(c);
     read_checked(c, &h, out.get(), sizeof(SearchOut), "k-core probe");
   }
@@ -1219,14 +1235,15 @@ void KCore::core_numbers_persistent(Ctx* c, uint32_t* dcore) {
   A.words = dev_words(c);
   A.timeout_ns = (unsigned long long)c->opt.timeout_ms * 1000000ULL;
   int per_sm = 0;
-  KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_levels, 256, 0));
+  KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_core_levels, kCoreThreads, 0));
   if (c->opt.kcore_blocks_per_sm > 0) per_sm = (int)std::min<int64_t>(per_sm, c->opt.kcore_blocks_per_sm);
-  const unsigned grid = coop_blocks_for(coop_blocks(c, per_sm), 2 * g.m, 8 * 32 * kWide);
+  const unsigned grid = coop_blocks_for(coop_blocks(c, per_sm), 2 * g.m, kCoreThreads * kWide);
   void* p[] = {&A};
   uint64_t h[5];
   {
     CoopLock coop(c);
-    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_levels, dim3(grid), dim3(256), p, 0, c->stream));
+    KT_CUDA(cudaLaunchCooperativeKernel((const void*)k_core_levels, dim3(grid), dim3(kCoreThreads), p, 0,
+                                        c->stream));
     KT_LAUNCHED(c);
     copy_d2h(c, h, cn.as<unsigned long long>() + 14, sizeof(h));
   }

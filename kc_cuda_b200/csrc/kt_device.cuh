@@ -79,6 +79,46 @@ __device__ __forceinline__ T warp_max(T v) {
   }
   return v;
 }
+// Items that a warp appends to a device list, gathered in its 64 entries of
+// shared memory and appended 33 to 64 at a time (flush() appends the rest):
+// the list's counter is one word for the whole grid, and an atomic for every
+// step in which a lane has an item made warps wait for it, and for each other.
+// Every method is called by the whole warp; an item past `cap` flags
+// kDevErrCapacity.
+struct WarpList {
+  static constexpr uint32_t kEntries = 64;
+  uint32_t* buf;
+  uint32_t* list;
+  unsigned long long* cnt;
+  uint64_t cap;
+  uint32_t* err;
+  uint32_t n = 0;
+  __device__ __forceinline__ WarpList(uint32_t* b, uint32_t* l, unsigned long long* c, uint64_t most, uint32_t* e)
+      : buf(b), list(l), cnt(c), cap(most), err(e) {}
+  __device__ __forceinline__ void push(bool want, uint32_t item) {
+    const unsigned b = __ballot_sync(kFull, want);
+    if (!b) return;
+    if (n + __popc(b) > kEntries) flush();
+    if (want) buf[n + __popc(b & lanemask_lt())] = item;
+    n += __popc(b);
+  }
+  __device__ __forceinline__ void flush() {
+    if (n == 0) return;
+    __syncwarp();
+    unsigned long long base = 0;
+    if (lane_id() == 0) base = atomicAdd(cnt, (unsigned long long)n);
+    base = __shfl_sync(kFull, base, 0);
+    for (uint32_t i = lane_id(); i < n; i += 32) {
+      if (base + i < cap)
+        list[base + i] = buf[i];
+      else
+        atomicOr(err, kDevErrCapacity);
+    }
+    __syncwarp();
+    n = 0;
+  }
+};
+
 // Inclusive warp scan.
 template <typename T>
 __device__ __forceinline__ T warp_incl_scan(T v) {

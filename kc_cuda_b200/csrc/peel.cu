@@ -48,7 +48,8 @@
 namespace kt {
 namespace {
 
-constexpr unsigned kPeelThreads = 256;
+constexpr unsigned kPeelThreads = 256;   // host-stepped rounds
+constexpr unsigned kLevelThreads = 512;  // k_levels, or fewer where the rows' shared memory wants it
 constexpr unsigned kCounters = 16;   // device counters before the blocks' kept counts
 constexpr unsigned kMaxGrid = 4096;  // blocks of a cooperative launch at most (one count per block is kept)
 
@@ -575,6 +576,10 @@ __device__ __forceinline__ void clear_deleted(const PeelArgs& A, const Level& V,
   }
 }
 
+// Shared memory of a k_levels block's rows at most (its static arrays and the
+// block's reserve take some of the 227 KB).
+constexpr size_t kRowsSmem = 200 << 10;
+
 constexpr uint64_t kRowsInL2 = 64u << 20;  // bytes of bitset rows that stay in L2 beside the rest
 
 // Dense recount round r: every surviving edge gets its exact support in the
@@ -686,12 +691,11 @@ __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcn
 // removes a few edges took 105 us (a core of 1,311 vertices, 609,432 edges), now
 // 43 us.  Dense mode uses W words of shared memory per warp for the recount
 // rounds.
-// Resident blocks per SM the register allocation aims at (a build constant).
-#ifndef KT_PEEL_MIN_BLOCKS
-#define KT_PEEL_MIN_BLOCKS 4
-#endif
+// Two blocks of 512 threads per SM: a barrier of 296 blocks takes 1.6 us, of 592
+// blocks of 256 threads 2.3 (64 mix graphs: 29.6 -> 29.1 ms of levels; one
+// block of 1024 threads waits longer for its own warps on small graphs).
 template <bool kLists>
-__global__ void __launch_bounds__(kPeelThreads, KT_PEEL_MIN_BLOCKS) k_levels(PeelArgs A, LevelsArgs L) {
+__global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsArgs L) {
   extern __shared__ __align__(16) uint32_t dense_smem[];
   __shared__ uint64_t woff[kLists ? kBigBatch + 1 : 1];
   __shared__ unsigned long long sh[3];
@@ -1087,6 +1091,7 @@ struct Peeler {
   uint32_t r = 1;  // next round number
   uint64_t fail_below = 0;  // set while a level is tried from a snapshot (PeelArgs::fail_below)
   unsigned coop_grid = 0;
+  unsigned threads = kLevelThreads;  // of a k_levels block
   size_t smem = 0;
   PeelResult* res;
 
@@ -1114,15 +1119,18 @@ struct Peeler {
                               c->stream));
     KT_LAUNCHED(c);
     na = m;
-    smem = s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, kPeelThreads);
+    threads = kLevelThreads;
+    auto rows_smem = [&] { return s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, threads); };
+    while (threads > 256 && rows_smem() > kRowsSmem) threads /= 2;
+    smem = rows_smem();
     coop_grid = 0;
     build_table();
     if (c->opt.persistent || s->W) {
       allow_max_dynamic_smem(kernel());
       int per_sm = 0;
-      KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(), kPeelThreads, smem));
+      KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(), (int)threads, smem));
       // A warp counts eight edges at once, or looks up kJobWide entries a lane.
-      coop_grid = coop_blocks_for(std::min(coop_blocks(c, per_sm), kMaxGrid), s->m, 64);
+      coop_grid = coop_blocks_for(std::min(coop_blocks(c, per_sm), kMaxGrid), s->m, threads / 4);
     }
   }
 
@@ -1226,7 +1234,7 @@ struct Peeler {
     {
       CoopLock coop(c);
       void* p[] = {&A, &L};
-      KT_CUDA(cudaLaunchCooperativeKernel(kernel(), dim3(coop_grid), dim3(kPeelThreads), p, smem,
+      KT_CUDA(cudaLaunchCooperativeKernel(kernel(), dim3(coop_grid), dim3(threads), p, smem,
                                           c->stream));
       KT_LAUNCHED(c);
       c->timer.end(c->stream, e0, &c->stats.ms_peel_kernel);

@@ -16,23 +16,24 @@ constexpr unsigned kBigBatch = 1024;  // long rows per batch of dealt windows
 // (the same block scan in every block, kBigBatch rows at a time) and warp w
 // takes windows w, w + warps, ...; `drop(i, b, e)` handles entries [b, e) (at
 // most kWin) of row(i).  Every thread of the block must call it (it
-// synchronises the block); blocks have 256 threads.
+// synchronises the block); blocks have 256, 512 or 1024 threads.
 template <unsigned kWin, class Row, class Drop>
 __device__ __forceinline__ void deal_windows(uint64_t nbig, Row row, const uint64_t* __restrict__ off, uint64_t* woff,
                                              uint64_t* tmp, Drop drop) {
   const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
-  constexpr unsigned per = kBigBatch / 256;  // rows per thread
+  constexpr unsigned kMost = kBigBatch / 256;
+  const unsigned per = kBigBatch / blockDim.x;  // rows per thread
   for (uint64_t base = 0; base < nbig; base += kBigBatch) {
     const uint64_t left = nbig - base;
     const uint32_t cnt = left < kBigBatch ? (uint32_t)left : kBigBatch;
-    uint64_t w[per];
+    uint64_t w[kMost];
     uint64_t sum = 0;
 #pragma unroll
-    for (unsigned j = 0; j < per; ++j) {
+    for (unsigned j = 0; j < kMost; ++j) {
       const uint32_t r = threadIdx.x * per + j;
       w[j] = 0;
-      if (r < cnt) {
+      if (j < per && r < cnt) {
         const uint32_t v = row(base + r);
         w[j] = (off[v + 1] - off[v] + kWin - 1) / kWin;
       }
@@ -41,9 +42,9 @@ __device__ __forceinline__ void deal_windows(uint64_t nbig, Row row, const uint6
     uint64_t total;
     uint64_t pre = block_excl_scan<uint64_t>(sum, tmp, &total);
 #pragma unroll
-    for (unsigned j = 0; j < per; ++j) {
+    for (unsigned j = 0; j < kMost; ++j) {
       const uint32_t r = threadIdx.x * per + j;
-      if (r < cnt) woff[r] = pre;
+      if (j < per && r < cnt) woff[r] = pre;
       pre += w[j];
     }
     if (threadIdx.x == 0) woff[cnt] = total;
