@@ -32,6 +32,13 @@ constexpr unsigned kOverhang = 1024;
 
 __device__ __forceinline__ uint32_t count_nl4(uint32_t w) { return __popc(__vcmpeq4(w, 0x0a0a0a0au)) >> 3; }
 
+// Bit i: byte i of w is a '\n'.
+__device__ __forceinline__ uint32_t newline_bits(uint32_t w) {
+  const uint32_t x = w ^ 0x0a0a0a0au;
+  const uint32_t z = ~(((x & 0x7f7f7f7fu) + 0x7f7f7f7fu) | x | 0x7f7f7f7fu);  // 0x80 in each zero byte of x
+  return ((z >> 7) * 0x01020408u) >> 24;
+}
+
 // Lines owned by a block: its '\n' bytes except one at len-1, plus line 0.
 __global__ void __launch_bounds__(kParseThreads) k_count_lines(const uint8_t* __restrict__ buf, uint64_t len,
                                                                uint64_t block0, uint32_t* __restrict__ block_lines) {
@@ -148,6 +155,58 @@ __device__ __forceinline__ bool parse_line_fast(const uint32_t* stage, uint64_t 
   return true;
 }
 
+// High bit of each byte of w that is no digit (below '0' as a signed char).
+__device__ __forceinline__ uint32_t non_digits(uint32_t w) {
+  const uint32_t t = (w | 0x80808080u) - 0x30303030u;  // no byte borrows
+  return (~t | w) & 0x80808080u;
+}
+
+// The number at byte `off` of the staged words, 1 to 8 digits: its value and
+// *n; false for any other length.
+__device__ __forceinline__ bool staged_number(const uint32_t* stage, uint32_t off, uint32_t* value, uint32_t* n) {
+  const uint32_t q = off >> 2, sh = 8 * (off & 3);
+  const uint32_t a = stage[q], b = stage[q + 1], c = stage[q + 2];
+  const uint32_t lo = __funnelshift_r(a, b, sh), hi = __funnelshift_r(b, c, sh);
+  const uint32_t m0 = non_digits(lo), m1 = non_digits(hi);
+  const uint32_t m = m0 ? m0 : m1;
+  uint32_t k = (m0 ? 0 : 4) + (__ffs(m) >> 3) - 1;
+  if (m == 0) {
+    k = 8;
+    if ((non_digits(reinterpret_cast<const uint8_t*>(stage)[off + 8]) & 0x80u) == 0) return false;  // a ninth digit
+  }
+  if (k == 0) return false;
+  // The k digits to the top of eight bytes (zeros before them): bytes past the
+  // number, whose subtraction may borrow, are shifted out.
+  const uint64_t d = (((uint64_t)(hi - 0x30303030u) << 32) | (lo - 0x30303030u)) << (64 - 8 * k);
+  const uint32_t d0 = (uint32_t)d, d1 = (uint32_t)(d >> 32);
+  constexpr uint32_t kHigh = 1000u | (100u << 16), kLow = 10u | (1u << 16);
+  const uint32_t v0 = __dp2a_hi(kLow, d0, __dp2a_lo(kHigh, d0, 0u));
+  const uint32_t v1 = __dp2a_hi(kLow, d1, __dp2a_lo(kHigh, d1, 0u));
+  *value = v0 * 10000u + v1;
+  *n = k;
+  return true;
+}
+
+// A line of the common form -- two numbers of at most 8 digits with one byte
+// between them -- without a loop: a number is two unaligned words, its length
+// the first byte that is no digit, its value four dot products of digits and
+// powers of ten (R-MAT scale 22, 250M lines: the byte loop, whose lanes wait
+// for the longest line of the warp, 4.66 ms; 1.91 with this, one update of the
+// id words per block and the newline bits below).  False (and the caller
+// takes the byte loop) for any other line, and where the 24 bytes it may read reach
+// past the staged ones.
+__device__ __forceinline__ bool parse_line_words(const uint32_t* stage, uint32_t off, uint32_t staged, uint64_t* key,
+                                                 uint32_t* vmax) {
+  if (off + 24 > staged) return false;
+  uint32_t x, y, nx, ny;
+  if (!staged_number(stage, off, &x, &nx)) return false;
+  if (reinterpret_cast<const uint8_t*>(stage)[off + nx] == '\n') return false;
+  if (!staged_number(stage, off + nx + 1, &y, &ny)) return false;
+  *vmax = max(*vmax, max(x, y));
+  *key = x == y ? ~0ull : (((uint64_t)y << 32) | x);
+  return true;
+}
+
 // Phase 1 finds the block's line starts (newlines a word at a time, a block
 // scan, offsets into shared memory); phase 2 deals the lines round-robin to
 // the threads, so the per-line work is balanced and the keys are written
@@ -171,35 +230,35 @@ __global__ void __launch_bounds__(kParseThreads) k_parse_lines(const uint8_t* __
   const uint64_t s = blo + (uint64_t)threadIdx.x * kChunk;
   const uint64_t e = min(len, s + kChunk);
   // Owned lines: one per '\n' in [s, e) that is not the last byte, plus line 0.
-  uint32_t nlmask[kChunk / 4];
-  uint32_t c = 0;
+  // One bit per byte of the chunk.
+  uint32_t low = 0, high = 0;
+  if (blo + kBlockBytes < len) {
 #pragma unroll
-  for (uint32_t j = 0; j < kChunk / 4; ++j) {
-    const uint64_t a = s + 4 * j;
-    uint32_t m = 0;
-    if (a < e) {
-      m = __vcmpeq4(stage[(a - blo) >> 2], 0x0a0a0a0au);
-      // Drop bytes at or past e, and a '\n' at len-1 (it starts no line).
-      const uint64_t lim = min(e, len - 1);
-      if (a + 4 > lim) m &= lim > a ? (0xffffffffu >> (8 * (4 - (uint32_t)(lim - a)))) : 0u;
+    for (uint32_t j = 0; j < kChunk / 4; ++j) {
+      const uint32_t m = newline_bits(stage[threadIdx.x * (kChunk / 4) + j]);
+      if (j < 8)
+        low |= m << (4 * j);
+      else
+        high |= m << (4 * (j - 8));
     }
-    nlmask[j] = m;
-    c += __popc(m) >> 3;
+  } else {
+    const uint64_t lim = min(e, len - 1);  // a '\n' at len-1 starts no line
+    for (uint32_t j = 0; j < kChunk / 4 && s + 4 * j < lim; ++j) {
+      uint32_t m = newline_bits(stage[threadIdx.x * (kChunk / 4) + j]);
+      if (lim - (s + 4 * j) < 4) m &= (1u << (lim - (s + 4 * j))) - 1;
+      if (j < 8)
+        low |= m << (4 * j);
+      else
+        high |= m << (4 * (j - 8));
+    }
   }
   const bool first = (s == 0 && len > 0);
-  if (first) c += 1;
   uint32_t total;
-  uint32_t pos = block_excl_scan<uint32_t>(c, tmp, &total);
+  uint32_t pos = block_excl_scan<uint32_t>(__popc(low) + __popc(high) + first, tmp, &total);
   if (first) starts[pos++] = 0;
-#pragma unroll
-  for (uint32_t j = 0; j < kChunk / 4; ++j) {
-    uint32_t m = nlmask[j];
-    while (m) {
-      const uint32_t k = (__ffs(m) - 1) >> 3;
-      m &= ~(0xffu << (8 * k));
-      starts[pos++] = (uint16_t)(s + 4 * j + k + 1 - blo);
-    }
-  }
+  const uint32_t chunk0 = threadIdx.x * kChunk;
+  for (; low; low &= low - 1) starts[pos++] = (uint16_t)(chunk0 + __ffs(low));
+  for (; high; high &= high - 1) starts[pos++] = (uint16_t)(chunk0 + 32 + __ffs(high));
   __syncthreads();
   const Bytes B{reinterpret_cast<const uint8_t*>(stage), buf, blo, blo + nvec * 16, len, ready,
                 reinterpret_cast<uint32_t*>(&words->counters[2])};
@@ -207,10 +266,12 @@ __global__ void __launch_bounds__(kParseThreads) k_parse_lines(const uint8_t* __
   uint32_t vmax = 0;
   bool any = false;
   const uint64_t lim = min(len, blo + nvec * 16);
+  const uint32_t staged_bytes = (uint32_t)(nvec * 16);
   for (uint32_t i = threadIdx.x; i < total; i += kParseThreads) {
     bool bad = false;
     uint64_t key;
-    if (!parse_line_fast(stage, blo, lim, blo + starts[i], &key, &bad, &vmax)) {
+    if (!parse_line_words(stage, starts[i], staged_bytes, &key, &vmax) &&
+        !parse_line_fast(stage, blo, lim, blo + starts[i], &key, &bad, &vmax)) {
       bad = false;
       key = parse_line(B, blo + starts[i], &bad, &vmax);
     }
@@ -221,11 +282,23 @@ __global__ void __launch_bounds__(kParseThreads) k_parse_lines(const uint8_t* __
     any = true;
     keys[slot0 + i] = key;
   }
+  // The largest id and whether there is a line, one update per block and only
+  // where it changes the words (read through L1: an old value only costs an
+  // update): they are two words for the whole grid, and an atomic on each per
+  // warp was what the kernel waited for, 0.7 ns apiece.
+  __shared__ uint32_t top[kParseThreads / 32];
   vmax = warp_max(vmax);
-  const unsigned anyw = __ballot_sync(kFull, any);
-  if (lane_id() == 0 && anyw) {
-    atomicMax(reinterpret_cast<unsigned int*>(&words->counters[0]), vmax);
-    atomicOr(reinterpret_cast<unsigned int*>(&words->counters[1]), 1u);
+  if (lane_id() == 0) top[warp_id()] = vmax;
+  const bool lines = __syncthreads_or(any) != 0;
+  if (threadIdx.x == 0 && lines) {
+    for (unsigned w = 1; w < kParseThreads / 32; ++w) vmax = max(vmax, top[w]);
+    unsigned int* const most = reinterpret_cast<unsigned int*>(&words->counters[0]);
+    unsigned int* const some = reinterpret_cast<unsigned int*>(&words->counters[1]);
+    unsigned int now, seen;
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(now) : "l"(most) : "memory");
+    asm volatile("ld.global.ca.u32 %0, [%1];" : "=r"(seen) : "l"(some) : "memory");
+    if (vmax > now) atomicMax(most, vmax);
+    if (!seen) atomicOr(some, 1u);
   }
 }
 
