@@ -374,14 +374,17 @@ __device__ __forceinline__ void close_entries(const PeelArgs& A, const Level& V,
   }
 }
 
-// A round over the frontier's shorter rows: a warp takes up to 32 edges (fewer
-// when the frontier is small for the grid) and walks their rows end to end;
-// rows of more than kLongJob entries go to A.big[0..*nbig), whose windows are
-// dealt to every warp after a barrier.  An entry costs its edge's state and,
-// if that is alive, one table slot or two, all independent of its neighbours';
-// the merge of the two sorted rows by one warp was a chain of as many dependent
-// steps as the rows have tiles of 32 entries (truss numbers of an R-MAT scale 16
-// graph, 850,000 edges, 828 rounds: levels 52.2 -> 15.9 ms).
+// A round over the frontier's shorter rows.  A frontier of at most kBigBatch
+// edges has the windows of all its rows dealt to every warp at once: every block
+// adds up the rows' lengths by itself, which is one batch of deal_windows, and
+// no warp is left with a row of many steps.  Of a larger one, a warp takes up to
+// 32 edges and walks their rows end to end; rows of more than kLongJob entries
+// go to A.big[0..*nbig), whose windows are dealt after a barrier.  An entry
+// costs its edge's state and, if that is alive, one table slot or two, all
+// independent of its neighbours'; the merge of the two sorted rows by one warp
+// was a chain of as many dependent steps as the rows have tiles of 32 entries
+// (truss numbers of an R-MAT scale 16 graph, 850,000 edges, 828 rounds: levels
+// 52.2 -> 15.9 ms, with small frontiers dealt 12.4).
 constexpr uint32_t kLongJob = 256;
 constexpr unsigned kJobWide = 2;
 
@@ -438,19 +441,20 @@ __device__ __forceinline__ void list_round(const PeelArgs& A, const Level& V, co
   tdec += ndec;
 }
 
-__device__ __forceinline__ void list_round_long(const PeelArgs& A, const Level& V, uint64_t nbig, uint32_t r,
-                                                uint32_t* next, unsigned long long* ncnt, uint64_t* woff,
-                                                uint64_t* tmp, uint64_t& tdec) {
+// The windows of the shorter rows of edges[0..n).
+__device__ __forceinline__ void list_round_windows(const PeelArgs& A, const Level& V, const uint32_t* edges,
+                                                   uint64_t n, uint32_t r, uint32_t* next, unsigned long long* ncnt,
+                                                   uint64_t* woff, uint64_t* tmp, uint64_t& tdec) {
   uint32_t ndec = 0;
   deal_windows<32 * kJobWide>(
-      nbig,
+      n,
       [&](uint64_t x) {
         uint32_t s, o;
-        shorter_row(A, A.big[x], s, o);
+        shorter_row(A, edges[x], s, o);
         return s;
       },
       A.off, woff, tmp, [&](uint64_t x, uint64_t b, uint64_t e) {
-        const uint32_t f = A.big[x];
+        const uint32_t f = edges[x];
         uint32_t s, o;
         shorter_row(A, f, s, o);
         uint32_t ee[kJobWide], oo[kJobWide];
@@ -747,7 +751,15 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
       unsigned long long* nc = &A.cnt[(i + 1) % 3];
       if (kLists) {
         unsigned long long* bc = &A.cnt[3 + (i & 1)];
-        list_round(A, V, fr, nf, r, nx, nc, bc, tdeg, tdec);
+        if (nf <= kBigBatch) {
+          for (uint64_t f = gtid; f < nf; f += gthreads) {
+            const uint64_t k = A.ends[fr[f]];
+            tdeg += (uint64_t)atomicSub(&A.adeg[(uint32_t)(k >> 32)], 1u) + atomicSub(&A.adeg[(uint32_t)k], 1u);
+          }
+          list_round_windows(A, V, fr, nf, r, nx, nc, woff, wtmp, tdec);
+        } else {
+          list_round(A, V, fr, nf, r, nx, nc, bc, tdeg, tdec);
+        }
         if (gtid == 0) {
           A.cnt[(i + 2) % 3] = 0;        // read at the start of round i-1
           A.cnt[3 + ((i + 1) & 1)] = 0;  // long rows of round i-1, read before the barrier ending it
@@ -757,7 +769,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
         if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
         const uint64_t nbig = sh[1];
         if (nbig) {
-          list_round_long(A, V, nbig, r, nx, nc, woff, wtmp, tdec);
+          list_round_windows(A, V, A.big, nbig, r, nx, nc, woff, wtmp, tdec);
           if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
         }
         alive -= nf;
