@@ -816,7 +816,7 @@ uint32_t big_row(const Ctx* c) {
 
 }  // namespace
 
-void KCore::reset_state(Ctx* c, const Graph& gr) {
+void KCore::ensure_state(Ctx* c, const Graph& gr) {
   n = gr.n;
   deg.ensure(c, (n ? n : 1) * sizeof(uint32_t));
   rem.ensure(c, (n ? n : 1) * sizeof(uint32_t));
@@ -825,6 +825,10 @@ void KCore::reset_state(Ctx* c, const Graph& gr) {
   front[1].ensure(c, (n ? n : 1) * sizeof(uint32_t));
   big.ensure(c, (n ? n : 1) * sizeof(uint32_t));
   cnt.ensure(c, (7 + kMaxGrid) * sizeof(unsigned long long));
+}
+
+void KCore::reset_state(Ctx* c, const Graph& gr) {
+  ensure_state(c, gr);
   if (n) {
     k_init_state<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(gr.deg.as<uint32_t>(), n,
                                                                              deg.as<uint32_t>(), rem.as<uint32_t>());
@@ -835,6 +839,7 @@ void KCore::reset_state(Ctx* c, const Graph& gr) {
 
 void KCore::init(Ctx* c, const Graph& gr) {
   base = &gr;
+  saved.clear();
   compacted = false;
   local_level = 0;
   levels.assign(1, 1);  // tag 0 = isolated, left at level 1
@@ -868,15 +873,24 @@ void KCore::compact_to_alive(Ctx* c, uint32_t level) {
             newid.as<uint32_t>(), L.off.as<uint64_t>(), g.max_deg, OutColumn{L.adj.as<uint32_t>()});
   L.max_deg = g.max_deg;  // an upper bound is enough here
   newid.release();
-  // Install; the previous compaction, if any, is kept for restores.
+  // Install; what was worked on so far is kept for restores.  (Its tags stay in
+  // their buffer; the ones freed here make up for that.)
+  Saved sv;
+  sv.rem = std::move(rem);
+  sv.levels = std::move(levels);
+  sv.succ = std::move(succ);
   if (compacted) {
-    Saved sv;
     sv.local = std::move(local);
     sv.idmap = std::move(idmap);
     sv.level = local_level;
-    saved.push_back(std::move(sv));
     local = Graph();
   }
+  saved.push_back(std::move(sv));
+  rem = std::move(snap);
+  alive2.release();
+  front[0].release();
+  front[1].release();
+  big.release();
   local.off = std::move(L.off);
   local.adj = std::move(L.adj);
   local.deg = std::move(L.deg);
@@ -1122,39 +1136,37 @@ uint32_t KCore::find_max_core(Ctx* c) {
 
 void KCore::restore_core(Ctx* c, uint32_t k) {
   if (compacted && k < local_level) {
-    // Below the compacted core: start over from the deepest earlier
-    // compaction at or below level k, else from the input graph.
-    while (!saved.empty() && saved.back().level > k) saved.pop_back();
-    if (!saved.empty()) {
-      local = std::move(saved.back().local);
-      idmap = std::move(saved.back().idmap);
-      local_level = saved.back().level;
-      saved.pop_back();
-      levels.assign(1, local_level);
-      succ.assign(1, 0);
-      reset_state(c, local);
-    } else {
-      compacted = false;
-      local = Graph();
-      idmap.release();
-      levels.assign(1, 1);
-      succ.assign(1, 0);
-      reset_state(c, *base);
-    }
+    // Below the compacted core: back to the deepest earlier graph whose level
+    // is at or below k, the input graph at the least.
+    while (saved.back().level > k) saved.pop_back();
+    Saved& sv = saved.back();
+    compacted = sv.level != 0;
+    local = std::move(sv.local);
+    idmap = std::move(sv.idmap);
+    local_level = sv.level;
+    rem = std::move(sv.rem);
+    levels = std::move(sv.levels);
+    succ = std::move(sv.succ);
+    saved.pop_back();
+    ensure_state(c, cur());
   }
   // Last successful probe at or below level k; everything newer is revived.
   uint32_t keep = 0;
   for (uint32_t t : succ)
     if (levels[t] <= k) keep = std::max(keep, t);
-  k_revive<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(rem.as<uint32_t>(), n, keep);
-  KT_LAUNCHED(c);
   levels.resize(keep + 1);
   std::vector<uint32_t> s2;
   for (uint32_t t : succ)
     if (t <= keep) s2.push_back(t);
   succ.swap(s2);
-  rebuild_alive(c);
-  recount(c);
+  if (keep == 0) {
+    reset_state(c, cur());  // every vertex with edges, at the graph's own degrees
+  } else {
+    k_revive<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(rem.as<uint32_t>(), n, keep);
+    KT_LAUNCHED(c);
+    rebuild_alive(c);
+    recount(c);
+  }
   const uint32_t tag = (uint32_t)levels.size();
   if (probe(c, k)) succ.push_back(tag);
 }

@@ -29,13 +29,17 @@ struct KCore {
   unsigned coop_grid = 0;
   std::vector<uint32_t> levels;  // levels[tag] = k of that probe
   std::vector<uint32_t> succ;    // tags of probes that were kept
-  // Earlier compactions (shallowest first), kept so that a restore below
-  // the current compaction's level starts from the deepest one at or below
-  // it instead of from the input graph.
+  // What was worked on before each compaction (the input graph first), kept
+  // with its probes' tags, so that a restore below the current copy's level goes
+  // on from the last probe at or below it.  (Starting over from a graph's first
+  // state, a recount of every row and a probe of everything: the 1,058-core of
+  // an R-MAT scale 22 graph in 4.0 ms, from its 738-core 1.2.)
   struct Saved {
-    Graph local;
+    Graph local;  // empty for the input graph
     DBuf idmap;
-    uint32_t level = 0;
+    DBuf rem;
+    std::vector<uint32_t> levels, succ;
+    uint32_t level = 0;  // 0 for the input graph
   };
   std::vector<Saved> saved;
 
@@ -63,6 +67,7 @@ struct KCore {
 
  private:
   void search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixed, uint64_t compact_below, void* result);
+  void ensure_state(Ctx* c, const Graph& gr);
   void reset_state(Ctx* c, const Graph& gr);
   void compact_to_alive(Ctx* c, uint32_t level);
 };
