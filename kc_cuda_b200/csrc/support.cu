@@ -1,5 +1,8 @@
 // Stage (d): support (triangles through each edge) of the working graph.
 //
+// Dense mode (bitsets): the product of the rows on the tensor cores where the
+// graph is dense enough for it (support_products), else a popcount per edge.
+//
 // List mode: the edges whose ends both have at most kFilterDeg neighbours are
 // counted from the triangles' lowest vertices (k_support_filter, a warp per
 // vertex).  The others are counted from their higher-degree end, with no
@@ -23,7 +26,9 @@
 
 #include "compact.cuh"
 #include "dense.cuh"
+#include "stages.h"
 #include "subgraph.h"
+#include "support_mma.h"
 
 namespace kt {
 namespace {
@@ -357,6 +362,16 @@ __global__ void __launch_bounds__(256) k_dense_support_capped(uint64_t m, const 
   if (lane_id() == 0 && wr) atomicAdd(row_words, wr);
 }
 
+// The entries of a tile-ordered list whose graphs are not flagged.
+struct Uncounted {
+  const uint32_t* order;
+  const uint64_t* ends;
+  const uint32_t* vgid;
+  const uint8_t* counted;
+  __device__ bool keep(uint64_t i) const { return !counted[vgid[(uint32_t)(ends[order[i]] >> 32)]]; }
+  __device__ uint32_t value(uint64_t i) const { return order[i]; }
+};
+
 // Tile keys: (u >> tb) << 16 | (v >> tb), stable-sorted with the edge ids.
 __global__ void k_tile_keys(uint64_t m, const uint64_t* __restrict__ ends, uint32_t tb, uint64_t* __restrict__ keys,
                             uint32_t* __restrict__ ids) {
@@ -368,18 +383,18 @@ __global__ void k_tile_keys(uint64_t m, const uint64_t* __restrict__ ends, uint3
 }
 
 // Grid of the resident blocks of `kernel` with the rows' shared memory.
-unsigned dense_grid(Ctx* c, const void* kernel, const Sub& s, size_t smem) {
+unsigned dense_grid(Ctx* c, const void* kernel, uint64_t m, size_t smem) {
   allow_max_dynamic_smem(kernel);
   int per_sm = 0;
   KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, 256, smem));
-  return grid_for((s.m + 31) / 32 * 32, 256, std::max(1, per_sm) * c->num_sms);
+  return grid_for((m + 31) / 32 * 32, 256, std::max(1, per_sm) * c->num_sms);
 }
 
 template <int NQ>
-void launch_exact(Ctx* c, const Sub& s, uint32_t* sup, unsigned long long* row_words, unsigned long long* cursor) {
+void launch_exact(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint32_t* sup, unsigned long long* row_words, unsigned long long* cursor) {
   const size_t smem = dense_smem_bytes(s.W, 256);
-  const unsigned grid = dense_grid(c, (const void*)k_dense_support<NQ>, s, smem);
-  k_dense_support<NQ><<<grid, 256, smem, c->stream>>>(s.m, s.order.as<uint32_t>(), s.ends.as<uint64_t>(),
+  const unsigned grid = dense_grid(c, (const void*)k_dense_support<NQ>, m, smem);
+  k_dense_support<NQ><<<grid, 256, smem, c->stream>>>(m, order, s.ends.as<uint64_t>(),
                                                       dense_rows(s), sup, row_words, cursor);
   KT_LAUNCHED(c);
 }
@@ -387,26 +402,26 @@ void launch_exact(Ctx* c, const Sub& s, uint32_t* sup, unsigned long long* row_w
 // Exact counts: option support_rows (1, 2 or 4) edges sharing row u per
 // shared-memory read of it.  Capped counts: two edges sharing row u side by
 // side, one per half of the warp.
-void launch_dense_support(Ctx* c, const Sub& s, uint32_t* sup, bool capped, uint32_t cap, const uint32_t* gcap,
+void launch_dense_support(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint32_t* sup, bool capped, uint32_t cap, const uint32_t* gcap,
                           unsigned long long* row_words, unsigned long long* cursor) {
   if (s.W <= kShortRow) {  // (exact also where a cap is given: there is little to abandon)
-    k_dense_support_short<<<grid_for((s.m + 7) / 8 * 32, 256, c->num_sms * 8), 256, 0, c->stream>>>(
-        s.m, s.order.as<uint32_t>(), s.ends.as<uint64_t>(), dense_rows(s), sup, row_words);
+    k_dense_support_short<<<grid_for((m + 7) / 8 * 32, 256, c->num_sms * 8), 256, 0, c->stream>>>(
+        m, order, s.ends.as<uint64_t>(), dense_rows(s), sup, row_words);
     KT_LAUNCHED(c);
   } else if (capped) {
     const size_t smem = dense_smem_bytes(s.W, 256);
-    const unsigned grid = dense_grid(c, (const void*)k_dense_support_capped, s, smem);
-    k_dense_support_capped<<<grid, 256, smem, c->stream>>>(s.m, s.order.as<uint32_t>(), s.ends.as<uint64_t>(),
+    const unsigned grid = dense_grid(c, (const void*)k_dense_support_capped, m, smem);
+    k_dense_support_capped<<<grid, 256, smem, c->stream>>>(m, order, s.ends.as<uint64_t>(),
                                                            dense_rows(s), cap, gcap,
                                                            gcap ? s.vgid.as<uint32_t>() : nullptr, sup, row_words,
                                                            cursor);
     KT_LAUNCHED(c);
   } else if (c->opt.support_rows <= 1) {
-    launch_exact<1>(c, s, sup, row_words, cursor);
+    launch_exact<1>(c, s, order, m, sup, row_words, cursor);
   } else if (c->opt.support_rows == 2) {
-    launch_exact<2>(c, s, sup, row_words, cursor);
+    launch_exact<2>(c, s, order, m, sup, row_words, cursor);
   } else {
-    launch_exact<4>(c, s, sup, row_words, cursor);
+    launch_exact<4>(c, s, order, m, sup, row_words, cursor);
   }
 }
 
@@ -584,10 +599,28 @@ void edge_support(Ctx* c, const Sub& s, uint32_t* sup, uint32_t cap, const uint3
   cudaEvent_t e0;
   if (c->opt.verbose) KT_CUDA(cudaEventRecord(c->ev[2], c->stream));
   c->timer.begin(c->stream, &c->stats.ms_support_kernel, &e0);
-  if (s.W) {
+  uint64_t product_words = 0;
+  const uint32_t* order = s.W ? s.order.as<uint32_t>() : nullptr;
+  uint64_t left = s.m;  // edges of `order` that the products leave
+  DBuf rest;
+  std::vector<uint8_t> counted;
+  const bool products = support_products(c, s, sup, counted, &product_words);
+  if (products) {
+    left = 0;
+    if (!counted.empty() && std::find(counted.begin(), counted.end(), 0) != counted.end()) {
+      DBuf flags(c, counted.size());
+      copy_h2d(c, flags.get(), counted.data(), counted.size());
+      rest.alloc(c, s.m * sizeof(uint32_t));
+      left = compact(c, s.m, Uncounted{order, s.ends.as<uint64_t>(), s.vgid.as<uint32_t>(), flags.as<uint8_t>()},
+                     rest.as<uint32_t>());
+      order = rest.as<uint32_t>();
+    }
+  }
+  if (!left) {
+  } else if (s.W) {
     unsigned long long* a = acc.as<unsigned long long>();
     const bool capped = cap || (gcap && s.vgid.get());
-    launch_dense_support(c, s, sup, capped, cap, s.vgid.get() ? gcap : nullptr, a + 1, a + 2);
+    launch_dense_support(c, s, order, left, sup, capped, cap, s.vgid.get() ? gcap : nullptr, a + 1, a + 2);
   } else {
     support_lists(c, s, sup);
   }
@@ -602,14 +635,15 @@ void edge_support(Ctx* c, const Sub& s, uint32_t* sup, uint32_t cap, const uint3
                                                                              acc.as<unsigned long long>());
   KT_LAUNCHED(c);
   uint64_t h[2];
-  copy_d2h(c, h, acc.get(), 16);
+  read_checked(c, h, acc.get(), 16, "support");
+  h[1] += product_words;
   const uint64_t merge = 4 * h[0] + 4 * s.m + 8 * ((uint64_t)s.n + 1);
   c->stats.support_bytes += merge;
   c->stats.support_row_words += h[1];
   // Dense: row words, plus per edge its list entry (4), ends (8) and result (4).
   c->stats.support_kernel_bytes += s.W ? 4 * h[1] + 16 * s.m : merge;
   KT_LOG(c, "kt: support (%s) on %u vertices (widest group %u), %llu edges: %llu row words, %.3f ms\n",
-         s.W ? (cap || (gcap && s.vgid.get()) ? "dense capped" : "dense") : "list", s.n,
+         products ? "products" : s.W ? (cap || (gcap && s.vgid.get()) ? "dense capped" : "dense") : "list", s.n,
          s.vbase.get() ? s.max_group : s.n, (unsigned long long)s.m, (unsigned long long)h[1],
          c->opt.verbose ? event_ms(c->ev[2], c->ev[3]) : 0.0);
 }
