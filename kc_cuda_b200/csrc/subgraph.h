@@ -42,6 +42,9 @@ struct Sub {
   std::vector<uint32_t> group_n;  // vertices of each graph (host)
 };
 
+// Bins of a support histogram that a block counts in shared memory.
+constexpr uint32_t kHistBins = 6144;
+
 // Builds the subgraph induced by the k-core state's alive vertices.
 void build_sub(Ctx* c, const Graph& g, const KCore& kc, Sub& s);
 // Builds the whole graph as a subgraph (every vertex of degree > 0).

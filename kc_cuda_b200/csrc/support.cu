@@ -439,16 +439,26 @@ __global__ void k_support_alg(uint64_t m, const uint64_t* __restrict__ ends, con
   if (lane_id() == 0 && s) atomicAdd(out, (unsigned long long)s);
 }
 
-// hist[min(sup, cap)] += 1, warp-aggregated over equal bins.
-__global__ void k_sup_hist(const uint32_t* __restrict__ sup, uint64_t m, uint32_t cap,
-                           unsigned long long* __restrict__ hist) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ((m + 31) & ~31ULL);
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const bool ok = i < m;
-    const uint32_t b = ok ? min(sup[i], cap) : 0xffffffffu;
-    const unsigned peers = __match_any_sync(kFull, b);
-    if (ok && lane_id() == (unsigned)(__ffs(peers) - 1)) atomicAdd(&hist[b], (unsigned long long)__popc(peers));
+// hist[min(sup, cap)] += 1.  Supports of a core crowd into few bins, so a block
+// counts the first kHistBins in shared memory and adds them up at its end
+// (10.5M edges, 1,686 bins: 0.61 ms with an atomic per distinct bin of a warp,
+// below 0.03 now).
+__global__ void __launch_bounds__(256) k_sup_hist(const uint32_t* __restrict__ sup, uint64_t m, uint32_t cap,
+                                                  unsigned long long* __restrict__ hist) {
+  __shared__ uint32_t bins[kHistBins];
+  const uint32_t have = min(cap + 1, kHistBins);
+  for (uint32_t b = threadIdx.x; b < have; b += blockDim.x) bins[b] = 0;
+  __syncthreads();
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t b = min(sup[i], cap);
+    if (b < kHistBins)
+      atomicAdd(&bins[b], 1u);
+    else
+      atomicAdd(&hist[b], 1ULL);
   }
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < have; b += blockDim.x)
+    if (bins[b]) atomicAdd(&hist[b], (unsigned long long)bins[b]);
 }
 
 }  // namespace
@@ -457,8 +467,8 @@ uint32_t support_bound(Ctx* c, const uint32_t* sup, uint64_t m, uint32_t cap) {
   if (m == 0 || cap < 3) return 0;
   DBuf hist(c, ((uint64_t)cap + 1) * 8);
   zero(c, hist.get(), hist.bytes());
-  k_sup_hist<<<grid_for(m, 256, c->num_sms * 16), 256, 0, c->stream>>>(sup, m, cap,
-                                                                       hist.as<unsigned long long>());
+  k_sup_hist<<<grid_for(m, 256, c->num_sms * 4), 256, 0, c->stream>>>(sup, m, cap,
+                                                                      hist.as<unsigned long long>());
   KT_LAUNCHED(c);
   std::vector<unsigned long long> h(cap + 1);
   copy_d2h(c, h.data(), hist.get(), h.size() * sizeof(unsigned long long));
