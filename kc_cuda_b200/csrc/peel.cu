@@ -1173,6 +1173,7 @@ struct Peeler {
     A.ends = s->ends.as<uint64_t>();
     A.off = s->off.as<uint64_t>();
     A.adj = s->adj.as<uint32_t>();
+    lower_ids(c, *s);
     A.eid = s->eid.as<uint32_t>();
     A.sup = sup;
     A.state = state.as<uint32_t>();

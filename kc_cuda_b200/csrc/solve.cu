@@ -63,6 +63,7 @@ bool truss_possible(Ctx* c, const Sub& s, const uint32_t* sup, uint32_t g) {
   if (s.n == 0 || s.m == 0) return false;
   DBuf cnt(c, 8);
   zero(c, cnt.get(), 8);
+  lower_ids(c, s);
   k_rows_at_least<<<grid_for((uint64_t)s.n * 32, 256, c->num_sms * 16), 256, 0, c->stream>>>(
       s.n, s.off.as<uint64_t>(), s.eid.as<uint32_t>(), sup, g - 2, g - 1, cnt.as<unsigned long long>());
   KT_LAUNCHED(c);

@@ -227,8 +227,7 @@ __global__ void k_upper_ids(const uint64_t* __restrict__ off, const uint32_t* __
 // rows' bitsets are built (R.spre) -- by the position of r in row c, a
 // popcount away.  Warp per row.
 __global__ void k_lower_ids(const uint64_t* __restrict__ off, const uint32_t* __restrict__ adj, uint64_t n,
-                            const uint64_t* __restrict__ up, const uint64_t* __restrict__ eoff, DenseRows R,
-                            uint32_t* __restrict__ eid) {
+                            const uint64_t* __restrict__ up, DenseRows R, uint32_t* eid) {
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   for (uint64_t r = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id(); r < n; r += warps) {
     const uint64_t b = off[r], u0 = up[r];
@@ -248,7 +247,7 @@ __global__ void k_lower_ids(const uint64_t* __restrict__ off, const uint32_t* __
         }
         pos = lo;
       }
-      eid[j] = (uint32_t)(eoff[col] + (pos - up[col]));
+      eid[j] = eid[pos];
     }
   }
 }
@@ -269,6 +268,7 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
                      uint32_t ngroups = 0) {
   if (na >= 0xffffffffULL) throw Error(KT_ERR_LIMIT, "subgraph: too many vertices");
   s.n = (uint32_t)na;
+  s.has_lower_ids = false;
   s.orig.alloc(c, (na ? na : 1) * sizeof(uint32_t));
   s.off.alloc(c, (na + 1) * sizeof(uint64_t));
   s.up.alloc(c, (na ? na : 1) * sizeof(uint64_t));
@@ -393,8 +393,8 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
   }
   gsize.release();
   // Edge ids: the upper entries number themselves; then the bitsets (dense
-  // mode, built from the sorted rows); then the lower entries' ids, from the
-  // bitsets' popcounts when they are there, else by binary search.
+  // mode, built from the sorted rows).  The lower entries' ids wait until
+  // something reads them (lower_ids).
   DBuf upcnt(c, (na + 1) * sizeof(uint32_t));
   zero(c, upcnt.get(), (na + 1) * sizeof(uint32_t));
   k_upper_start<<<grid_for(na, 256, c->num_sms * 16), 256, 0, c->stream>>>(
@@ -414,12 +414,6 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
   copy_d2h(c, &md, sdeg.as<uint32_t>() + (na - 1), sizeof(uint32_t));
   s.max_deg = md;
   build_bits(c, s);
-  DenseRows R = dense_rows(s);
-  if (!s.W) R.spre = nullptr;
-  k_lower_ids<<<grid_for(na * 32, 256, c->num_sms * 16), 256, 0, c->stream>>>(
-      s.off.as<uint64_t>(), s.adj.as<uint32_t>(), na, s.up.as<uint64_t>(), eoff.as<uint64_t>(), R,
-      s.eid.as<uint32_t>());
-  KT_LAUNCHED(c);
   if (idmap) {
     k_map_ids<<<grid_for(na, 256, c->num_sms * 16), 256, 0, c->stream>>>(s.orig.as<uint32_t>(), na, idmap);
     KT_LAUNCHED(c);
@@ -427,6 +421,16 @@ void build_from_list(Ctx* c, const Graph& g, const uint32_t* alive, uint64_t na,
 }
 
 }  // namespace
+
+void lower_ids(Ctx* c, const Sub& s) {
+  if (s.has_lower_ids || !s.m) return;
+  DenseRows R = dense_rows(s);
+  if (!s.W) R.spre = nullptr;
+  k_lower_ids<<<grid_for((uint64_t)s.n * 32, 256, c->num_sms * 16), 256, 0, c->stream>>>(
+      s.off.as<uint64_t>(), s.adj.as<uint32_t>(), s.n, s.up.as<uint64_t>(), R, s.eid.as<uint32_t>());
+  KT_LAUNCHED(c);
+  s.has_lower_ids = true;
+}
 
 void build_sub(Ctx* c, const Graph& g, const KCore& kc, Sub& s) {
   (void)g;

@@ -591,6 +591,7 @@ static void support_lists(Ctx* c, const Sub& s, uint32_t* sup) {
   DBuf list(c, (uint64_t)s.n * sizeof(uint32_t));
   const uint64_t nl = compact(c, s.n, LongRow{s.off.as<uint64_t>()}, list.as<uint32_t>());
   if (!nl) return;
+  lower_ids(c, s);
   DBuf cur(c, 8);
   zero(c, cur.get(), 8);
   const unsigned grid = (unsigned)std::min<uint64_t>((uint64_t)per_sm * c->num_sms, nl);
