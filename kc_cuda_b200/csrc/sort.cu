@@ -3,14 +3,20 @@
 //
 // One pass = tile histograms -> digit-major exclusive scan -> stable scatter:
 // a tile of kSortTile keys ranks them (each warp owns consecutive keys and
-// ranks them with __match_any_sync against warp-private running digit
-// counters), places the tile in shared memory sorted by digit and writes every
+// finds the lanes with a key's digit by a ballot per bit, against warp-private
+// running digit counters), places the tile in shared memory sorted by digit and writes every
 // digit's run with consecutive threads on consecutive addresses.  (Counting
 // all passes at once and finding each tile's places by look-back over the tiles
 // before it, one word per digit and tile, reads the keys once less but was
 // slower, 113 against 100 us a pass of 16M keys: the words are an eighth of the
 // keys' bytes, read several times over.)  At most one tile of keys is sorted in
 // shared memory by one block in one launch.
+//
+// The scatter is bound by the shared-memory pipe (87 % busy, DRAM 24 %, with the
+// lanes matched by __match_any_sync, which is the slower the more digits a warp
+// has): 1.05-1.14 ms a pass of 214M random keys by ballots, 1.26-1.39 by match;
+// taking places by atomics of the first lane instead of a load and a store:
+// 1.10-1.20.
 #include <algorithm>
 
 #include "kt_device.cuh"
@@ -53,15 +59,15 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_hist(const uint64_t* __re
 }
 
 struct SortShared {
-  uint32_t wrun[kSortWarps][256];  // running counts per warp and digit, then the warps' first places
+  uint32_t wrun[kSortWarps][256];  // running counts per warp and digit, then the warps' first places in the tile
   uint32_t dstart[256];            // the digits' first places in the tile
   uint32_t tmp[33];
 };
 
 // Ranks the tile's keys k[] (entry j of lane l of warp w is key w * kWarpKeys +
 // j * 32 + l, valid below tn) by a digit: on return rank[] is each key's place in
-// its warp's run of the digit, S.wrun the warps' first places in it, S.dstart the
-// digits' first places.
+// its warp's run of the digit, S.wrun the warps' first places of it in the tile,
+// S.dstart the digits' first places.
 __device__ __forceinline__ void rank_tile(SortShared& S, const uint64_t (&k)[kSortIpt], uint32_t tn, int shift,
                                               uint32_t mask, uint32_t (&rank)[kSortIpt]) {
   const unsigned w = warp_id(), l = lane_id();
@@ -71,8 +77,14 @@ __device__ __forceinline__ void rank_tile(SortShared& S, const uint64_t (&k)[kSo
 #pragma unroll
   for (unsigned j = 0; j < kSortIpt; ++j) {
     const bool valid = w * kWarpKeys + j * 32 + l < tn;
-    const uint32_t d = valid ? (uint32_t)(k[j] >> shift) & mask : 256u;
-    const unsigned peers = __match_any_sync(kFull, d);
+    const uint32_t d = (uint32_t)(k[j] >> shift) & mask;
+    unsigned peers = __ballot_sync(kFull, valid);
+#pragma unroll
+    for (unsigned b = 0; b < 8; ++b) {
+      if (!((mask >> b) & 1)) break;  // (a mask of low bits)
+      const unsigned have = __ballot_sync(kFull, (d >> b) & 1);
+      peers &= (d >> b) & 1 ? have : ~have;
+    }
     const uint32_t base = valid ? S.wrun[w][d] : 0u;
     __syncwarp();
     if (valid && l == (unsigned)(__ffs(peers) - 1)) S.wrun[w][d] = base + __popc(peers);
@@ -80,21 +92,23 @@ __device__ __forceinline__ void rank_tile(SortShared& S, const uint64_t (&k)[kSo
     rank[j] = base + __popc(peers & lt);
   }
   __syncthreads();
+  // One digit a thread: its first place, then the warps' places after it.
   const unsigned d = threadIdx.x;
   uint32_t s = 0;
-  if (d < 256) {
 #pragma unroll
-    for (unsigned q = 0; q < kSortWarps; ++q) {
-      const uint32_t t = S.wrun[q][d];
-      S.wrun[q][d] = s;
-      s += t;
-    }
-  }
+  for (unsigned q = 0; q < kSortWarps; ++q) s += S.wrun[q][d];
   uint32_t total;
   s = block_excl_scan<uint32_t>(s, S.tmp, &total);
-  if (d < 256) S.dstart[d] = s;
+  S.dstart[d] = s;
+#pragma unroll
+  for (unsigned q = 0; q < kSortWarps; ++q) {
+    const uint32_t t = S.wrun[q][d];
+    S.wrun[q][d] = s;
+    s += t;
+  }
   __syncthreads();
 }
+static_assert(kSortThreads == 256, "a thread per digit");
 
 template <bool kVals>
 __device__ __forceinline__ void place_tile(const SortShared& S, const uint64_t (&k)[kSortIpt],
@@ -105,7 +119,7 @@ __device__ __forceinline__ void place_tile(const SortShared& S, const uint64_t (
   for (unsigned j = 0; j < kSortIpt; ++j) {
     if (w * kWarpKeys + j * 32 + l < tn) {
       const uint32_t d = (uint32_t)(k[j] >> shift) & mask;
-      const uint32_t p = S.dstart[d] + S.wrun[w][d] + rank[j];
+      const uint32_t p = S.wrun[w][d] + rank[j];
       skeys[p] = k[j];
       if (kVals) svals[p] = v[j];
     }
