@@ -494,7 +494,7 @@ void solve_wave(Ctx* c, const std::vector<BatchItem*>& items) {
   {
     KCore kc;
     kc.init(c, U);
-    kc.core_numbers(c, dcore.as<uint32_t>());
+    kc.core_numbers(c, dcore.as<uint32_t>(), &vbase);
   }
   DBuf dvb(c, (G + 1) * sizeof(uint64_t)), dgid(c, (nv ? nv : 1) * sizeof(uint32_t)), dcm(c, G * sizeof(uint32_t));
   copy_h2d(c, dvb.get(), vbase.data(), (G + 1) * sizeof(uint64_t));

@@ -60,10 +60,11 @@ struct KCore {
   void restore_core(Ctx* c, uint32_t k);
   // member[v] (base ids) = v is alive.
   void members(Ctx* c, uint8_t* dout);
-  // Full decomposition (consumes the state; never compacts).
-  void core_numbers(Ctx* c, uint32_t* dcore);
+  // Full decomposition (consumes the state; never compacts).  Of a union of
+  // graphs, starts gives the first vertex of each and the number of all.
+  void core_numbers(Ctx* c, uint32_t* dcore, const std::vector<uint64_t>* starts = nullptr);
   // The same in one cooperative launch (levels stepped on the device).
-  void core_numbers_persistent(Ctx* c, uint32_t* dcore);
+  void core_numbers_persistent(Ctx* c, uint32_t* dcore, const std::vector<uint64_t>* starts);
 
  private:
   void search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixed, uint64_t compact_below, void* result);

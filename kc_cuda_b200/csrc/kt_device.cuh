@@ -176,9 +176,16 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
   return v;
 }
 
+// The blocks that work together: all of the grid, or a team's consecutive ones.
+struct Crew {
+  unsigned rank, blocks;
+  __device__ Crew() : rank(blockIdx.x), blocks(gridDim.x * gridDim.y * gridDim.z) {}
+  __device__ Crew(unsigned r, unsigned b) : rank(r), blocks(b) {}
+};
+
 // Bounded grid barrier for kernels launched with cudaLaunchCooperativeKernel
-// (which guarantees that every block is resident).  Every block must call it
-// the same number of times.  A wait longer than `timeout_ns` sets
+// (which guarantees that every block is resident).  Every block (or every
+// block of the crew that `w` belongs to) must call it the same number of times.  A wait longer than `timeout_ns` sets
 // kDevErrBarrier and returns; callers test the returned flag and leave the
 // kernel, so a mismatch can never hang the device.  Returns true when no
 // error is flagged.
@@ -196,17 +203,17 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
 template <int N>
 __device__ __forceinline__ bool grid_barrier_read(DevWords* w, unsigned long long timeout_ns,
                                                   const unsigned long long* const (&src)[N],
-                                                  unsigned long long* sh) {
+                                                  unsigned long long* sh, Crew crew = Crew()) {
   __syncthreads();
   bool ok = true;
-  const uint32_t nb = gridDim.x * gridDim.y * gridDim.z;
+  const uint32_t nb = crew.blocks;
   if (nb == 1 && threadIdx.x == 0) {  // nobody to wait for
     __threadfence();
     if (timeout_ns == 0) atomicOr(&w->err, kDevErrBarrier);
     ok = ld_acquire_u32(&w->err) == 0;
   } else if (threadIdx.x == 0) {
     __threadfence();
-    const uint32_t old = atomicAdd(&w->bar, blockIdx.x == 0 ? 0x80000000u - (nb - 1) : 1u);
+    const uint32_t old = atomicAdd(&w->bar, crew.rank == 0 ? 0x80000000u - (nb - 1) : 1u);
     unsigned long long t0 = 0;
     for (unsigned spins = 0;; ++spins) {
       const unsigned long long v = ld_acquire_u64(reinterpret_cast<const unsigned long long*>(&w->err));

@@ -11,7 +11,7 @@ namespace kt {
 constexpr unsigned kBigBatch = 1024;  // long rows per batch of dealt windows
 
 // Deals the kWin-entry windows of the rows row(0), ..., row(nbig - 1) of
-// `off` to every warp of the grid, so one long row is spread over the whole
+// `off` to every warp of the grid (or crew), so one long row is spread over the whole
 // GPU instead of one block: each block lists the rows' first window numbers
 // (the same block scan in every block, kBigBatch rows at a time) and warp w
 // takes windows w, w + warps, ...; `drop(i, b, e)` handles entries [b, e) (at
@@ -19,9 +19,9 @@ constexpr unsigned kBigBatch = 1024;  // long rows per batch of dealt windows
 // synchronises the block); blocks have 256, 512 or 1024 threads.
 template <unsigned kWin, class Row, class Drop>
 __device__ __forceinline__ void deal_windows(uint64_t nbig, Row row, const uint64_t* __restrict__ off, uint64_t* woff,
-                                             uint64_t* tmp, Drop drop) {
-  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-  const uint64_t gwarp = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
+                                             uint64_t* tmp, Drop drop, Crew crew = Crew()) {
+  const uint64_t gwarps = (uint64_t)crew.blocks * (blockDim.x >> 5);
+  const uint64_t gwarp = (uint64_t)crew.rank * (blockDim.x >> 5) + warp_id();
   constexpr unsigned kMost = kBigBatch / 256;
   const unsigned per = kBigBatch / blockDim.x;  // rows per thread
   for (uint64_t base = 0; base < nbig; base += kBigBatch) {
