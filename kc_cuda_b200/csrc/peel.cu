@@ -58,6 +58,7 @@ struct PeelArgs {
   const uint64_t* off;
   const uint32_t* adj;
   const uint32_t* eid;
+  uint32_t n;       // vertices
   uint32_t* sup;
   uint32_t* state;
   uint32_t* truss;  // may be null
@@ -93,6 +94,12 @@ struct PeelArgs {
   const unsigned long long* table;
   uint32_t table_bits;  // 2^table_bits slots
   uint32_t* big;
+  // and the rows, each of rlen[v] entries from off[v] on (with `pack`, copies
+  // that k_levels may drop dead entries from).
+  uint32_t* radj;
+  uint32_t* reid;
+  uint32_t* rlen;
+  bool pack;
   // A level tried from a snapshot: give up (the level's truss is empty) as
   // soon as fewer than this many edges can remain, t(t-1)/2 for level t
   // (0: peel to the end).  The state is then partial; the caller undoes it.
@@ -312,6 +319,11 @@ __device__ __forceinline__ uint32_t edge_hash(uint32_t u, uint32_t v) {
 __device__ __forceinline__ uint32_t edge_tag(uint32_t u, uint32_t v) { return (u * 0x27D4EB2Fu) ^ (v + (v << 13)); }
 constexpr unsigned long long kNoEdge = ~0ULL;
 
+__global__ void k_row_lengths(const uint64_t* __restrict__ off, uint64_t n, uint32_t* __restrict__ len) {
+  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+    len[v] = (uint32_t)(off[v + 1] - off[v]);
+}
+
 __global__ void k_table_build(uint64_t m, const uint64_t* __restrict__ ends, unsigned long long* table,
                               uint32_t bits) {
   const uint64_t mask = (1ULL << bits) - 1;
@@ -340,7 +352,7 @@ __device__ __forceinline__ void shorter_row(const PeelArgs& A, uint32_t e, uint3
   const uint64_t k = A.ends[e];
   s = (uint32_t)(k >> 32);
   other = (uint32_t)k;
-  if (A.off[s + 1] - A.off[s] > A.off[other + 1] - A.off[other]) {
+  if (A.rlen[s] > A.rlen[other]) {
     const uint32_t t = s;
     s = other;
     other = t;
@@ -348,7 +360,9 @@ __device__ __forceinline__ void shorter_row(const PeelArgs& A, uint32_t e, uint3
 }
 
 // N row entries per lane (row positions j[t], where ok[t]) of the shorter rows
-// of frontier edges e[t], whose other ends are o[t].
+// of frontier edges e[t], whose other ends are o[t].  (Looking the third edges
+// up before the entries' own states are known, an access less in a small
+// round's chain, costs more for the dead entries than it saves.)
 template <unsigned N>
 __device__ __forceinline__ void close_entries(const PeelArgs& A, const Level& V, const uint32_t (&e)[N],
                                               const uint32_t (&o)[N], const uint64_t (&j)[N], const bool (&ok)[N],
@@ -356,8 +370,8 @@ __device__ __forceinline__ void close_entries(const PeelArgs& A, const Level& V,
   uint32_t a[N], w[N], b[N];
 #pragma unroll
   for (unsigned t = 0; t < N; ++t) {
-    a[t] = ok[t] ? A.eid[j[t]] : 0u;
-    w[t] = ok[t] ? A.adj[j[t]] : 0u;
+    a[t] = ok[t] ? A.reid[j[t]] : 0u;
+    w[t] = ok[t] ? A.radj[j[t]] : 0u;
   }
   bool live[N];
 #pragma unroll
@@ -374,6 +388,30 @@ __device__ __forceinline__ void close_entries(const PeelArgs& A, const Level& V,
   }
 }
 
+// Drops the dead entries of every row, in place, a warp per row.
+__device__ __forceinline__ void pack_rows(const PeelArgs& A, uint64_t gwarp, uint64_t gwarps) {
+  const unsigned lane = lane_id();
+  for (uint64_t v = gwarp; v < A.n; v += gwarps) {
+    const uint64_t b = A.off[v];
+    const uint32_t len = A.rlen[v];
+    uint32_t kept = 0;
+    for (uint32_t j0 = 0; j0 < len; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      const uint32_t e = j < len ? A.reid[b + j] : 0u, w = j < len ? A.radj[b + j] : 0u;
+      const bool keep = j < len && A.state[e] == kAlive;
+      const unsigned bal = __ballot_sync(kFull, keep);
+      __syncwarp();
+      if (keep) {
+        const uint64_t at = b + kept + __popc(bal & lanemask_lt());
+        A.reid[at] = e;
+        A.radj[at] = w;
+      }
+      kept += __popc(bal);
+    }
+    if (lane == 0) A.rlen[v] = kept;
+  }
+}
+
 // A round over the frontier's shorter rows.  A frontier of at most kBigBatch
 // edges has the windows of all its rows dealt to every warp at once: every block
 // adds up the rows' lengths by itself, which is one batch of deal_windows, and
@@ -384,7 +422,8 @@ __device__ __forceinline__ void close_entries(const PeelArgs& A, const Level& V,
 // independent of its neighbours'; the merge of the two sorted rows by one warp
 // was a chain of as many dependent steps as the rows have tiles of 32 entries
 // (truss numbers of an R-MAT scale 16 graph, 850,000 edges, 828 rounds: levels
-// 52.2 -> 15.9 ms, with small frontiers dealt 12.4).
+// 52.2 -> 15.9 ms, with small frontiers dealt 12.4, now 11.0; dealing up to
+// 4,096 edges so is slower by 0.4).
 constexpr uint32_t kLongJob = 256;
 constexpr unsigned kJobWide = 2;
 
@@ -407,9 +446,9 @@ __device__ __forceinline__ void list_round(const PeelArgs& A, const Level& V, co
       shorter_row(A, e, s, o);
       tdeg += (uint64_t)atomicSub(&A.adeg[s], 1u) + atomicSub(&A.adeg[o], 1u);
       start = A.off[s];
-      const uint64_t l = A.off[s + 1] - start;
+      const uint32_t l = A.rlen[s];
       is_long = l > kLongJob;
-      len = is_long ? 0u : (uint32_t)l;
+      len = is_long ? 0u : l;
     }
     push_warp_full(is_long, e, A.big, nbig, A.cap, &A.words->err);
     const uint32_t incl = warp_incl_scan(len);
@@ -441,34 +480,76 @@ __device__ __forceinline__ void list_round(const PeelArgs& A, const Level& V, co
   tdec += ndec;
 }
 
-// The windows of the shorter rows of edges[0..n).
+// The shorter rows of up to kBigBatch frontier edges, in shared memory: each
+// edge and its other end, where the row starts, how long it is, and the first of
+// its windows.
+struct RowBatch {
+  uint64_t start[kBigBatch];
+  uint32_t first[kBigBatch + 1], len[kBigBatch], edge[kBigBatch], other[kBigBatch];
+  uint32_t tmp[33];
+};
+
+// The windows of the shorter rows of edges[0..n), dealt to every warp.  As
+// deal_windows, but a warp finds its window's row in shared memory: from the
+// frontier through the edges to the offsets is a chain of three accesses, which
+// every window would go through again (828 rounds: 12.4 -> 12.1 ms).
 __device__ __forceinline__ void list_round_windows(const PeelArgs& A, const Level& V, const uint32_t* edges,
                                                    uint64_t n, uint32_t r, uint32_t* next, unsigned long long* ncnt,
-                                                   uint64_t* woff, uint64_t* tmp, uint64_t& tdec) {
+                                                   RowBatch& B, uint64_t& tdec) {
+  constexpr uint32_t kWin = 32 * kJobWide;
+  const uint32_t gwarps = gridDim.x * (blockDim.x >> 5), gwarp = blockIdx.x * (blockDim.x >> 5) + warp_id();
+  const uint32_t per = kBigBatch / blockDim.x;  // rows per thread
   uint32_t ndec = 0;
-  deal_windows<32 * kJobWide>(
-      n,
-      [&](uint64_t x) {
-        uint32_t s, o;
-        shorter_row(A, edges[x], s, o);
-        return s;
-      },
-      A.off, woff, tmp, [&](uint64_t x, uint64_t b, uint64_t e) {
-        const uint32_t f = edges[x];
-        uint32_t s, o;
-        shorter_row(A, f, s, o);
-        uint32_t ee[kJobWide], oo[kJobWide];
-        uint64_t j[kJobWide];
-        bool ok[kJobWide];
+  for (uint64_t base = 0; base < n; base += kBigBatch) {
+    const uint32_t cnt = (uint32_t)min((uint64_t)kBigBatch, n - base);
+    uint32_t sum = 0;
+    for (uint32_t j = 0; j < per; ++j) {
+      const uint32_t x = threadIdx.x * per + j;
+      if (x >= cnt) break;
+      const uint32_t e = edges[base + x];
+      uint32_t s, o;
+      shorter_row(A, e, s, o);
+      const uint32_t l = A.rlen[s];
+      B.start[x] = A.off[s];
+      B.len[x] = l;
+      B.edge[x] = e;
+      B.other[x] = o;
+      sum += (l + kWin - 1) / kWin;
+    }
+    uint32_t total;
+    uint32_t pre = block_excl_scan<uint32_t>(sum, B.tmp, &total);
+    for (uint32_t j = 0; j < per; ++j) {
+      const uint32_t x = threadIdx.x * per + j;
+      if (x >= cnt) break;
+      B.first[x] = pre;
+      pre += (B.len[x] + kWin - 1) / kWin;
+    }
+    __syncthreads();
+    for (uint32_t u = gwarp; u < total; u += gwarps) {
+      uint32_t lo = 0, hi = cnt;  // last row with first <= u
+      while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (B.first[mid] <= u)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      const uint32_t at = (u - B.first[lo]) * kWin, len = B.len[lo];
+      uint32_t ee[kJobWide], oo[kJobWide];
+      uint64_t j[kJobWide];
+      bool ok[kJobWide];
 #pragma unroll
-        for (unsigned t = 0; t < kJobWide; ++t) {
-          ee[t] = f;
-          oo[t] = o;
-          j[t] = b + 32 * t + lane_id();
-          ok[t] = j[t] < e;
-        }
-        close_entries<kJobWide>(A, V, ee, oo, j, ok, r, next, ncnt, ndec);
-      });
+      for (unsigned t = 0; t < kJobWide; ++t) {
+        const uint32_t p = at + 32 * t + lane_id();
+        ee[t] = B.edge[lo];
+        oo[t] = B.other[lo];
+        j[t] = B.start[lo] + p;
+        ok[t] = p < len;
+      }
+      close_entries<kJobWide>(A, V, ee, oo, j, ok, r, next, ncnt, ndec);
+    }
+    __syncthreads();
+  }
   tdec += ndec;
 }
 
@@ -701,10 +782,10 @@ __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcn
 template <bool kLists>
 __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsArgs L) {
   extern __shared__ __align__(16) uint32_t dense_smem[];
-  __shared__ uint64_t woff[kLists ? kBigBatch + 1 : 1];
   __shared__ unsigned long long sh[3];
   __shared__ uint64_t wtmp[33];
-  uint32_t* su = dense_smem + warp_id() * (kLists ? 0 : A.R.W);
+  RowBatch* batch = reinterpret_cast<RowBatch*>(dense_smem);  // lists
+  uint32_t* su = dense_smem + warp_id() * (kLists ? 0 : A.R.W);  // bitsets
   const unsigned long long* src[3] = {nullptr, nullptr, nullptr};
   const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -717,6 +798,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
   uint32_t end = kEndEmpty;
   bool gave_up = false;
   uint64_t left = V.na;  // edges alive (the list may hold dead ones too)
+  uint64_t packed = V.na;  // edges alive when the rows were last packed
   while (true) {
     // Slot (i + 1) % 3 is zero; slot (i + 2) % 3, and the long rows' count
     // that the next round uses, were read before the barrier of the last round.
@@ -756,7 +838,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
             const uint64_t k = A.ends[fr[f]];
             tdeg += (uint64_t)atomicSub(&A.adeg[(uint32_t)(k >> 32)], 1u) + atomicSub(&A.adeg[(uint32_t)k], 1u);
           }
-          list_round_windows(A, V, fr, nf, r, nx, nc, woff, wtmp, tdec);
+          list_round_windows(A, V, fr, nf, r, nx, nc, *batch, tdec);
         } else {
           list_round(A, V, fr, nf, r, nx, nc, bc, tdeg, tdec);
         }
@@ -769,7 +851,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
         if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
         const uint64_t nbig = sh[1];
         if (nbig) {
-          list_round_windows(A, V, A.big, nbig, r, nx, nc, woff, wtmp, tdec);
+          list_round_windows(A, V, A.big, nbig, r, nx, nc, *batch, tdec);
           if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
         }
         alive -= nf;
@@ -915,6 +997,14 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
       V.tval = rec_mn + 2;
     }
     if (end == kEndEmpty && L.max_levels && levels == L.max_levels) end = kEndLevels;
+    // Rows of mostly dead entries are packed: an entry of a row costs its edge's
+    // state whether it is alive or not (truss numbers of an R-MAT scale 16 graph:
+    // levels 12.1 ms without, 11.0 with; at three quarters 11.3).
+    if (kLists && A.pack && left * 2 <= packed) {
+      pack_rows(A, gwarp, gwarps);
+      packed = left;
+      if (!grid_barrier(A.words, A.timeout_ns)) return;
+    }
     // The list is rewritten (in order) once an eighth of it is gone, and for
     // the host; dead entries are passed over until then.
     const bool rewrite = end != kEndEmpty || left * 8 <= V.na * 7;
@@ -1096,6 +1186,7 @@ struct Peeler {
   uint32_t* sup;
   uint32_t* truss;
   DBuf state, alive[2], front[2], cnt, out, mm, adeg, acct, table, big;
+  DBuf rows_len, rows_adj, rows_eid;  // list mode: PeelArgs::rlen, radj, reid
   uint32_t table_bits = 0;
   uint64_t scanned = 0;  // alive-list entries scanned by level frontiers
   int ai = 0;
@@ -1134,9 +1225,9 @@ struct Peeler {
     threads = kLevelThreads;
     auto rows_smem = [&] { return s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, threads); };
     while (threads > 256 && rows_smem() > kRowsSmem) threads /= 2;
-    smem = rows_smem();
     coop_grid = 0;
     build_table();
+    smem = table.get() ? sizeof(RowBatch) : rows_smem();
     if (c->opt.persistent || s->W) {
       allow_max_dynamic_smem(kernel());
       int per_sm = 0;
@@ -1155,17 +1246,35 @@ struct Peeler {
   void build_table() {
     table.release();
     big.release();
+    rows_len.release();
+    rows_adj.release();
+    rows_eid.release();
     if (s->W || !c->opt.persistent) return;
     table_bits = 10;
     while (table_bits < 32 && (2ull << table_bits) < 5 * s->m) ++table_bits;
-    const uint64_t bytes = (8ull << table_bits) + s->m * sizeof(uint32_t);
-    if ((2ull << table_bits) < 5 * s->m || (c->budget && c->in_use + bytes + (1u << 20) > c->budget)) return;
+    const uint64_t bytes = (8ull << table_bits) + (s->m + s->n) * sizeof(uint32_t);
+    // (Beside it, what the levels may ask for later: snapshots, a rebuilt graph.)
+    const uint64_t later = (truss ? 0 : 32 * s->m) + (1u << 20);
+    if ((2ull << table_bits) < 5 * s->m || (c->budget && c->in_use + bytes + later > c->budget)) return;
     table.alloc(c, 8ull << table_bits);
     big.alloc(c, s->m * sizeof(uint32_t));
     KT_CUDA(cudaMemsetAsync(table.get(), 0xff, 8ull << table_bits, c->stream));
     k_table_build<<<grid_for(s->m, 256, c->num_sms * 16), 256, 0, c->stream>>>(
         s->m, s->ends.as<uint64_t>(), table.as<unsigned long long>(), table_bits);
     KT_LAUNCHED(c);
+    rows_len.alloc(c, s->n * sizeof(uint32_t));
+    k_row_lengths<<<grid_for(s->n, 256, c->num_sms * 16), 256, 0, c->stream>>>(s->off.as<uint64_t>(), s->n,
+                                                                             rows_len.as<uint32_t>());
+    KT_LAUNCHED(c);
+    // Rows that may be packed, when every level is peeled and there is room for
+    // a copy.
+    const uint64_t rows = 2 * s->m * sizeof(uint32_t);
+    if (!truss || (c->budget && c->in_use + 2 * rows + (1u << 20) > c->budget)) return;
+    lower_ids(c, *s);
+    rows_adj.alloc(c, rows);
+    rows_eid.alloc(c, rows);
+    KT_CUDA(cudaMemcpyAsync(rows_adj.get(), s->adj.get(), rows, cudaMemcpyDeviceToDevice, c->stream));
+    KT_CUDA(cudaMemcpyAsync(rows_eid.get(), s->eid.get(), rows, cudaMemcpyDeviceToDevice, c->stream));
   }
 
   PeelArgs args(uint32_t t) {
@@ -1204,6 +1313,11 @@ struct Peeler {
     A.table = table.as<unsigned long long>();
     A.table_bits = table_bits;
     A.big = big.as<uint32_t>();
+    A.n = s->n;
+    A.pack = rows_adj.get() && !fail_below;  // (a level tried may be undone)
+    A.radj = rows_adj.get() ? rows_adj.as<uint32_t>() : s->adj.as<uint32_t>();
+    A.reid = rows_eid.get() ? rows_eid.as<uint32_t>() : s->eid.as<uint32_t>();
+    A.rlen = rows_len.as<uint32_t>();
     A.fail_below = fail_below;
     return A;
   }

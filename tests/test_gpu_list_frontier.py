@@ -36,3 +36,28 @@ def test_rounds_at_the_line(edges, persistent):
         assert int((want == 2).sum()) == edges
         assert np.array_equal(dg.trussness(), want)
         dg.free()
+
+
+@pytest.mark.parametrize("budget", [0, 1])
+def test_rows_packed_as_edges_leave(budget):
+    """Many levels over which the edges halve several times, with room for the
+    rows' copies and (a budget just below the peak with them) without."""
+    rng = np.random.default_rng(8)
+    parts = [np.stack(np.triu_indices(n, 1), 1) + off for n, off in
+             [(20, 0), (40, 10), (80, 30), (120, 70), (160, 150)]]
+    parts.append(rng.integers(0, 3000, (60_000, 2)))
+    e = np.concatenate(parts)
+    with K.Context(0) as ctx:
+        ctx.set_option("dense_max_n", 0)
+        dg = ctx.load_edges(e)
+        want = O.trussness(dg.edges())
+        ctx.reset_stats()
+        assert np.array_equal(dg.trussness(), want)
+        peak = ctx.stats()["device_bytes_peak"]
+        dg.free()
+    if budget:
+        with K.Context(0, hbm_budget=peak - (1 << 16)) as ctx:
+            ctx.set_option("dense_max_n", 0)
+            dg = ctx.load_edges(e)
+            assert np.array_equal(dg.trussness(), want)
+            dg.free()
