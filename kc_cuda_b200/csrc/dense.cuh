@@ -162,18 +162,21 @@ __device__ __forceinline__ void take_same_row(unsigned& todo, uint32_t u, uint32
 }
 
 // Rows of at most kShortRow words: eight lanes per edge, two edges per lane
-// in flight, so a warp works on eight edges at once, and both rows come
-// straight from L2.  With a warp per edge a row of 44 words kept 11 lanes of
-// 32 busy, and a group's 16 pairs of edges waited one after another (609,432
-// edges, rows of 44 words: 32 rounds, 25 of them recounts, 1.10 -> 0.78 ms).  Beyond 64 words a row fills
-// the warp, and row u is worth keeping in shared memory.
+// in flight, so a warp works on eight edges at once.  With a warp per edge a row
+// of 44 words kept 11 lanes of 32 busy, and a group's 16 pairs of edges waited
+// one after another (609,432 edges, rows of 44 words: 32 rounds, 25 of them
+// recounts, 1.10 -> 0.78 ms).  Eight lanes take `span` consecutive edges of the
+// list and keep row u in registers while they share it, which halves what is read
+// from L2 (the Chung-Lu solve, 97 recounts of such rows, 15.7 -> 15.2 ms).
+// Beyond 64 words a row fills the warp, and row u is worth keeping in shared
+// memory.
 constexpr uint32_t kShortRow = 64;
 
-// dense_group (below) for such rows.
+// dense_group (below) for such rows; the group has 4 * span entries, span even.
 __device__ __forceinline__ void dense_group_short(const uint32_t* list, uint64_t base, uint64_t cnt,
                                                   const uint64_t* __restrict__ ends, const DenseRows& R,
-                                                  const uint32_t* state, uint32_t& my_e, uint32_t& my_s, bool& my_ok,
-                                                  unsigned long long* wr = nullptr) {
+                                                  const uint32_t* state, unsigned span, uint32_t& my_e,
+                                                  uint32_t& my_s, bool& my_ok, unsigned long long* wr = nullptr) {
   const unsigned l = lane_id();
   const uint64_t idx = base + l;
   uint32_t e = 0, u = 0, v = 0;
@@ -191,28 +194,45 @@ __device__ __forceinline__ void dense_group_short(const uint32_t* list, uint64_t
   my_ok = ok;
   my_s = 0;
   const unsigned todo = __ballot_sync(kFull, ok);
-  for (unsigned j0 = 0; j0 < 32 && (todo >> j0); j0 += 8) {
-    uint32_t c[2];
+  if (!todo) return;
+  const unsigned sub = l >> 3, i = l & 7;
+  uint4 ru[2];  // this lane's vectors of row cu
+  uint32_t cu = 0xffffffffu;
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  ru[0] = ru[1] = z;
+  for (unsigned jj = 0; jj < span; jj += 2) {
+    uint32_t uj[2], n4[2], c[2] = {0u, 0u};
+    uint4 rv[2][2];
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const unsigned j = j0 + 4 * q + (l >> 3);
-      const uint32_t uj = __shfl_sync(kFull, u, j), vj = __shfl_sync(kFull, v, j);
-      c[q] = 0;
-      if ((todo >> j) & 1u) {
-        const uint32_t W = R.words(uj);
-        const uint4* pu = reinterpret_cast<const uint4*>(R.bits + R.off(uj));
-        const uint4* pv = reinterpret_cast<const uint4*>(R.bits + R.off(vj));
-        for (uint32_t i = l & 7; i < W / 4; i += 8) c[q] += popc_and4(__ldcg(pu + i), __ldcg(pv + i));
-        if (wr && (l & 7) == 0) *wr += 2 * W;
+      const unsigned j = sub * span + jj + q;
+      uj[q] = __shfl_sync(kFull, u, j);
+      const uint32_t vj = __shfl_sync(kFull, v, j);
+      n4[q] = (todo >> j) & 1u ? R.words(vj) / 4 : 0u;
+      const uint4* pv = reinterpret_cast<const uint4*>(R.bits + R.off(vj));
+      rv[q][0] = i < n4[q] ? __ldcg(pv + i) : z;
+      rv[q][1] = i + 8 < n4[q] ? __ldcg(pv + i + 8) : z;
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (!n4[q]) continue;
+      if (uj[q] != cu) {
+        const uint4* pu = reinterpret_cast<const uint4*>(R.bits + R.off(uj[q]));
+        ru[0] = i < n4[q] ? __ldcg(pu + i) : z;
+        ru[1] = i + 8 < n4[q] ? __ldcg(pu + i + 8) : z;
+        cu = uj[q];
+        if (wr && i == 0) *wr += 4 * n4[q];
       }
+      c[q] = popc_and4(ru[0], rv[q][0]) + popc_and4(ru[1], rv[q][1]);
+      if (wr && i == 0) *wr += 4 * n4[q];
     }
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) c[q] += __shfl_xor_sync(kFull, c[q], o);
-      const uint32_t x = __shfl_sync(kFull, c[q], (l & 3) * 8);
-      if (l >= j0 + 4 * q && l < j0 + 4 * q + 4) my_s = x;
+      const uint32_t x = __shfl_sync(kFull, c[q], (l / span * 8) & 31);
+      if (l < 4 * span && l % span == jj + q) my_s = x;
     }
   }
 }

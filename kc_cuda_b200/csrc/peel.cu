@@ -700,7 +700,7 @@ __device__ __forceinline__ void recount_round(const PeelArgs& A, const Level& V,
     bool ok;
     const uint64_t last = min(V.na, (uint64_t)(g + 1) * size);
     if (A.R.W <= kShortRow)
-      dense_group_short(V.alive, g * size, last, A.ends, A.R, A.state, e, sc, ok);
+      dense_group_short(V.alive, g * size, last, A.ends, A.R, A.state, size / 4, e, sc, ok);
     else
       dense_group<2>(V.alive, g * size, last, A.ends, A.R, A.state, su, e, sc, ok);
     trec += __popc(__ballot_sync(kFull, ok));

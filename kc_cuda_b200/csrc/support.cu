@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(256) k_dense_support_short(uint64_t m, const u
   for (uint64_t g = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g * size < m; g += warps) {
     uint32_t e, s;
     bool ok;
-    dense_group_short(order, g * size, min(m, (g + 1) * size), ends, R, nullptr, e, s, ok, &wr);
+    dense_group_short(order, g * size, min(m, (g + 1) * size), ends, R, nullptr, size / 4, e, s, ok, &wr);
     if (ok) sup[e] = s;
   }
   wr = warp_sum(wr);

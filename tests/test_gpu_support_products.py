@@ -4,6 +4,7 @@ more tiles than blocks, sparse and empty parts of a dense matrix."""
 import numpy as np
 import pytest
 
+import kt_oracle as O
 import kc_cuda_b200 as K
 
 pytestmark = pytest.mark.gpu
@@ -30,6 +31,23 @@ def test_support_is_the_square(n, p, hole):
         e = d.edges()
         got = d.tricount()
         assert np.array_equal(got, square[e >> 32, e & 0xffffffff])
+        d.free()
+
+
+@pytest.mark.parametrize("n", [5, 40, 127, 129, 1000, 1025, 2048])
+def test_short_rows(n):
+    """Rows of 4 to 64 words, by popcounts: both vectors of a lane, runs of edges
+    that share a row and ends of the list within a group."""
+    a = dense(n, 0.3 if n > 200 else 0.8, n)
+    u, v = np.nonzero(np.triu(a))
+    b = a.astype(np.float32)
+    square = (b @ b).astype(np.uint32)
+    with K.Context(0) as ctx:
+        ctx.set_option("dense_min_fill", 1000)
+        d = ctx.load_edges(np.stack([u, v], 1))
+        e = d.edges()
+        assert np.array_equal(d.tricount(), square[e >> 32, e & 0xffffffff])
+        assert np.array_equal(d.trussness(), O.trussness(e))
         d.free()
 
 
