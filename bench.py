@@ -596,16 +596,6 @@ def run_reference(args, rank, threads):
     print(json.dumps(line))
 
 
-# DRAM traffic of the dense support kernel, from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum) of a k_dense_support launch
-# on the core55k-support case of cases.py: G(n=55455, 95M draws), whose core
-# has the bench graph's search-core shape (92.1M edges, rows of 1736 words);
-# the launch read 166.3G row words.  The bench graph's launches are too large
-# to capture under the profiling size rule, so their traffic is scaled from
-# this one by the row words each launch reads.
-SUPPORT_CAPTURE = {"dram_bytes": 6_683_428_000 + 373_861_632, "row_words": 166_313_504_560}
-
-
 def roofline(name, kbytes, kms, klaunch, steps, hbm, peak_kind, **extra):
     achieved = (kbytes / (kms / 1000.0)) / 1e9 if kms > 0 else 0.0
     r = {"kernel": name, "bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
@@ -680,21 +670,14 @@ def run_single(args, world, rank, local, pg, threads):
 
     hbm, peak_kind = load_peaks()
     S = args.steps
-    sup_traffic = None
-    if SUPPORT_CAPTURE and sup_launch:
-        per_word = SUPPORT_CAPTURE["dram_bytes"] / SUPPORT_CAPTURE["row_words"]
-        sup_traffic = per_word * acc["support_row_words"] / sup_launch
     roof_sup = roofline(
-        "support: k_dense_support (edge support by bitset AND/popcount, all launches of a solve)",
+        "support: k_support_mma, k_dense_support (edge support by products of byte rows or by AND/popcount of "
+        "bitsets, all launches of a solve)",
         acc["support_kernel_bytes"], acc["ms_support_kernel"], sup_launch, S, hbm, peak_kind,
-        bytes_model="row words the kernels read (row u loads, row v words ANDed) x 4 + 16 per edge",
+        bytes_model="words the kernels read (tiles' byte rows; row u loads, row v words ANDed) x 4 + 16 per edge",
         merge_model_bytes_per_step=acc["support_bytes"] / S, row_words_per_step=acc["support_row_words"] / S)
-    roof_sup["traffic"] = sup_traffic
-    if sup_traffic is not None:
-        roof_sup["traffic_basis"] = ("DRAM bytes per row word of the core55k-support capture x the row words "
-                                     "of an average launch here")
     roof_peel = roofline(
-        "peel: k_cascade (one cooperative launch per truss level)", acc["peel_bytes"], acc["ms_peel_kernel"],
+        "peel: k_levels (the levels of a peel in one cooperative launch)", acc["peel_bytes"], acc["ms_peel_kernel"],
         peel_launch, S, hbm, peak_kind,
         bytes_model="8 per alive-degree unit of each deleted edge + 8 per support decrement + 4 per alive-list "
                     "entry scanned",
@@ -761,7 +744,7 @@ def run_single(args, world, rank, local, pg, threads):
             "device_step_ms": [round(x, 1) for x in dev_ms],
             "roofline": dict(dominant, note=(
                 "dense support rows are read mostly from L2 (tile order), so frac near 1 of the HBM copy "
-                "bandwidth is L2-served work; traffic is the DRAM share")),
+                "bandwidth is L2-served work")),
             "rooflines": {"support": roof_sup, "peel": roof_peel},
             "stage_ms": dict({k: round(stats_last[k], 3) for k in
                               ("ms_parse", "ms_csr", "ms_kcore", "ms_subgraph", "ms_support", "ms_peel")},

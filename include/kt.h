@@ -73,7 +73,7 @@ const char* kt_status_string(kt_status s);
  *                               much at once (allocations mid-solve then reuse it)
  *   kcore_big_row (512)         k-core rounds deal longer rows to all warps in
  *                               windows (256 entries in the maximum-core probes,
- *                               32 in the full decomposition)
+ *                               128 in the full decomposition)
  *   peel_search_ratio (16)      peel: per-lane binary search when one row is this
  *                               many times longer than the other
  *   dense_tile_mb (48)          dense support: bitset rows of two tile blocks fit
@@ -91,7 +91,8 @@ const char* kt_status_string(kt_status s);
  *                               graph's edges (0 = never)
  *   peel_split (16)             peel: a round whose frontier edges x 8-word row
  *                               chunks <= this x warps deals (edge, chunk) units
- *                               to warps instead of edges (0 = off)
+ *                               to warps instead of edges, in chunks of 1 to 8
+ *                               words (0 = off)
  *   serve_lanes (2)             serving: waves in flight at once, 1..4
  *   serve_small_mb (128)        serving with two or more lanes: the last lane admits
  *                               only requests whose estimated footprint is at most
@@ -322,8 +323,9 @@ typedef struct kt_stats {
   /* Bytes the support kernels that ran moved, by their own access pattern:
    * for the dense (bitset) kernels 4 per row word read (row u loads, and the
    * words of row v actually ANDed, so a capped count's abandoned segments are
-   * not counted) plus 16 per edge (list entry, ends, result); for the list
-   * kernels the merge model of support_bytes. */
+   * not counted; of a product, the words of byte rows its tiles read) plus 16
+   * per edge (list entry, ends, result); for the list kernels the merge model
+   * of support_bytes. */
   uint64_t support_kernel_bytes;
   uint64_t support_row_words;               /* the dense kernels' row words read */
   uint64_t peel_recount_bytes;              /* bitset rows read by the peel's recount rounds */

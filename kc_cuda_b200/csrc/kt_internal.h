@@ -56,7 +56,7 @@ struct Options {
   int64_t debug_checks = 0;       // extra host-side consistency checks
   int64_t verbose = 0;            // stage decisions on stderr
   int64_t pool_reserve_mb = 0;    // setting it grows the memory pool by this much at once
-  int64_t kcore_big_row = 512;    // k-core rounds: longer rows are dealt to all warps in 32-entry windows
+  int64_t kcore_big_row = 512;    // k-core rounds: longer rows are dealt to all warps in windows
   int64_t peel_search_ratio = 16; // peel: binary-search the long row when it is this many times longer
   int64_t dense_tile_mb = 48;     // dense support: bitset rows of two tile blocks within this many MB
   int64_t kcore_blocks_per_sm = 0;  // core decomposition: resident blocks per SM (0 = as many as fit)
@@ -64,7 +64,7 @@ struct Options {
   int64_t peel_bitset = 1;        // peel: dense rows intersected as bitsets when shorter than the lists
   int64_t kcore_compact = 4;      // max-core search: compact once the core's edges are < 1/this of the graph's (0 = never)
   int64_t wave_budget_pct = 50;   // batch: a wave's estimated footprint within this % of the free budget
-  int64_t peel_split = 16;        // peel: (edge, 8-word chunk) units when frontier x chunks <= this x warps (0 = off)
+  int64_t peel_split = 16;        // peel: (edge, chunk of at most 8 words) units when frontier x chunks <= this x warps (0 = off)
   int64_t serve_lanes = 2;        // serving: waves in flight at once (each on a stream of its own)
   int64_t serve_small_mb = 128;   // serving, two or more lanes: the last lane admits only requests this small (0: any)
   int64_t serve_small_coop = 0;   // serving: the small lane's kernels cooperative (1) or host-stepped (0)

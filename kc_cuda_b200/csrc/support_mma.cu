@@ -376,7 +376,9 @@ bool product_pays(uint64_t m, uint32_t W, uint64_t tiles, unsigned sms, bool alo
 
 bool support_products(Ctx* c, const Sub& s, uint32_t* sup, std::vector<uint8_t>& counted, uint64_t* words) {
   *words = 0;
-  if (!s.W || !s.spre.get() || !encode_tiled()) return false;
+  // (Not where rounds are host-stepped: a block here takes an SM's shared memory,
+  // so a lane that runs beside another's cooperative grids would wait for them.)
+  if (!s.W || !s.spre.get() || !c->opt.persistent || !encode_tiled()) return false;
   std::vector<MmaBlock> blocks;
   uint64_t row_bytes = 0;
   auto add = [&](uint64_t first_word, uint32_t v0, uint32_t n, uint32_t W) {
