@@ -24,6 +24,7 @@
 //   scatter (rows unsorted; the k-core stage does not need them sorted, the
 //   subgraph stage re-sorts).
 #include "stages.h"
+#include "teams.h"
 
 namespace kt {
 namespace {
@@ -58,6 +59,17 @@ __global__ void k_fill(const uint64_t* __restrict__ edges, uint64_t m, const uin
       adj[off[v] + atomicAdd(&cur[v], 1u)] = u;
     }
   }
+}
+
+__global__ void k_gather_u64(const uint64_t* __restrict__ at, uint64_t n, const uint64_t* __restrict__ from,
+                             uint64_t* __restrict__ to) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    to[i] = from[at[i]];
+}
+
+__global__ void k_team_errors(const DevWords* __restrict__ team_words, uint32_t nteams, DevWords* words) {
+  for (uint32_t t = threadIdx.x; t < nteams; t += blockDim.x)
+    if (team_words[t].err) atomicOr(&words->err, team_words[t].err);
 }
 
 __global__ void k_max_u32(const uint32_t* __restrict__ a, uint64_t n, uint32_t* out) {
@@ -287,6 +299,22 @@ __global__ void k_not_ascending(const uint64_t* __restrict__ keys, uint64_t n, u
 }
 
 }  // namespace
+
+std::vector<uint64_t> gather_offsets(Ctx* c, const uint64_t* off, const std::vector<uint64_t>& at) {
+  std::vector<uint64_t> out(at.size());
+  DBuf da(c, at.size() * 8), dv(c, at.size() * 8);
+  copy_h2d(c, da.get(), at.data(), at.size() * 8);
+  k_gather_u64<<<grid_for(at.size(), 256, c->num_sms), 256, 0, c->stream>>>(da.as<uint64_t>(), at.size(), off,
+                                                                            dv.as<uint64_t>());
+  KT_LAUNCHED(c);
+  copy_d2h(c, out.data(), dv.get(), at.size() * 8);
+  return out;
+}
+
+void merge_team_errors(Ctx* c, const void* team_words, uint32_t nteams) {
+  k_team_errors<<<1, 64, 0, c->stream>>>(static_cast<const DevWords*>(team_words), nteams, dev_words(c));
+  KT_LAUNCHED(c);
+}
 
 void build_graph(Ctx* c, uint64_t* keys, uint64_t nkeys, uint64_t n, Graph& g, bool lines, bool sorted) {
   // Vertex counts travel as u32 through the later stages: the all-ones id

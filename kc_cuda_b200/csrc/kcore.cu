@@ -27,6 +27,7 @@
 #include "compact.cuh"
 #include "kcore.h"
 #include "rows.cuh"
+#include "teams.h"
 
 namespace kt {
 namespace {
@@ -665,12 +666,6 @@ __device__ __forceinline__ void drop_entries_core(const DecompArgs& A, const uin
   }
 }
 
-__global__ void k_gather_u64(const uint64_t* __restrict__ at, uint64_t n, const uint64_t* __restrict__ from,
-                             uint64_t* __restrict__ to) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    to[i] = from[at[i]];
-}
-
 // The entries of the alive list in each team's vertices, and its least degrees
 // at their start.
 __global__ void k_team_lists(Team* __restrict__ teams, uint32_t nteams, const uint32_t* __restrict__ alive,
@@ -693,10 +688,6 @@ __global__ void k_team_lists(Team* __restrict__ teams, uint32_t nteams, const ui
   }
   teams[t].list0 = at[0];
   teams[t].n_list = at[1] - at[0];
-}
-
-__global__ void k_team_errors(const DevWords* __restrict__ team_words, uint32_t nteams, DevWords* words) {
-  if (threadIdx.x < nteams && team_words[threadIdx.x].err) atomicOr(&words->err, team_words[threadIdx.x].err);
 }
 
 template <bool kTeams>
@@ -1298,39 +1289,12 @@ void KCore::core_numbers(Ctx* c, uint32_t* dcore, const std::vector<uint64_t>* s
 
 namespace kt {
 
-// Teams of a union's graphs (vertices starts[g] .. starts[g + 1]): stretches of
-// graphs of about the same number of edges, a graph beyond that by itself, and
-// blocks by their edges.
+// Teams of a union's graphs (vertices starts[g] .. starts[g + 1]) by edges.
 static std::vector<Team> make_teams(Ctx* c, const Graph& g, const std::vector<uint64_t>& starts, unsigned grid) {
   std::vector<Team> teams;
-  const uint64_t G = starts.size() - 1;
-  const unsigned most = (unsigned)std::min<uint64_t>(std::min<uint64_t>(kMaxTeams, G), grid);
-  if (most < 2 || 2 * g.m < kTeamEntries) return teams;
-  std::vector<uint64_t> at(G + 1);  // first adjacency entry of each graph
-  DBuf ds(c, (G + 1) * 8), da(c, (G + 1) * 8);
-  copy_h2d(c, ds.get(), starts.data(), (G + 1) * 8);
-  k_gather_u64<<<grid_for(G + 1, 256, c->num_sms), 256, 0, c->stream>>>(ds.as<uint64_t>(), G + 1, g.off.as<uint64_t>(),
-                                                                        da.as<uint64_t>());
-  KT_LAUNCHED(c);
-  copy_d2h(c, at.data(), da.get(), (G + 1) * 8);
-  const uint64_t total = at[G];
-  uint64_t first = 0;
-  for (uint64_t i = 1; i <= G; ++i) {
-    // Close the team before a graph that would take it past its share, and at the end.
-    const uint64_t share = total / most + 1;
-    if (i < G && at[i + 1] - at[first] <= share) continue;
-    if (i < G && teams.size() + 1 == most) continue;
-    teams.push_back(Team{0, 0, starts[first], starts[i], 0, at[i] - at[first]});
-    first = i;
-  }
-  if (teams.size() < 2) return {};
-  unsigned block = 0;
-  const unsigned spare = grid - (unsigned)teams.size();
-  for (Team& t : teams) {
-    t.block0 = block;
-    t.blocks = 1 + (unsigned)((double)t.n_list / (double)std::max<uint64_t>(total, 1) * spare);
-    block += t.blocks;
-  }
+  if (starts.size() < 3 || 2 * g.m < kTeamEntries) return teams;
+  for (const TeamSpan& t : split_teams(gather_offsets(c, g.off.as<uint64_t>(), starts), kMaxTeams, grid))
+    teams.push_back(Team{t.block0, t.blocks, starts[t.first], starts[t.last], 0, 0});
   return teams;
 }
 
@@ -1394,8 +1358,7 @@ void KCore::core_numbers_persistent(Ctx* c, uint32_t* dcore, const std::vector<u
                                         c->stream));
     KT_LAUNCHED(c);
     if (!teams.empty()) {
-      k_team_errors<<<1, kMaxTeams, 0, c->stream>>>(words.as<DevWords>(), nteams, dev_words(c));
-      KT_LAUNCHED(c);
+      merge_team_errors(c, words.get(), nteams);
     }
     if (teams.empty()) {
       copy_d2h(c, h, cn.as<unsigned long long>() + 14, sizeof(h));

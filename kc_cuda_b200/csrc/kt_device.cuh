@@ -242,10 +242,10 @@ __device__ __forceinline__ bool grid_barrier_read(DevWords* w, unsigned long lon
   return __syncthreads_and(ok) != 0;
 }
 
-__device__ __forceinline__ bool grid_barrier(DevWords* w, unsigned long long timeout_ns) {
+__device__ __forceinline__ bool grid_barrier(DevWords* w, unsigned long long timeout_ns, Crew crew = Crew()) {
   __shared__ unsigned long long none[1];
   const unsigned long long* const src[1] = {nullptr};
-  return grid_barrier_read<1>(w, timeout_ns, src, none);
+  return grid_barrier_read<1>(w, timeout_ns, src, none, crew);
 }
 
 // One bulk copy by the TMA engine (cp.async.bulk, no multicast) of `bytes`

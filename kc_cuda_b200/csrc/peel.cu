@@ -44,6 +44,7 @@
 #include "dense.cuh"
 #include "rows.cuh"
 #include "subgraph.h"
+#include "teams.h"
 
 namespace kt {
 namespace {
@@ -77,7 +78,7 @@ struct PeelArgs {
   uint32_t* adeg;  // alive degree per vertex (for the byte accounting)
   DenseRows R;     // dense mode: alive adjacency bitsets (R.bits null otherwise)
   float wavg;      // mean words per bitset row
-  uint64_t bit_words;  // words of all bitset rows (a multiple of 4)
+  uint64_t bit0 = 0, bit_words;  // first and number of the bitset rows' words (multiples of 4)
   uint32_t gamma;  // recount round when nf * thr * gamma > alive * wavg
   uint32_t search_ratio;  // binary-search the long row when it is this many times longer
   uint32_t split;         // split rounds when frontier x chunks <= split x warps (0 = never)
@@ -636,7 +637,7 @@ __device__ __forceinline__ void clear_edge_bits(const PeelArgs& A, uint32_t e) {
 // a grid barrier, in the caller) set the bits of the alive-list edges still
 // alive -- fewer atomics than clearing the deleted edges one by one.
 __device__ __forceinline__ void zero_bits(const PeelArgs& A, uint64_t gtid, uint64_t gthreads) {
-  uint4* p = reinterpret_cast<uint4*>(A.R.bits);
+  uint4* p = reinterpret_cast<uint4*>(A.R.bits + A.bit0);
   for (uint64_t w = gtid; w < A.bit_words / 4; w += gthreads) p[w] = make_uint4(0u, 0u, 0u, 0u);
 }
 __device__ __forceinline__ void set_alive_bits(const PeelArgs& A, const Level& V, uint64_t gtid, uint64_t gthreads) {
@@ -680,13 +681,13 @@ constexpr uint64_t kRowsInL2 = 64u << 20;  // bytes of bitset rows that stay in 
 // group waits for, 10 us of a 25 us round of 230,000 edges.
 __device__ __forceinline__ void recount_round(const PeelArgs& A, const Level& V, uint32_t r, uint32_t* next,
                                               unsigned long long* ncnt, unsigned long long* cursor,
-                                              uint64_t& trec, uint32_t* su) {
-  const uint64_t gwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+                                              uint64_t& trec, uint32_t* su, const Crew& crew) {
+  const uint64_t gwarps = (uint64_t)crew.blocks * (blockDim.x >> 5);
   const uint64_t share = V.na / gwarps;
   const uint32_t size = share >= 128 ? 32u : share >= 64 ? 16u : 8u;
   const uint64_t groups = (V.na + size - 1) / size;
   const bool in_l2 = A.bit_words <= kRowsInL2 / 4;
-  uint64_t mine = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp_id();
+  uint64_t mine = (uint64_t)crew.rank * (blockDim.x >> 5) + warp_id();
   for (;;) {
     unsigned long long g = mine;
     if (in_l2) {
@@ -742,6 +743,7 @@ struct LevelsArgs {
   // Batched unions (ngroups > 0): every graph's alive edges and least support
   // of a level, its record and its next threshold.
   uint32_t ngroups;
+  uint32_t group0, group1;  // the graphs whose levels are recorded here
   unsigned long long* gcnt;
   uint32_t* gmin;
   uint32_t* kmax;
@@ -749,7 +751,22 @@ struct LevelsArgs {
   uint32_t* gthr;
   uint32_t* tmax;
   const uint64_t* stop;
+  // Teams of blocks, each with a stretch of the graphs (dense unions): the alive
+  // list is in the teams' order.
+  const struct PeelTeam* teams;
+  uint32_t nteams;
+  uint32_t counters;  // a team's words of PeelArgs::cnt
+  DevWords* team_words;
 };
+
+struct PeelTeam {
+  uint32_t block0, blocks;
+  uint32_t group0, group1;
+  uint64_t list0, na;        // its edges in the alive list
+  uint64_t bit0, bit_words;  // its bitset rows
+  float wavg;
+};
+constexpr unsigned kMaxPeelTeams = 32;  // (their results are read through the context's pinned words)
 
 __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcnt, uint32_t* gmin, uint32_t* kmax,
                                              uint64_t* count, uint32_t* gthr, const uint64_t* stop, bool first) {
@@ -779,16 +796,57 @@ __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcn
 // Two blocks of 512 threads per SM: a barrier of 296 blocks takes 1.6 us, of 592
 // blocks of 256 threads 2.3 (64 mix graphs: 29.6 -> 29.1 ms of levels; one
 // block of 1024 threads waits longer for its own warps on small graphs).
-template <bool kLists>
-__global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsArgs L) {
+//
+// kTeams: the graphs of a union by teams of blocks, as in the core
+// decomposition (Peeler::init_teams): 64 cores of up to 1,340 vertices, 3.9M
+// edges, in step 516 rounds and 15.1 ms, by teams 232 at most and 10.7.
+template <bool kLists, bool kTeams>
+__global__ void __launch_bounds__(kLevelThreads, 2)
+    k_levels(const __grid_constant__ PeelArgs all, const __grid_constant__ LevelsArgs all_levels) {
   extern __shared__ __align__(16) uint32_t dense_smem[];
+  __shared__ __align__(16) unsigned char args_store[sizeof(PeelArgs)], levels_store[sizeof(LevelsArgs)];
+  __shared__ unsigned team_block0, team_blocks;
+  PeelArgs& my_args = *reinterpret_cast<PeelArgs*>(args_store);
+  LevelsArgs& my_levels = *reinterpret_cast<LevelsArgs*>(levels_store);
+  if (kTeams) {
+    if (threadIdx.x == 0) {
+      uint32_t t = 0;
+      while (t + 1 < all_levels.nteams && all_levels.teams[t + 1].block0 <= blockIdx.x) ++t;
+      const PeelTeam T = all_levels.teams[t];
+      team_block0 = T.block0;
+      team_blocks = T.blocks;
+      my_args = all;
+      my_levels = all_levels;
+      my_args.alive += T.list0;
+      my_args.na = T.na;
+      my_args.cap = T.na;
+      my_args.front[0] += T.list0;
+      my_args.front[1] += T.list0;
+      my_args.cnt += (uint64_t)t * all_levels.counters;
+      my_args.words = all_levels.team_words + t;
+      my_args.bit0 = T.bit0;
+      my_args.bit_words = T.bit_words;
+      my_args.wavg = T.wavg;
+      my_args.gthr_max = all.gthr_max + t;
+      my_levels.alive[0] += T.list0;
+      my_levels.alive[1] += T.list0;
+      my_levels.group0 = T.group0;
+      my_levels.group1 = T.group1;
+      my_levels.tmax += t;
+      my_levels.out += t;
+    }
+    __syncthreads();
+  }
+  const PeelArgs& A = kTeams ? my_args : all;
+  const LevelsArgs& L = kTeams ? my_levels : all_levels;
+  const Crew crew = kTeams ? Crew(blockIdx.x - team_block0, team_blocks) : Crew();
   __shared__ unsigned long long sh[3];
   __shared__ uint64_t wtmp[33];
   RowBatch* batch = reinterpret_cast<RowBatch*>(dense_smem);  // lists
   uint32_t* su = dense_smem + warp_id() * (kLists ? 0 : A.R.W);  // bitsets
   const unsigned long long* src[3] = {nullptr, nullptr, nullptr};
-  const uint64_t gthreads = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint64_t gthreads = (uint64_t)crew.blocks * blockDim.x;
+  const uint64_t gtid = (uint64_t)crew.rank * blockDim.x + threadIdx.x;
   const uint64_t gwarps = gthreads >> 5, gwarp = gtid >> 5;
   unsigned long long* kept = A.cnt + kCounters;
   Level V = first_level(A);
@@ -812,7 +870,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
     ++i;
     src[0] = &A.cnt[i % 3];
     src[1] = src[2] = nullptr;
-    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh, crew)) return;
     // The next level's figures, last read before this barrier.
     unsigned long long* fig = A.cnt + 8 + 4 * (levels & 1);
     if (gtid == 0)
@@ -848,11 +906,11 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
         }
         src[0] = nc;
         src[1] = bc;
-        if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+        if (!grid_barrier_read(A.words, A.timeout_ns, src, sh, crew)) return;
         const uint64_t nbig = sh[1];
         if (nbig) {
           list_round_windows(A, V, A.big, nbig, r, nx, nc, *batch, tdec);
-          if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+          if (!grid_barrier_read(A.words, A.timeout_ns, src, sh, crew)) return;
         }
         alive -= nf;
         ++i;
@@ -876,7 +934,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
         if (gtid == 0) A.cnt[6 + ((nrec + 1) & 1)] = 0;
         if (pending > alive - nf) {
           zero_bits(A, gtid, gthreads);
-          if (!grid_barrier(A.words, A.timeout_ns)) return;
+          if (!grid_barrier(A.words, A.timeout_ns, crew)) return;
           set_alive_bits(A, V, gtid, gthreads);
         } else if (cleared + 1 == r) {  // only this round's frontier to clear
           for (uint64_t f = gtid; f < nf; f += gthreads) clear_edge_bits(A, fr[f]);
@@ -885,8 +943,8 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
         }
         cleared = r;
         pending = 0;
-        if (!grid_barrier(A.words, A.timeout_ns)) return;
-        recount_round(A, V, r, nx, nc, &A.cnt[6 + (nrec & 1)], trec, su);
+        if (!grid_barrier(A.words, A.timeout_ns, crew)) return;
+        recount_round(A, V, r, nx, nc, &A.cnt[6 + (nrec & 1)], trec, su, crew);
       } else {
         // Few frontier edges for the grid: deal (edge, chunk) units instead,
         // in the shortest chunks that give every warp one unit at most (a
@@ -902,7 +960,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
       }
       if (gtid == 0) A.cnt[(i + 2) % 3] = 0;  // read at the start of round i-1, next written in round i+1
       src[0] = nc;
-      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+      if (!grid_barrier_read(A.words, A.timeout_ns, src, sh, crew)) return;
       alive -= nf;
       ++i;
       ++rounds;
@@ -913,7 +971,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
     if (!kLists && A.R.bits && pending) {
       if (pending > alive) {
         zero_bits(A, gtid, gthreads);
-        if (!grid_barrier(A.words, A.timeout_ns)) return;
+        if (!grid_barrier(A.words, A.timeout_ns, crew)) return;
         set_alive_bits(A, V, gtid, gthreads);
       } else {
         clear_deleted(A, V, cleared, A.r0 + i, gtid, gthreads);
@@ -922,8 +980,8 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
     cleared = A.r0 + i;
     // What is left, and its least and largest support.  Block b owns
     // [b, b + 1) * stretch of the list.
-    const uint64_t stretch = (V.na + gridDim.x - 1) / gridDim.x;
-    const uint64_t s0 = min(V.na, blockIdx.x * stretch), s1 = min(V.na, s0 + stretch);
+    const uint64_t stretch = (V.na + crew.blocks - 1) / crew.blocks;
+    const uint64_t s0 = min(V.na, crew.rank * stretch), s1 = min(V.na, s0 + stretch);
     uint64_t n = 0;
     uint32_t mn = 0xffffffffu, mx = 0;
     for (uint64_t j0 = s0; j0 < s1; j0 += kListWide * blockDim.x) {
@@ -969,13 +1027,13 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
       atomicMax(&fig[1], (unsigned long long)mx);
     }
     if (threadIdx.x == 0) {
-      kept[blockIdx.x] = n;
+      kept[crew.rank] = n;
       if (n) atomicAdd(&fig[2], (unsigned long long)n);
     }
     src[0] = &fig[0];
     src[1] = &fig[1];
     src[2] = &fig[2];
-    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh)) return;
+    if (!grid_barrier_read(A.words, A.timeout_ns, src, sh, crew)) return;
     rec_mn = 0xffffffffu - (uint32_t)sh[0];
     rec_mx = (uint32_t)sh[1];
     left = sh[2];
@@ -1003,14 +1061,14 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
     if (kLists && A.pack && left * 2 <= packed) {
       pack_rows(A, gwarp, gwarps);
       packed = left;
-      if (!grid_barrier(A.words, A.timeout_ns)) return;
+      if (!grid_barrier(A.words, A.timeout_ns, crew)) return;
     }
     // The list is rewritten (in order) once an eighth of it is gone, and for
     // the host; dead entries are passed over until then.
     const bool rewrite = end != kEndEmpty || left * 8 <= V.na * 7;
     if (rewrite) {
       uint64_t at = 0;
-      for (uint32_t b = threadIdx.x; b < blockIdx.x; b += blockDim.x) at += ld_relaxed_u64(&kept[b]);
+      for (uint32_t b = threadIdx.x; b < crew.rank; b += blockDim.x) at += ld_relaxed_u64(&kept[b]);
       at = block_sum<uint64_t>(at, wtmp);
       uint32_t* to = L.alive[list ^ 1];
       for (uint64_t j0 = s0; j0 < s1; j0 += blockDim.x) {
@@ -1029,9 +1087,9 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
     }
     if (L.ngroups) {
       if (gtid == 0) *L.tmax = 0;
-      if (!grid_barrier(A.words, A.timeout_ns)) return;
+      if (!grid_barrier(A.words, A.timeout_ns, crew)) return;
       uint32_t top = 0;
-      for (uint64_t g = gtid; g < L.ngroups; g += gthreads) {
+      for (uint64_t g = L.group0 + gtid; g < L.group1; g += gthreads) {
         record_group((uint32_t)g, L.gcnt, L.gmin, L.kmax, L.count, L.gthr, L.stop, nkept == 1);
         top = max(top, L.gthr[g]);
       }
@@ -1040,7 +1098,7 @@ __global__ void __launch_bounds__(kLevelThreads, 2) k_levels(PeelArgs A, LevelsA
     // Without a new list or new thresholds nothing was written since the last
     // barrier that the next level reads.
     if (!rewrite && !L.ngroups) continue;
-    if (!grid_barrier(A.words, A.timeout_ns)) return;
+    if (!grid_barrier(A.words, A.timeout_ns, crew)) return;
   }
   flush_tallies(A, tdeg, tdec);
   if (lane_id() == 0 && trec) atomicAdd(&A.acct[2], (unsigned long long)trec);
@@ -1158,6 +1216,22 @@ __global__ void k_track_init(uint64_t m, const uint64_t* __restrict__ ends, cons
   }
 }
 
+// Each team's largest threshold.
+__global__ void k_team_tmax(const PeelTeam* __restrict__ teams, uint32_t nteams, const uint32_t* __restrict__ gthr,
+                            uint32_t* __restrict__ tmax) {
+  const uint32_t t = threadIdx.x;
+  if (t >= nteams) return;
+  uint32_t mx = 0;
+  for (uint32_t g = teams[t].group0; g < teams[t].group1; ++g) mx = max(mx, gthr[g]);
+  tmax[t] = mx;
+}
+
+__global__ void k_team_keys(uint64_t m, const uint32_t* __restrict__ list, const uint32_t* __restrict__ egr,
+                            const uint32_t* __restrict__ team, uint64_t* __restrict__ keys) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x)
+    keys[i] = team[egr[list[i]]];
+}
+
 struct StillAlive {
   const uint32_t* list;
   const uint32_t* state;
@@ -1238,7 +1312,8 @@ struct Peeler {
   }
 
   const void* kernel() const {
-    return table.get() ? (const void*)k_levels<true> : (const void*)k_levels<false>;
+    if (table.get()) return (const void*)k_levels<true, false>;
+    return teams.empty() ? (const void*)k_levels<false, false> : (const void*)k_levels<false, true>;
   }
 
   // List mode: the edge hash table, 8 to 20 bytes an edge, when the budget
@@ -1351,8 +1426,15 @@ struct Peeler {
       L.gthr = gthr.as<uint32_t>();
       L.tmax = tmax.as<uint32_t>();
       L.stop = track->stop;
+      L.group1 = track->ngroups;
     }
-    zero(c, cnt.get(), kCounters * sizeof(unsigned long long));
+    if (!teams.empty()) {
+      L.teams = dteams.as<PeelTeam>();
+      L.nteams = (uint32_t)teams.size();
+      L.counters = kCounters + coop_grid;
+      L.team_words = team_words.as<DevWords>();
+    }
+    zero(c, cnt.get(), teams.empty() ? kCounters * sizeof(unsigned long long) : cnt.bytes());
     cudaEvent_t e0;
     c->timer.begin(c->stream, &c->stats.ms_peel_kernel, &e0);
     const auto t_start = std::chrono::steady_clock::now();
@@ -1361,11 +1443,26 @@ struct Peeler {
     {
       CoopLock coop(c);
       void* p[] = {&A, &L};
-      KT_CUDA(cudaLaunchCooperativeKernel(kernel(), dim3(coop_grid), dim3(threads), p, smem,
-                                          c->stream));
+      KT_CUDA(cudaLaunchCooperativeKernel(kernel(), dim3(teams.empty() ? coop_grid : team_blocks(teams)), dim3(threads),
+                                          p, smem, c->stream));
       KT_LAUNCHED(c);
       c->timer.end(c->stream, e0, &c->stats.ms_peel_kernel);
-      read_checked(c, &h, out.get(), sizeof(h), "truss peel");
+      if (teams.empty()) {
+        read_checked(c, &h, out.get(), sizeof(h), "truss peel");
+      } else {
+        merge_team_errors(c, team_words.get(), (uint32_t)teams.size());
+        LevelsOut each[kMaxPeelTeams];
+        static_assert(sizeof(each) <= 3072, "read through the context's pinned words");
+        read_checked(c, each, out.get(), teams.size() * sizeof(LevelsOut), "truss peel");
+        h = each[0];
+        for (size_t i = 1; i < teams.size(); ++i) {  // the most of each; every team ends empty
+          h.rounds = std::max(h.rounds, each[i].rounds);
+          h.levels = std::max(h.levels, each[i].levels);
+          h.r_next = std::max(h.r_next, each[i].r_next);
+          h.scanned += each[i].scanned;
+          h.recounts += each[i].recounts;
+        }
+      }
     }
     c->stats.peel_launches++;
     KT_LOG(c,
@@ -1468,6 +1565,58 @@ struct Peeler {
     KT_LAUNCHED(c);
     update_tmax();
   }
+  // Teams for the levels of a union with bitset rows of at most kShortRow words:
+  // its alive list is put in their order, where the sort of it has room.  (With
+  // longer rows the recounts of a graph are bound by bandwidth, of which a team
+  // has its share only: 7.3M edges, rows of up to 196 words, 9.4 ms in step and
+  // 10.9 by teams; 3.9M edges, rows of up to 44 words, 15.1 and 10.7.)
+  std::vector<TeamSpan> teams;
+  DBuf dteams, team_words;
+  void init_teams() {
+    constexpr uint64_t kLeastEdges = 1u << 19;  // (smaller unions are no faster by teams)
+    const size_t G = s->group_n.size();
+    if (!s->W || s->W > kShortRow || !s->roff.get() || G != track->ngroups || s->m < kLeastEdges) return;
+    if (c->budget && c->in_use + 40 * s->m > c->budget) return;
+    std::vector<uint64_t> starts(G + 1, 0), words(G + 1, 0);
+    for (size_t g = 0; g < G; ++g) {
+      starts[g + 1] = starts[g] + s->group_n[g];
+      words[g + 1] = words[g] + (uint64_t)s->group_n[g] * (((s->group_n[g] + 31) / 32 + 3) & ~3u);
+    }
+    const std::vector<uint64_t> at = gather_offsets(c, s->off.as<uint64_t>(), starts);
+    const void* by_teams = (const void*)k_levels<false, true>;
+    allow_max_dynamic_smem(by_teams);
+    int per_sm = 0;
+    KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, by_teams, (int)threads, smem));
+    if (per_sm < 1) return;
+    teams = split_teams(at, kMaxPeelTeams, std::min(coop_grid, coop_blocks(c, per_sm)));
+    if (teams.empty()) return;
+    std::vector<PeelTeam> t;
+    std::vector<uint32_t> of(G);  // each graph's team
+    for (const TeamSpan& x : teams) {
+      for (uint64_t g = x.first; g < x.last; ++g) of[g] = (uint32_t)t.size();
+      const uint64_t w = words[x.last] - words[x.first], n = starts[x.last] - starts[x.first];
+      t.push_back(PeelTeam{x.block0, x.blocks, (uint32_t)x.first, (uint32_t)x.last, at[x.first] / 2,
+                           (at[x.last] - at[x.first]) / 2, words[x.first], w,
+                           (float)((double)w / std::max<uint64_t>(n, 1))});
+    }
+    dteams = DBuf(c, t.size() * sizeof(PeelTeam));
+    copy_h2d(c, dteams.get(), t.data(), t.size() * sizeof(PeelTeam));
+    team_words = DBuf(c, t.size() * sizeof(DevWords));
+    zero(c, team_words.get(), team_words.bytes());
+    out = DBuf(c, t.size() * sizeof(LevelsOut));
+    cnt = DBuf(c, t.size() * (kCounters + coop_grid) * sizeof(unsigned long long));
+    tmax = DBuf(c, t.size() * sizeof(uint32_t));
+    k_team_tmax<<<1, kMaxPeelTeams, 0, c->stream>>>(dteams.as<PeelTeam>(), (uint32_t)t.size(), gthr.as<uint32_t>(),
+                                                   tmax.as<uint32_t>());
+    KT_LAUNCHED(c);
+    DBuf dof(c, G * sizeof(uint32_t)), keys(c, s->m * sizeof(uint64_t));
+    copy_h2d(c, dof.get(), of.data(), G * sizeof(uint32_t));
+    k_team_keys<<<grid_for(s->m, 256, c->num_sms * 16), 256, 0, c->stream>>>(
+        s->m, alive[ai].as<uint32_t>(), egr.as<uint32_t>(), dof.as<uint32_t>(), keys.as<uint64_t>());
+    KT_LAUNCHED(c);
+    radix_sort_u64(c, keys.as<uint64_t>(), alive[ai].as<uint32_t>(), s->m, {{0, bits_for(t.size())}});
+  }
+
   void update_tmax() {
     zero(c, tmax.get(), 4);
     k_max_u32<<<grid_for(track->ngroups, 256, c->num_sms * 4), 256, 0, c->stream>>>(
@@ -1608,6 +1757,7 @@ PeelResult truss_peel(Ctx* c, const Sub& s, uint32_t* sup, uint32_t t0, uint64_t
     if (track->ngroups == 0) return res;
     P.init_track(t0);
     if (P.coop_grid) {
+      P.init_teams();
       P.levels(t, 0, 0, 0);
       P.account();
       return res;

@@ -31,6 +31,7 @@
 #include "stages.h"
 #include "subgraph.h"
 #include "support_mma.h"
+#include "teams.h"
 
 namespace kt {
 namespace {
@@ -351,13 +352,6 @@ CUtensorMap rows_map(void* base, uint32_t n, uint32_t W) {
   return map;
 }
 
-// entries[g]: adjacency entries of the graph on vertices starts[g] .. starts[g + 1].
-__global__ void k_group_entries(const uint32_t* __restrict__ starts, uint32_t groups, const uint64_t* __restrict__ off,
-                                uint64_t* __restrict__ entries) {
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < groups; g += gridDim.x * blockDim.x)
-    entries[g] = off[starts[g + 1]] - off[starts[g]];
-}
-
 // Whether the product of a graph's rows takes less time than a popcount of W
 // words per edge, both with the whole GPU working on graphs like it.  A tile
 // measures 0.55-0.6 us for 128 columns (the rate of the tensor cores) and up to 18
@@ -397,24 +391,18 @@ bool support_products(Ctx* c, const Sub& s, uint32_t* sup, std::vector<uint8_t>&
     constexpr double kLeastWords = 100e6;
     if ((double)s.m * s.W < kLeastWords) return false;
     const uint32_t G = (uint32_t)s.group_n.size();
-    std::vector<uint32_t> starts(G + 1, 0);
+    std::vector<uint64_t> starts(G + 1, 0);
     for (uint32_t g = 0; g < G; ++g) starts[g + 1] = starts[g] + s.group_n[g];
-    std::vector<uint64_t> entries(G);
-    DBuf ds(c, (G + 1) * 4ull), de(c, G * 8ull);
-    copy_h2d(c, ds.get(), starts.data(), (G + 1) * 4ull);
-    k_group_entries<<<grid_for(G, 256, c->num_sms), 256, 0, c->stream>>>(ds.as<uint32_t>(), G, s.off.as<uint64_t>(),
-                                                                         de.as<uint64_t>());
-    KT_LAUNCHED(c);
-    copy_d2h(c, entries.data(), de.get(), G * 8ull);
+    const std::vector<uint64_t> at = gather_offsets(c, s.off.as<uint64_t>(), starts);
     counted.assign(G, 0);
     uint64_t word = 0;
     double gain = 0;
     for (uint32_t g = 0; g < G; ++g) {
       const uint32_t n = s.group_n[g], W = ((n + 31) / 32 + 3) & ~3u;
-      if (n && blocks.size() < 65535 && product_pays(entries[g] / 2, W, tiles_of(n), c->num_sms, false)) {
-        add(word, starts[g], n, W);
+      if (n && blocks.size() < 65535 && product_pays((at[g + 1] - at[g]) / 2, W, tiles_of(n), c->num_sms, false)) {
+        add(word, (uint32_t)starts[g], n, W);
         counted[g] = 1;
-        gain += (double)entries[g] / 2 * W;
+        gain += (double)(at[g + 1] - at[g]) / 2 * W;
       }
       word += (uint64_t)n * W;
     }
