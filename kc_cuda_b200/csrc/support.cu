@@ -615,7 +615,7 @@ void edge_support(Ctx* c, const Sub& s, uint32_t* sup, uint32_t cap, const uint3
   uint64_t left = s.m;  // edges of `order` that the products leave
   DBuf rest;
   std::vector<uint8_t> counted;
-  const bool products = support_products(c, s, sup, counted, &product_words);
+  const bool products = support_products(c, s, sup, cap || (gcap && s.vgid.get()), counted, &product_words);
   if (products) {
     left = 0;
     if (!counted.empty() && std::find(counted.begin(), counted.end(), 0) != counted.end()) {

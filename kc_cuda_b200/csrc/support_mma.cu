@@ -10,11 +10,11 @@
 // 3.07 G words, 12.3 GB, in 1.52 ms for the 9,022-vertex maximum core of an
 // R-MAT scale 22 graph (10.5M edges).  A tile of 256 x 256 reads 512 rows for
 // 65,536 products whatever its edges are, so its traffic and its time follow n^3
-// alone, and product_pays has the line between the two.  That core takes 0.32 ms
-// (0.28 the product: 666 tiles, 0.79 P operations, 2.8 P/s), the 9,109 vertices
-// and 10.6M edges of the search 0.34 instead of 2.62 (capped popcounts), a union
-// of 63,796 vertices, 18.8M edges in graphs of up to 6,178 vertices 0.82 instead
-// of 3.80 ms.
+// alone, and product_pays has the line between the two.  That core takes 0.31 ms
+// (0.27 the product: 666 tiles, 0.75 P operations, 2.8 P/s; 3.4 at 13,000
+// vertices, 4.1 at 36,000), the 9,109 vertices and 10.6M edges of the search 0.34
+// instead of 2.62 (capped popcounts), a union of 63,796 vertices, 18.8M edges in
+// graphs of up to 6,178 vertices 0.82 instead of 3.80 ms.
 //
 // One block per SM keeps a queue of kStages stages, each 128 columns (128
 // bytes) of 256 rows of either side, brought in by TMA with 128-byte swizzling.
@@ -143,6 +143,8 @@ struct MmaArgs {
   unsigned long long timeout_ns;
 };
 
+constexpr uint32_t kSquare = 12;
+
 // Tile t: its block, and its place (i, j) with i <= j.
 __device__ __forceinline__ uint32_t find_tile(const MmaArgs& A, uint64_t t, uint32_t& i, uint32_t& j) {
   uint32_t lo = 0, hi = A.nblocks;
@@ -153,11 +155,33 @@ __device__ __forceinline__ uint32_t find_tile(const MmaArgs& A, uint64_t t, uint
     else
       hi = mid;
   }
+  // Squares of kSquare x kSquare tiles one after another: the tiles in flight
+  // share 2 * kSquare row stretches, where a row of tiles would read every row of
+  // the matrix from memory again once it is beyond L2.
   uint64_t x = t - A.blocks[lo].tile0;
   const uint32_t side = A.blocks[lo].side;
-  i = 0;
-  while (x >= side - i) x -= side - i++;
-  j = i + (uint32_t)x;
+  uint32_t i0 = 0, j0 = 0, rows = min(kSquare, side), cols = rows;
+  while (true) {
+    const uint32_t n = i0 == j0 ? rows * (rows + 1) / 2 : rows * cols;
+    if (x < n) break;
+    x -= n;
+    j0 += kSquare;
+    if (j0 >= side) {
+      i0 += kSquare;
+      j0 = i0;
+      rows = min(kSquare, side - i0);
+    }
+    cols = min(kSquare, side - j0);
+  }
+  if (i0 != j0) {
+    i = i0 + (uint32_t)x % rows;
+    j = j0 + (uint32_t)x / rows;
+  } else {
+    uint32_t y = 0;
+    while (x >= rows - y) x -= rows - y++;
+    i = i0 + y;
+    j = i + (uint32_t)x;
+  }
   return lo;
 }
 
@@ -356,19 +380,26 @@ CUtensorMap rows_map(void* base, uint32_t n, uint32_t W) {
 // words per edge, both with the whole GPU working on graphs like it.  A tile
 // measures 0.55-0.6 us for 128 columns (the rate of the tensor cores) and up to 18
 // beyond that for its counts' way out, the launches and the byte rows about 20 in
-// all; popcounts go at 2.0 G words a millisecond, 1.1 in rows of at most kShortRow.
-// The line lies near 6 % of a large graph's pairs: 2.86M edges on 9,109 vertices
-// (6.9 %) take 0.30 ms as products, 0.43 as popcounts.
-bool product_pays(uint64_t m, uint32_t W, uint64_t tiles, unsigned sms, bool alone) {
+// all.  Popcounts of rows of up to kShortRow words go at 1.1 G words a
+// millisecond; of longer ones they take a time per edge up to some 600 words and
+// 3.5 G words a millisecond beyond, capped ones more time per edge but up to 5.5
+// G words for those they abandon.  So the line lies between 4 and 8 % of a
+// graph's pairs (exact counts at 12 %: 9,100 vertices 0.27 ms as products, 0.72
+// as popcounts; 36,000 vertices 11.5 and 23.7 ms; capped counts of 92M edges on
+// 55,455 vertices, 6 %: about 42 and 30).
+bool product_pays(uint64_t m, uint32_t W, uint64_t tiles, unsigned sms, bool alone, bool capped) {
   const double rounds = alone ? (double)((tiles + sms - 1) / sms) : (double)tiles / sms;
   const double product_us = (alone ? 20.0 : 0.0) + rounds * (18.0 + 0.57 * (W / 4));
-  const double popcount_us = (double)m * W / (W <= kShortRow ? 1.1e6 : 2.0e6);
-  return product_us < popcount_us;
+  const double words_per_us = W <= kShortRow ? 1.1e6
+                              : capped       ? std::min(4.1e3 * W, 5.5e6)
+                                             : std::min(5.5e3 * W, 3.5e6);
+  return product_us < (double)m * W / words_per_us;
 }
 
 }  // namespace
 
-bool support_products(Ctx* c, const Sub& s, uint32_t* sup, std::vector<uint8_t>& counted, uint64_t* words) {
+bool support_products(Ctx* c, const Sub& s, uint32_t* sup, bool capped, std::vector<uint8_t>& counted,
+                      uint64_t* words) {
   *words = 0;
   // (Not where rounds are host-stepped: a block here takes an SM's shared memory,
   // so a lane that runs beside another's cooperative grids would wait for them.)
@@ -384,7 +415,7 @@ bool support_products(Ctx* c, const Sub& s, uint32_t* sup, std::vector<uint8_t>&
     return side * (side + 1) / 2;
   };
   if (!s.roff.get()) {
-    if (!product_pays(s.m, s.W, tiles_of(s.n), c->num_sms, true)) return false;
+    if (!product_pays(s.m, s.W, tiles_of(s.n), c->num_sms, true, capped)) return false;
     add(0, 0, s.n, s.W);
   } else {
     // (Its launches have to pay as well: 2e6 words take a microsecond.)
@@ -399,7 +430,7 @@ bool support_products(Ctx* c, const Sub& s, uint32_t* sup, std::vector<uint8_t>&
     double gain = 0;
     for (uint32_t g = 0; g < G; ++g) {
       const uint32_t n = s.group_n[g], W = ((n + 31) / 32 + 3) & ~3u;
-      if (n && blocks.size() < 65535 && product_pays((at[g + 1] - at[g]) / 2, W, tiles_of(n), c->num_sms, false)) {
+      if (n && blocks.size() < 65535 && product_pays((at[g + 1] - at[g]) / 2, W, tiles_of(n), c->num_sms, false, capped)) {
         add(word, (uint32_t)starts[g], n, W);
         counted[g] = 1;
         gain += (double)(at[g + 1] - at[g]) / 2 * W;
