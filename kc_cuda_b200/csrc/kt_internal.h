@@ -127,6 +127,17 @@ class DBuf {
     return *this;
   }
   void alloc(Ctx* c, size_t bytes);
+  // False, and nothing held, where the budget or the device has no room.
+  bool try_alloc(Ctx* c, size_t bytes) {
+    try {
+      alloc(c, bytes);
+    } catch (const Error& e) {
+      if (e.status != KT_ERR_NOMEM) throw;
+      release();
+      return false;
+    }
+    return true;
+  }
   void release();
   // Grows (discarding contents) when smaller than `bytes`.
   void ensure(Ctx* c, size_t bytes) {

@@ -1331,13 +1331,13 @@ struct Peeler {
     // (Beside it, what the levels may ask for later: snapshots, a rebuilt graph.)
     const uint64_t later = (truss ? 0 : 32 * s->m) + (1u << 20);
     if ((2ull << table_bits) < 5 * s->m || (c->budget && c->in_use + bytes + later > c->budget)) return;
-    table.alloc(c, 8ull << table_bits);
-    big.alloc(c, s->m * sizeof(uint32_t));
+    if (!big.try_alloc(c, s->m * sizeof(uint32_t)) || !rows_len.try_alloc(c, s->n * sizeof(uint32_t)) ||
+        !table.try_alloc(c, 8ull << table_bits))
+      return;
     KT_CUDA(cudaMemsetAsync(table.get(), 0xff, 8ull << table_bits, c->stream));
     k_table_build<<<grid_for(s->m, 256, c->num_sms * 16), 256, 0, c->stream>>>(
         s->m, s->ends.as<uint64_t>(), table.as<unsigned long long>(), table_bits);
     KT_LAUNCHED(c);
-    rows_len.alloc(c, s->n * sizeof(uint32_t));
     k_row_lengths<<<grid_for(s->n, 256, c->num_sms * 16), 256, 0, c->stream>>>(s->off.as<uint64_t>(), s->n,
                                                                              rows_len.as<uint32_t>());
     KT_LAUNCHED(c);
@@ -1345,9 +1345,11 @@ struct Peeler {
     // a copy.
     const uint64_t rows = 2 * s->m * sizeof(uint32_t);
     if (!truss || (c->budget && c->in_use + 2 * rows + (1u << 20) > c->budget)) return;
+    if (!rows_adj.try_alloc(c, rows) || !rows_eid.try_alloc(c, rows)) {
+      rows_adj.release();
+      return;
+    }
     lower_ids(c, *s);
-    rows_adj.alloc(c, rows);
-    rows_eid.alloc(c, rows);
     KT_CUDA(cudaMemcpyAsync(rows_adj.get(), s->adj.get(), rows, cudaMemcpyDeviceToDevice, c->stream));
     KT_CUDA(cudaMemcpyAsync(rows_eid.get(), s->eid.get(), rows, cudaMemcpyDeviceToDevice, c->stream));
   }
@@ -1576,7 +1578,9 @@ struct Peeler {
     constexpr uint64_t kLeastEdges = 1u << 19;  // (smaller unions are no faster by teams)
     const size_t G = s->group_n.size();
     if (!s->W || s->W > kShortRow || !s->roff.get() || G != track->ngroups || s->m < kLeastEdges) return;
-    if (c->budget && c->in_use + 40 * s->m > c->budget) return;
+    DBuf room;  // for the sort
+    if ((c->budget && c->in_use + 40 * s->m > c->budget) || !room.try_alloc(c, 24 * s->m)) return;
+    room.release();
     std::vector<uint64_t> starts(G + 1, 0), words(G + 1, 0);
     for (size_t g = 0; g < G; ++g) {
       starts[g + 1] = starts[g] + s->group_n[g];

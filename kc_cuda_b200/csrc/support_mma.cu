@@ -441,12 +441,7 @@ bool support_products(Ctx* c, const Sub& s, uint32_t* sup, bool capped, std::vec
   }
   if (c->budget && c->in_use + row_bytes + blocks.size() * 256 + 4096 > c->budget) return false;
   DBuf rows;
-  try {
-    rows.alloc(c, row_bytes);
-  } catch (const Error&) {  // no room: the popcounts need none
-    cudaGetLastError();
-    return false;
-  }
+  if (!rows.try_alloc(c, row_bytes)) return false;  // the popcounts need no room
   // The longest first: a block of the grid takes every 148th tile.
   std::sort(blocks.begin(), blocks.end(), [](const MmaBlock& a, const MmaBlock& b) { return a.W > b.W; });
   std::vector<CUtensorMap> maps;
