@@ -6,18 +6,19 @@
 // degree steps from k to k-1 (atomicSub returns k) joins the next frontier,
 // so every vertex enters a frontier at most once.  The whole search runs in
 // one cooperative launch (k_core_search), which ends early only for a
-// compaction.  Rows of more than
-// kcore_big_row (option, 512) entries are cut into windows dealt to every
-// warp of the grid, so hub rows do not serialise on one warp.
+// compaction.  Rows of more than kcore_big_row (option, 512) entries are cut
+// into windows dealt to every warp of the grid, so hub rows do not serialise on
+// one warp.
 //
 // The search for the maximum core (the reference steps k by a fixed stride
 // with host backups, src/kc.cu:770-884) ramps k geometrically from the
 // current core (each success is permanent; removed vertices keep the probe's
 // tag), then bisects; a probe that empties the graph is undone by reviving
-// its tag and recounting degrees.  The tags of successful probes increase
+// its tag and copying the degrees before it back.  The tags of successful probes increase
 // with their level, which lets any lower core be restored later without a
 // snapshot: revive the vertices whose tag is newer than the last probe at or
-// below that level, recount degrees, and probe once more.
+// below that level, recount degrees, and probe once more; below a compacted
+// copy, in the graph that it was made from, which keeps its tags.
 #include <algorithm>
 #include <chrono>
 #include <cmath>

@@ -11,12 +11,12 @@
 // shorter row of a frontier edge (x, y) are looked up as edges to its other
 // end in a hash table of the edges (list_round).  With bitsets, a warp takes a
 // frontier edge and ANDs the two rows, or where the sorted rows are shorter
-// (and in list mode without a table) merges them: 32-wide tiles of both rows are compared
-// with a 5-step shuffle search, and whichever tile ends lower is retired
-// (both when the ends tie), so every common neighbour is met exactly once;
-// when one row is more than peel_search_ratio (16) times longer the lanes
-// binary-search the long row instead.  A common w closes the triangle {e, a, b}; it is skipped if a or b
-// was deleted in an earlier round.  Each surviving side edge loses one
+// (and in list mode without a table) merges them: 32-wide tiles of both rows
+// are compared with a 5-step shuffle search, and whichever tile ends lower is
+// retired (both when the ends tie), so every common neighbour is met exactly
+// once; when one row is more than peel_search_ratio (16) times longer the lanes
+// binary-search the long row instead.  A common w closes the triangle {e, a, b};
+// it is skipped if a or b was deleted in an earlier round.  Each surviving side edge loses one
 // triangle, decremented by exactly one frontier edge of the triangle (the
 // one with the smallest id among those in this round); an edge whose support
 // steps from t-2 to t-3 joins the next frontier, so each edge enters a
@@ -557,8 +557,8 @@ __device__ __forceinline__ void list_round_windows(const PeelArgs& A, const Leve
 // A decrement round over (frontier edge, chunk of cw words) units, a warp
 // each, so a small frontier of edges with many triangles keeps the whole grid
 // busy (a round of one edge in a core of 1,311 vertices: 13.2 us in chunks of 8
-// words, 5.4 us in the shortest that fill the grid); edges that use the sorted-list merge go whole to the warp of their
-// first chunk.
+// words, 5.4 us in the shortest that fill the grid); edges that use the
+// sorted-list merge go whole to the warp of their first chunk.
 constexpr uint32_t kSplitWords = 8;  // words of a chunk at most
 
 __device__ __forceinline__ void split_round(const PeelArgs& A, const Level& V, const uint32_t* fr, uint32_t nf,

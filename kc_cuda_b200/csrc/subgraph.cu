@@ -6,12 +6,13 @@
 // src/kc.cu:1405-1580, with CPU sorts of the ranks and of every row).  Here:
 // sort (degree << 32 | id) keys for the new order; write every surviving
 // adjacency entry's new column into its new row, and sort each row -- in a
-// shared-memory bitmap of the row's id range when the rows are dense
-// enough, else by one radix sort of (new u << 32 | new v) over all entries;
-// the upper entries (neighbour > row) number the edges row by row (an
+// shared-memory bitmap of the row's id range when the rows are dense enough,
+// else by a warp in registers (long rows by bitmap), or where long rows are many
+// by one radix sort of (new u << 32 | new v) over all entries; the upper entries (neighbour > row) number the edges row by row (an
 // exclusive scan of the upper-part sizes); the row bitsets of dense mode are
 // built; a lower entry (r, c < r) takes the id of (c, r) from the position of
-// r in row c -- a popcount of the bitsets, or a binary search.
+// r in row c -- a popcount of the bitsets, or a binary search -- when something
+// first reads it (lower_ids).
 #include <algorithm>
 #include <vector>
 
