@@ -262,6 +262,10 @@ struct BitField {
 // fields (the least significant first); bits outside them do not count.
 // `keys`/`vals` hold the input and receive the output.
 void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::initializer_list<BitField> fields);
+// Sets *bad unless the keys, so sorted, are want[0..n) (the last pass compares
+// instead of writing; `keys` is left in no useful order).
+void radix_sort_compare(Ctx* c, uint64_t* keys, uint64_t n, std::initializer_list<BitField> fields,
+                        const uint64_t* want, uint32_t* bad);
 // Bits that hold every value below n.
 inline int bits_for(uint64_t n) {
   int b = 0;

@@ -128,14 +128,17 @@ __device__ __forceinline__ void place_tile(const SortShared& S, const uint64_t (
 }
 
 // Scatter of one tile by the digit (key >> shift) & mask; tile_off: the first
-// place of each (digit, tile).
-template <bool kVals>
+// place of each (digit, tile).  kCheck: nothing is written; each key is compared
+// with the one that `want` has in its place, and *bad set where they differ.
+template <bool kVals, bool kCheck>
 __global__ void __launch_bounds__(kSortThreads, kSortBlocks) k_scatter(const uint64_t* __restrict__ keys,
                                                           const uint32_t* __restrict__ vals, uint64_t n, int shift,
                                                           uint32_t mask, uint32_t ntiles,
                                                           const uint32_t* __restrict__ tile_off,
                                                           uint64_t* __restrict__ keys_out,
-                                                          uint32_t* __restrict__ vals_out) {
+                                                          uint32_t* __restrict__ vals_out,
+                                                          const uint64_t* __restrict__ want,
+                                                          uint32_t* __restrict__ bad) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   uint64_t* skeys = reinterpret_cast<uint64_t*>(smem_raw);                  // kSortTile
   uint32_t* svals = reinterpret_cast<uint32_t*>(smem_raw + kSortTile * 8);  // kSortTile (kVals)
@@ -160,9 +163,20 @@ __global__ void __launch_bounds__(kSortThreads, kSortBlocks) k_scatter(const uin
     const uint64_t key = skeys[i];
     const uint32_t q = (uint32_t)(key >> shift) & mask;
     const uint32_t pos = toff[q] + (i - S.dstart[q]);
-    keys_out[pos] = key;
-    if (kVals) vals_out[pos] = svals[i];
+    if (kCheck) {
+      if (want[pos] != key) *bad = 1u;
+    } else {
+      keys_out[pos] = key;
+      if (kVals) vals_out[pos] = svals[i];
+    }
   }
+}
+
+// keys[0..n) against want[0..n).
+__global__ void k_equal_u64(const uint64_t* __restrict__ keys, const uint64_t* __restrict__ want, uint64_t n,
+                            uint32_t* __restrict__ bad) {
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    if (keys[i] != want[i]) *bad = 1u;
 }
 
 // All passes of at most one tile, in place.
@@ -208,7 +222,13 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_tile(uint64_t* __restrict
 
 }  // namespace
 
-void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::initializer_list<BitField> fields) {
+static void sort_passes(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::initializer_list<BitField> fields,
+                        const uint64_t* want, uint32_t* bad) {
+  auto compare = [&] {
+    if (!want || !n) return;
+    k_equal_u64<<<grid_for(n, 256, c->num_sms * 16), 256, 0, c->stream>>>(keys, want, n, bad);
+    KT_LAUNCHED(c);
+  };
   Digits D{};
   for (const BitField& f : fields) {
     // Digits of equal width, at most 8 bits each.
@@ -220,7 +240,10 @@ void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::ini
       D.mask[D.passes++] = (1u << (hi - lo)) - 1;
     }
   }
-  if (n < 2 || D.passes == 0) return;
+  if (n < 2 || D.passes == 0) {
+    compare();
+    return;
+  }
   if (n >= 0xffffffffULL) throw Error(KT_ERR_LIMIT, "radix sort: more than 2^32-1 keys");
   const size_t smem = kSortTile * (vals ? 12 : 8);
   if (n <= kSortTile) {
@@ -232,11 +255,13 @@ void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::ini
       k_sort_tile<false><<<1, kSortThreads, smem, c->stream>>>(keys, nullptr, (uint32_t)n, D);
     }
     KT_LAUNCHED(c);
+    compare();
     return;
   }
   const uint32_t ntiles = (uint32_t)((n + kSortTile - 1) / kSortTile);
-  allow_max_dynamic_smem((const void*)k_scatter<true>);
-  allow_max_dynamic_smem((const void*)k_scatter<false>);
+  allow_max_dynamic_smem((const void*)k_scatter<true, false>);
+  allow_max_dynamic_smem((const void*)k_scatter<false, false>);
+  allow_max_dynamic_smem((const void*)k_scatter<false, true>);
   DBuf keys_alt(c, n * sizeof(uint64_t));
   DBuf vals_alt;
   if (vals) vals_alt.alloc(c, n * sizeof(uint32_t));
@@ -249,12 +274,19 @@ void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::ini
     k_tile_hist<<<ntiles, kSortThreads, 0, c->stream>>>(ksrc, n, D.shift[p], D.mask[p], ntiles, th.as<uint32_t>());
     KT_LAUNCHED(c);
     scan_u32(c, th.as<uint32_t>(), th.as<uint32_t>(), (uint64_t)ntiles * (D.mask[p] + 1));
+    if (want && p + 1 == D.passes) {
+      k_scatter<false, true><<<ntiles, kSortThreads, smem, c->stream>>>(ksrc, nullptr, n, D.shift[p], D.mask[p], ntiles,
+                                                                        th.as<uint32_t>(), nullptr, nullptr, want, bad);
+      KT_LAUNCHED(c);
+      return;
+    }
     if (vals)
-      k_scatter<true><<<ntiles, kSortThreads, smem, c->stream>>>(ksrc, vsrc, n, D.shift[p], D.mask[p], ntiles,
-                                                                 th.as<uint32_t>(), kdst, vdst);
+      k_scatter<true, false><<<ntiles, kSortThreads, smem, c->stream>>>(ksrc, vsrc, n, D.shift[p], D.mask[p], ntiles,
+                                                                        th.as<uint32_t>(), kdst, vdst, nullptr, nullptr);
     else
-      k_scatter<false><<<ntiles, kSortThreads, smem, c->stream>>>(ksrc, nullptr, n, D.shift[p], D.mask[p], ntiles,
-                                                                  th.as<uint32_t>(), kdst, nullptr);
+      k_scatter<false, false><<<ntiles, kSortThreads, smem, c->stream>>>(ksrc, nullptr, n, D.shift[p], D.mask[p],
+                                                                         ntiles, th.as<uint32_t>(), kdst, nullptr,
+                                                                         nullptr, nullptr);
     KT_LAUNCHED(c);
     std::swap(ksrc, kdst);
     std::swap(vsrc, vdst);
@@ -263,6 +295,15 @@ void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::ini
     KT_CUDA(cudaMemcpyAsync(keys, ksrc, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, c->stream));
     if (vals) KT_CUDA(cudaMemcpyAsync(vals, vsrc, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, c->stream));
   }
+}
+
+void radix_sort_u64(Ctx* c, uint64_t* keys, uint32_t* vals, uint64_t n, std::initializer_list<BitField> fields) {
+  sort_passes(c, keys, vals, n, fields, nullptr, nullptr);
+}
+
+void radix_sort_compare(Ctx* c, uint64_t* keys, uint64_t n, std::initializer_list<BitField> fields,
+                        const uint64_t* want, uint32_t* bad) {
+  sort_passes(c, keys, nullptr, n, fields, want, bad);
 }
 
 }  // namespace kt
