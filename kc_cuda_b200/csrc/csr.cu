@@ -378,7 +378,8 @@ void build_graph_sorted(Ctx* c, uint64_t* keys, uint64_t nkeys, uint64_t n, Grap
   } else {
     // Keys are min << 32 | max with both halves below 2^vb - 1; the radix sort
     // runs 2 ceil(vb / 8) passes over the two halves' bits once the "no edge"
-    // key ~0 is rewritten to ((2^vb - 1) << 32) | (2^vb - 1) (still last).  When packing to min << vb | max saves a pass (2 vb bits,
+    // key ~0 is rewritten to ((2^vb - 1) << 32) | (2^vb - 1) (still last).  When
+    // packing to min << vb | max saves a pass (2 vb bits,
     // ceil(2 vb / 8) passes), the keys are packed instead.
     const int vb = bits_for(n + 1);
     const bool small = vb < 32 && nkeys;

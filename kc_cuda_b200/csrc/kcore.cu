@@ -1373,7 +1373,9 @@ void KCore::core_numbers_persistent(Ctx* c, uint32_t* dcore, const std::vector<u
   rounds += h[0];
   probes += h[1];
   check_words(c, "core decomposition");
-  KT_LOG(c, "kt: core decomposition of %llu vertices by %u teams: %llu levels, %llu rounds, %llu passes (%llu full), max core %llu\n",
+  KT_LOG(c,
+         "kt: core decomposition of %llu vertices by %u teams: %llu levels, %llu rounds, %llu passes (%llu full), "
+         "max core %llu\n",
          (unsigned long long)n_alive, nteams, (unsigned long long)h[1], (unsigned long long)h[0],
          (unsigned long long)h[2],
          (unsigned long long)h[3], (unsigned long long)(h[4] ? h[4] - 1 : 0));

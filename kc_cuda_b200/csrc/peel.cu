@@ -150,8 +150,8 @@ __device__ __forceinline__ uint64_t find_sorted(const uint32_t* a, uint64_t lo, 
 
 // Triangle {e, a, b} seen from frontier edge e in round r; returns which of
 // a, b crossed below the threshold (to be pushed).
-__device__ __forceinline__ void close_triangle(const PeelArgs& A, const Level& V, uint32_t e, uint32_t a, uint32_t b, uint32_t r,
-                                               uint32_t thr, bool& pa, bool& pb, uint32_t& ndec) {
+__device__ __forceinline__ void close_triangle(const PeelArgs& A, const Level& V, uint32_t e, uint32_t a, uint32_t b,
+                                               uint32_t r, uint32_t thr, bool& pa, bool& pb, uint32_t& ndec) {
   const uint32_t sa = A.state[a], sb = A.state[b];
   if (sa < r || sb < r) return;  // broken in an earlier round
   if (sa > r && !(sb == r && b < e)) {
@@ -1124,7 +1124,8 @@ __global__ void __launch_bounds__(kLevelThreads, 2)
 // Host-stepped variant (one launch per round), used when cooperative launch
 // is switched off.
 __global__ void __launch_bounds__(kPeelThreads) k_level_frontier(PeelArgs A) {
-  level_frontier(A, first_level(A), A.r0, A.front[0], &A.cnt[0], (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x);
+  level_frontier(A, first_level(A), A.r0, A.front[0], &A.cnt[0], (uint64_t)blockIdx.x * blockDim.x + threadIdx.x,
+                 (uint64_t)gridDim.x * blockDim.x);
 }
 
 __global__ void __launch_bounds__(kPeelThreads) k_round(PeelArgs A, uint32_t i, uint64_t nf) {

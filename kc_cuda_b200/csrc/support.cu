@@ -391,7 +391,8 @@ unsigned dense_grid(Ctx* c, const void* kernel, uint64_t m, size_t smem) {
 }
 
 template <int NQ>
-void launch_exact(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint32_t* sup, unsigned long long* row_words, unsigned long long* cursor) {
+void launch_exact(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint32_t* sup, unsigned long long* row_words,
+                  unsigned long long* cursor) {
   const size_t smem = dense_smem_bytes(s.W, 256);
   const unsigned grid = dense_grid(c, (const void*)k_dense_support<NQ>, m, smem);
   k_dense_support<NQ><<<grid, 256, smem, c->stream>>>(m, order, s.ends.as<uint64_t>(),
@@ -402,7 +403,8 @@ void launch_exact(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint3
 // Exact counts: option support_rows (1, 2 or 4) edges sharing row u per
 // shared-memory read of it.  Capped counts: two edges sharing row u side by
 // side, one per half of the warp.
-void launch_dense_support(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint32_t* sup, bool capped, uint32_t cap, const uint32_t* gcap,
+void launch_dense_support(Ctx* c, const Sub& s, const uint32_t* order, uint64_t m, uint32_t* sup, bool capped,
+                          uint32_t cap, const uint32_t* gcap,
                           unsigned long long* row_words, unsigned long long* cursor) {
   if (s.W <= kShortRow) {  // (exact also where a cap is given: there is little to abandon)
     k_dense_support_short<<<grid_for((m + 7) / 8 * 32, 256, c->num_sms * 8), 256, 0, c->stream>>>(

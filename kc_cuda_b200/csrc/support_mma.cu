@@ -186,8 +186,8 @@ __device__ __forceinline__ uint32_t find_tile(const MmaArgs& A, uint64_t t, uint
 }
 
 // 16 bits of a row -> 16 bytes.
-__global__ void __launch_bounds__(256) k_expand_rows(const uint32_t* __restrict__ bits, const MmaBlock* __restrict__ blocks,
-                                                     uint8_t* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_expand_rows(const uint32_t* __restrict__ bits,
+                                                     const MmaBlock* __restrict__ blocks, uint8_t* __restrict__ out) {
   const MmaBlock B = blocks[blockIdx.y];
   const uint64_t halves = 2ull * B.n * B.W;
   const uint16_t* src = reinterpret_cast<const uint16_t*>(bits + B.words);
@@ -430,10 +430,11 @@ bool support_products(Ctx* c, const Sub& s, uint32_t* sup, bool capped, std::vec
     double gain = 0;
     for (uint32_t g = 0; g < G; ++g) {
       const uint32_t n = s.group_n[g], W = ((n + 31) / 32 + 3) & ~3u;
-      if (n && blocks.size() < 65535 && product_pays((at[g + 1] - at[g]) / 2, W, tiles_of(n), c->num_sms, false, capped)) {
+      const uint64_t m = (at[g + 1] - at[g]) / 2;
+      if (n && blocks.size() < 65535 && product_pays(m, W, tiles_of(n), c->num_sms, false, capped)) {
         add(word, (uint32_t)starts[g], n, W);
         counted[g] = 1;
-        gain += (double)(at[g + 1] - at[g]) / 2 * W;
+        gain += (double)m * W;
       }
       word += (uint64_t)n * W;
     }
