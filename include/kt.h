@@ -62,7 +62,11 @@ const char* kt_status_string(kt_status s);
  *   capped_support (1)          search phase: abandon supports below the threshold
  *   timeout_ms (20000)          bound on every device-side wait, 0..3600000; 0 makes
  *                               every bounded wait give up at once, so a solve
- *                               returns KT_ERR_TIMEOUT (a test of the error path)
+ *                               returns KT_ERR_TIMEOUT (a test of the error path).
+ *                               A tile of a scan waits for its predecessors 10 ms at
+ *                               most and then adds them up itself, which is no error;
+ *                               the waits for a kernel's own copies, which no other
+ *                               block can hold up, have bounds of their own
  *   parse_pipeline_mb (256)     host->device chunk of file ingest, and of host TSV
  *                               bytes parsed chunk by chunk as they land (inputs of
  *                               three chunks or more)

@@ -19,7 +19,7 @@ Lookback begin_lookback(Ctx* c, uint64_t tiles);
 void end_lookback(Ctx* c, uint64_t tiles);
 
 template <class F, typename T>
-__global__ void __launch_bounds__(kCompactThreads) k_compact(uint64_t n, F f, T* __restrict__ out, Lookback L,
+__global__ void __launch_bounds__(kCompactThreads, 8) k_compact(uint64_t n, F f, T* __restrict__ out, Lookback L,
                                                              unsigned long long* __restrict__ count) {
   constexpr unsigned kWarps = kCompactThreads / 32;
   __shared__ uint32_t first[kCompactItems * kWarps];  // kept before each (row, warp) of the tile
@@ -41,7 +41,6 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(uint64_t n, F f, T*
     if (lane == 0) first[i * kWarps + w] = __popc(kept[i]);
   }
   __syncthreads();
-  bool ok = true;
   if (w == 0) {
     static_assert(kCompactItems * kWarps == 64, "two counts per lane");
     const uint32_t a = first[2 * lane], b = first[2 * lane + 1];
@@ -51,13 +50,20 @@ __global__ void __launch_bounds__(kCompactThreads) k_compact(uint64_t n, F f, T*
     first[2 * lane] = incl - a - b;
     first[2 * lane + 1] = incl - b;
     unsigned long long p = 0;
-    if (gridDim.x > 1) p = tile_prefix(L, tile, own, &ok);
+    if (gridDim.x > 1)
+      p = tile_prefix(L, tile, own, false, [&](uint64_t t) {
+        unsigned long long s = 0;
+#pragma unroll 1
+        for (unsigned i = lane; i < kCompactTile; i += 32)
+          s += t * kCompactTile + i < n && f.keep(t * kCompactTile + i);
+        return warp_sum(s);
+      });
     if (lane == 0) {
       sh[1] = p;
-      if (ok && tile == gridDim.x - 1) *count = p + own;
+      if (tile == gridDim.x - 1) *count = p + own;
     }
   }
-  if (!__syncthreads_and(ok)) return;
+  __syncthreads();
   const uint64_t at = sh[1];
 #pragma unroll
   for (unsigned i = 0; i < kCompactItems; ++i)

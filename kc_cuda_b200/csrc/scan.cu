@@ -25,7 +25,8 @@ Lookback begin_lookback(Ctx* c, uint64_t tiles) {
     c->lb_epoch = 1;
   }
   return Lookback{c->lb_status.as<unsigned long long>(), c->lb_ticket.as<unsigned long long>(), c->lb_tickets,
-                  c->lb_epoch, &dev_words(c)->err};
+                  c->lb_epoch,
+                  std::min((unsigned long long)c->opt.timeout_ms * 1000000ULL, kTileWaitNs)};
 }
 void end_lookback(Ctx* c, uint64_t tiles) { c->lb_tickets += tiles; }
 
@@ -35,9 +36,10 @@ constexpr unsigned kScanThreads = 256;
 constexpr unsigned kScanItems = 8;
 constexpr unsigned kScanTile = kScanThreads * kScanItems;
 
-// Exclusive scan.  In-place safe: a tile is read before any of it is written.
+// Exclusive scan.  In-place safe (out is in, or they are apart): a tile is read
+// before any of it is written.
 template <typename Tin, typename Tout>
-__global__ void __launch_bounds__(kScanThreads) k_scan(const Tin* in, Tout* out, uint64_t n, Lookback L) {
+__global__ void __launch_bounds__(kScanThreads, 6) k_scan(const Tin* in, Tout* out, uint64_t n, Lookback L) {
   __shared__ Tout stage[kScanTile];
   __shared__ Tout tmp[33];
   __shared__ unsigned long long sh[2];
@@ -59,16 +61,22 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const Tin* in, Tout* out,
   }
   Tout total;
   const Tout excl = block_excl_scan<Tout>(run, tmp, &total);
-  bool ok = true;
   if (gridDim.x > 1) {
     if (warp_id() == 0) {
-      const unsigned long long p = tile_prefix(L, tile, (unsigned long long)total, &ok);
+      const bool in_place = (const void*)in == (const void*)out;
+      const unsigned long long p = tile_prefix(L, tile, (unsigned long long)total, in_place, [&](uint64_t t) {
+        const volatile Tin* from = in + t * kScanTile;
+        Tout s = 0;
+#pragma unroll 1
+        for (unsigned i = lane_id(); i < kScanTile; i += 32) s += (Tout)(t * kScanTile + i < n ? from[i] : Tin(0));
+        return (unsigned long long)warp_sum(s);
+      });
       if (lane_id() == 0) sh[1] = p;
     }
   } else if (threadIdx.x == 0) {
     sh[1] = 0;
   }
-  if (!__syncthreads_and(ok)) return;
+  __syncthreads();
   const Tout off = (Tout)sh[1] + excl;
 #pragma unroll
   for (unsigned i = 0; i < kScanItems; ++i) stage[threadIdx.x * kScanItems + i] = v[i] + off;
