@@ -46,7 +46,7 @@ constexpr unsigned kMmaThreads = 320;
 constexpr unsigned kOutWarps = 8;
 constexpr size_t kMmaSmem = kStages * kStageBytes + 1024;  // (stages start on 1024 bytes)
 constexpr uint32_t kTmemCols = 512;
-constexpr unsigned long long kDrainNs = 2000000000ULL;  // bound on the last waits of a block that gave up
+constexpr unsigned long long kDrainNs = 2000000000ULL;  // bound on a block's last waits, for its own copies and products
 
 // Instruction descriptor of tcgen05.mma kind::i8: unsigned bytes, 32-bit sums,
 // both sides with consecutive columns in a row, 128 x 256.
@@ -252,12 +252,12 @@ __global__ void __launch_bounds__(kMmaThreads, 1) k_support_mma(MmaArgs A) {
           load_rows(at + kSideBytes, map, k * kDepth, j * kTile, bar);
         }
       }
-      // The copies in flight end before the block does.
-      if (!ok)
-        for (uint32_t x = it > kStages ? it - kStages : 0; x < it; ++x) {
-          volatile uint32_t none = 0;
-          wait_phase(full + 8 * (x % kStages), (x / kStages) & 1, kDrainNs, &none, A.err);
-        }
+      // The copies in flight end before the block does: also where all of them
+      // were issued, since the products may have given up on the last ones.
+      for (uint32_t x = it > kStages ? it - kStages : 0; x < it; ++x) {
+        volatile uint32_t none = 0;
+        wait_phase(full + 8 * (x % kStages), (x / kStages) & 1, kDrainNs, &none, A.err);
+      }
     }
   } else if (warp == 1) {
     if (lane == 0) {
