@@ -48,15 +48,16 @@ __global__ void k_init_state(const uint32_t* __restrict__ deg0, uint64_t n, uint
   }
 }
 
-// Warp-aggregated push of `want` lanes into list[cnt...].
+// Warp-aggregated push of `want` lanes into list[cnt...].  Called by the whole
+// warp.
 __device__ __forceinline__ void push_warp(bool want, uint32_t item, uint32_t* list, unsigned long long* cnt,
                                           uint64_t cap, uint32_t* err) {
-  const unsigned b = __ballot_sync(__activemask(), want);
+  const unsigned b = __ballot_sync(kFull, want);
   if (!b) return;
   const unsigned leader = __ffs(b) - 1;
   unsigned long long base = 0;
   if (lane_id() == leader) base = atomicAdd(cnt, (unsigned long long)__popc(b));
-  base = __shfl_sync(__activemask(), base, leader);
+  base = __shfl_sync(kFull, base, leader);
   if (want) {
     const unsigned long long p = base + __popc(b & lanemask_lt());
     if (p < cap)
