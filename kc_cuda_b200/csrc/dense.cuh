@@ -58,7 +58,7 @@ inline DenseRows dense_rows(const Sub& s) {
 // Shared memory a block of `threads` needs for rows of W words.
 inline size_t dense_smem_bytes(uint32_t W, unsigned threads) { return (size_t)(threads / 32) * W * 4; }
 
-__device__ __forceinline__ void dense_load_row(const uint32_t* __restrict__ p, uint32_t W, uint32_t* su) {
+__device__ __forceinline__ void dense_load_row(const uint32_t* p, uint32_t W, uint32_t* su) {
   const uint4* p4 = reinterpret_cast<const uint4*>(p);
   uint4* s4 = reinterpret_cast<uint4*>(su);
   for (uint32_t i = lane_id(); i < W / 4; i += 32) s4[i] = p4[i];
@@ -240,11 +240,12 @@ __device__ __forceinline__ void dense_group_short(const uint32_t* list, uint64_t
 // One group of up to 32 list entries [base, min(base+32, cnt)).  Entries
 // whose state is not kAlive (when state != nullptr) are skipped.  On return
 // lane j holds (my_e, my_s) of the group's j-th entry, my_ok = counted.
-// su is this warp's W-word slice of shared memory.
+// su is this warp's W-word slice of shared memory.  (The list and the states
+// change between two calls of one launch: they are not __restrict__.)
 template <int NQ = 4>
-__device__ __forceinline__ void dense_group(const uint32_t* __restrict__ list, uint64_t base, uint64_t cnt,
+__device__ __forceinline__ void dense_group(const uint32_t* list, uint64_t base, uint64_t cnt,
                                             const uint64_t* __restrict__ ends, const DenseRows& R,
-                                            const uint32_t* __restrict__ state, uint32_t* su, uint32_t& my_e,
+                                            const uint32_t* state, uint32_t* su, uint32_t& my_e,
                                             uint32_t& my_s, bool& my_ok, unsigned long long* wr = nullptr) {
   const unsigned l = lane_id();
   const uint64_t idx = base + l;
