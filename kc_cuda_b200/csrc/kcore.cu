@@ -346,10 +346,12 @@ struct SearchArgs {
   const uint32_t* adj;
   uint32_t* deg;
   uint32_t* rem;
-  uint32_t* snap;       // degrees before the probe, of the alive vertices
+  uint32_t* snap;       // degrees before the probe, of the alive vertices (not fixed)
   uint32_t* alive[2];   // the list in use, and the one the next is written to
   uint64_t n_alive;
-  uint32_t* front[2];
+  // Frontier of the odd rounds; the even rounds' is the alive list not in use,
+  // which the next list replaces once a probe's rounds are over.
+  uint32_t* front;
   uint32_t* big;
   // [0..2] frontier sizes, [3..4] big-row counts, [5] least degree, [6] sum of
   // degrees; then one kept count per block
@@ -406,6 +408,7 @@ __global__ void __launch_bounds__(kCoreThreads, 2) k_core_search(SearchArgs A) {
   uint32_t list = 0, probes = 0, tag = A.tag, compact = 0;
   uint32_t i = 0;  // round index, continued across probes (it picks the counters)
   bool undo = false;
+  auto front = [&](uint32_t round) { return (round & 1) ? A.front : A.alive[list ^ 1]; };
   while ((hi - lo > 1 || A.fixed) && na && probes < kMaxProbes) {
     uint32_t k;
     if (A.fixed) {
@@ -423,7 +426,7 @@ __global__ void __launch_bounds__(kCoreThreads, 2) k_core_search(SearchArgs A) {
       A.cnt[6] = 0;
     }
     const uint32_t* alive = A.alive[list];
-    WarpList first(items[warp_id()], (i & 1) ? A.front[0] : A.front[1], &A.cnt[(i + 1) % 3], A.cap, &A.words->err);
+    WarpList first(items[warp_id()], front(i + 1), &A.cnt[(i + 1) % 3], A.cap, &A.words->err);
     for (uint64_t j = gtid; j < ((na + 31) & ~31ULL); j += gthreads) {
       bool want = false;
       uint32_t v = 0;
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__(kCoreThreads, 2) k_core_search(SearchArgs A) {
           A.rem[v] = kAlive;
         } else {
           d = A.deg[v];
-          A.snap[v] = d;
+          if (!A.fixed) A.snap[v] = d;
         }
         if (d < k) {
           A.rem[v] = tag;
@@ -463,11 +466,10 @@ __global__ void __launch_bounds__(kCoreThreads, 2) k_core_search(SearchArgs A) {
         empty = true;
         break;
       }
-      const uint32_t* fr = A.front[i & 1];
-      uint32_t* nx = A.front[(i + 1) & 1];
+      const uint32_t* fr = front(i);
       unsigned long long* nc = &A.cnt[(i + 1) % 3];
       unsigned long long* bc = &A.cnt[3 + (i & 1)];
-      WarpList next(items[warp_id()], nx, nc, A.cap, &A.words->err);
+      WarpList next(items[warp_id()], front(i + 1), nc, A.cap, &A.words->err);
       walk_rows(
           fr, nf, A.off, A.adj, A.big_row, A.big, bc, A.cap, &A.words->err,
           [&](const uint32_t(&w)[kWide], const bool(&ok)[kWide]) { drop_entries<kWide>(A, w, ok, k, tag, next); });
@@ -961,7 +963,6 @@ void KCore::compact_to_alive(Ctx* c, uint32_t level) {
   }
   saved.push_back(std::move(sv));
   rem = std::move(snap);
-  alive2.release();
   front[0].release();
   front[1].release();
   big.release();
@@ -1001,8 +1002,7 @@ void KCore::recount(Ctx* c) {
 void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixed, uint64_t compact_below,
                           void* result) {
   const Graph& g = cur();
-  snap.ensure(c, (n ? n : 1) * sizeof(uint32_t));
-  alive2.ensure(c, (n ? n : 1) * sizeof(uint32_t));
+  if (!fixed) snap.ensure(c, (n ? n : 1) * sizeof(uint32_t));
   out.ensure(c, sizeof(SearchOut));
   if (!coop_grid) {
     int per_sm = 0;
@@ -1016,10 +1016,9 @@ void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixe
   A.rem = rem.as<uint32_t>();
   A.snap = snap.as<uint32_t>();
   A.alive[0] = alive.as<uint32_t>();
-  A.alive[1] = alive2.as<uint32_t>();
+  A.alive[1] = front[0].as<uint32_t>();
   A.n_alive = n_alive;
-  A.front[0] = front[0].as<uint32_t>();
-  A.front[1] = front[1].as<uint32_t>();
+  A.front = front[1].as<uint32_t>();
   A.big = big.as<uint32_t>();
   A.cnt = cnt.as<unsigned long long>();
   A.cap = n;
@@ -1047,7 +1046,7 @@ void KCore::search_launch(Ctx* c, uint32_t lo, uint32_t hi, bool ramp, bool fixe
   rounds += h.rounds;
   probes += h.probes;
   n_alive = h.n_alive;
-  if (h.list) std::swap(alive, alive2);
+  if (h.list) std::swap(alive, front[0]);
   for (uint32_t i = 0; i < h.probes; ++i) {
     KT_LOG(c, "kt: k-core probe %u: %u vertices left\n", h.k[i], h.left[i]);
     if (!h.left[i] && !fixed) continue;
@@ -1145,6 +1144,7 @@ uint32_t KCore::find_max_core(Ctx* c) {
                (unsigned long long)n, (unsigned long long)local.m);
       }
     }
+    snap.release();
     cmax = (uint32_t)lo;
     return cmax;
   }

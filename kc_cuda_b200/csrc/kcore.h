@@ -16,10 +16,9 @@ struct KCore {
   DBuf deg;        // uint32[n]: alive degree of alive vertices
   DBuf rem;        // uint32[n]: kAlive, or the tag of the probe that removed it
   DBuf alive;      // uint32[n]: compact list of alive vertices (ascending)
-  DBuf alive2;     // the list the search writes next
   DBuf snap;       // uint32[n]: degrees before a probe of the search
   DBuf out;        // the search's result
-  DBuf front[2];   // frontiers
+  DBuf front[2];   // frontiers (the search writes its next alive list over the first)
   DBuf big;        // rows handled by whole blocks
   DBuf cnt;        // counters
   uint64_t n_alive = 0;

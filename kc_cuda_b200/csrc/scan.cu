@@ -20,7 +20,7 @@ Lookback begin_lookback(Ctx* c, uint64_t tiles) {
     c->lb_tickets = 0;
   }
   if (c->lb_status.bytes() < tiles * sizeof(unsigned long long) || ++c->lb_epoch >= kEpochs) {
-    c->lb_status.ensure(c, std::max<uint64_t>(tiles, 1 << 12) * sizeof(unsigned long long));
+    c->lb_status.ensure(c, std::max<uint64_t>(tiles, 1 << 9) * sizeof(unsigned long long));
     zero(c, c->lb_status.get(), c->lb_status.bytes());
     c->lb_epoch = 1;
   }
