@@ -403,14 +403,13 @@ void kt_destroy(kt_ctx* h) {
     for (auto& e : h->c.ev)
       if (e) cudaEventDestroy(e);
     if (h->c.pinned) cudaFreeHost(h->c.pinned);
-    for (auto& e : h->c.slot_done)
-      if (e) cudaEventDestroy(e);
-    if (h->c.slots) cudaFreeHost(h->c.slots);
     if (h->c.stream) cudaStreamDestroy(h->c.stream);
     if (h->c.copy_stream) cudaStreamDestroy(h->c.copy_stream);
-    // The last context on the device hands the pool's cached memory back,
-    // so the next one (or anything else in the process) can have it.
+    // The last context on the device hands the pool's cached memory and the
+    // pinned slots back, so the next one (or anything else in the process) can
+    // have it.
     if (h->counted && live_contexts(h->c.device, -1) == 0) {
+      kt::release_copy_slots(h->c.device);
       cudaMemPool_t pool;
       if (cudaDeviceGetDefaultMemPool(&pool, h->c.device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
       cudaGetLastError();

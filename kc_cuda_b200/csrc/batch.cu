@@ -217,7 +217,7 @@ void BatchItem::from_pairs(const uint64_t* xy, uint64_t count) {
   extra.resize(count);
   uint64_t* to = extra.data();
   uint32_t mx = 0;
-#pragma omp parallel for schedule(static) num_threads(8) reduction(max : mx) if (count >= (1u << 16))
+#pragma omp parallel for schedule(static) num_threads(copy_threads()) reduction(max : mx) if (count >= (1u << 16))
   for (int64_t i = 0; i < (int64_t)count; ++i) {
     const uint64_t k = xy[i];
     to[i] = k;

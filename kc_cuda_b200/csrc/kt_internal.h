@@ -162,8 +162,6 @@ struct Stats {
 };
 
 constexpr size_t kPinnedBytes = 4096;
-constexpr size_t kSlotBytes = 4 << 20;
-constexpr int kCopySlots = 4;
 
 struct Ctx {
   int device = 0;
@@ -186,10 +184,6 @@ struct Ctx {
   Options opt;
   kt_stats stats{};
   mutable std::recursive_mutex mu;  // every entry point, readers included
-  // Pinned slots for large copies from and to pageable memory (made on first
-  // use, kept with the context), and the event of each slot's last copy.
-  char* slots = nullptr;
-  cudaEvent_t slot_done[kCopySlots] = {};
   // Pinned host words (kPinnedBytes) for small device-to-host reads.
   uint64_t* pinned = nullptr;
   cudaEvent_t ev[8] = {};
@@ -243,6 +237,11 @@ T read_word(Ctx* c, const T* dptr) {
   memcpy(&v, c->pinned, sizeof(T));
   return v;
 }
+// Threads that fill or empty host buffers together, at most.
+int copy_threads();
+// Frees the pinned slots that copies on the device have shared (runtime.cu);
+// called when its last context is gone.
+void release_copy_slots(int device);
 void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes);
 void copy_h2d(Ctx* c, void* dst, const void* src, size_t bytes);
 void zero(Ctx* c, void* dptr, size_t bytes);

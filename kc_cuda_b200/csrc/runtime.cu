@@ -1,11 +1,16 @@
 // Context plumbing: device buffers charged to the HBM budget, small copies,
 // and the CUDA error -> kt::Error conversion.
+#include <omp.h>
+
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
+#include <new>
 #include <set>
 #include <utility>
+#include <vector>
 
 #include "kt_internal.h"
 
@@ -71,33 +76,107 @@ void sync(Ctx* c) { KT_CUDA(cudaStreamSynchronize(c->stream)); }
 
 namespace {
 
-// Whether a copy of `bytes` at host address p goes through the pinned slots:
-// large, and to or from pageable memory, which the driver would stage with one
-// thread (loading and solving 48 MB of records 5.6 -> 3.7 ms, 32 MB of supports
-// counted and returned 6.8 -> 4.9 ms).
-bool through_slots(Ctx* c, const void* p, size_t bytes) {
-  if (bytes < (1 << 20)) return false;
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+constexpr size_t kSlotBytes = 4 << 20;
+constexpr int kCopySlots = 4;
+
+// Pinned slots for large copies from and to pageable memory, which the driver
+// would stage with one thread (48 MB to the device 2.9 -> 1.1 ms, back 2.6 ->
+// 1.0; slots of 1 MB 1.8, of 256 KB 1.9).  Pinning these 16 MB takes 15 ms, so
+// they are made once the copies of a device have lost a part of that to the
+// driver's staging (kSlotsAfter bytes, about 5 ms), and then serve all contexts
+// there: made by a context's first large copy, they cost a program of one call, and
+// each lane of a new server, more than all that they saved it.
+struct CopySlots {
+  int device;
+  char* bytes = nullptr;
+  cudaEvent_t done[kCopySlots] = {};  // each slot's last copy
+  ~CopySlots() {
+    for (cudaEvent_t e : done)
+      if (e) {
+        cudaEventSynchronize(e);
+        cudaEventDestroy(e);
+      }
+    if (bytes) cudaFreeHost(bytes);
     cudaGetLastError();
-    return false;
   }
-  if (a.type != cudaMemoryTypeUnregistered) return false;
-  if (c->slots) return true;
-  if (cudaHostAlloc(reinterpret_cast<void**>(&c->slots), kSlotBytes * kCopySlots, cudaHostAllocDefault) !=
-      cudaSuccess) {
-    cudaGetLastError();
-    c->slots = nullptr;  // no pinned memory to be had: the driver's staging
-    return false;
-  }
-  for (cudaEvent_t& e : c->slot_done)
-    if (!e) KT_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  return true;
+};
+constexpr uint64_t kSlotsAfter = 128ull << 20;
+constexpr int kMostSlots = 4;  // sets on a device: copies at once that have slots
+
+struct SlotPool {
+  std::mutex mu;
+  struct Device {
+    std::vector<CopySlots*> idle;
+    int made = 0;
+    uint64_t staged = 0;  // bytes left to the driver since the last set was made
+  };
+  std::map<int, Device> devices;
+};
+SlotPool& slot_pool() {
+  static SlotPool* p = new SlotPool;  // (never destroyed: contexts may outlive static objects)
+  return *p;
 }
+
+// A set of slots for one copy, where it is large and to or from pageable memory
+// and a set is idle or may be made.
+class SlotLease {
+ public:
+  SlotLease(Ctx* c, const void* p, size_t bytes) {
+    if (bytes < (1 << 20)) return;
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    if (a.type != cudaMemoryTypeUnregistered) return;
+    SlotPool& pool = slot_pool();
+    {
+      std::lock_guard<std::mutex> lk(pool.mu);
+      SlotPool::Device& d = pool.devices[c->device];
+      if (!d.idle.empty()) {
+        s_ = d.idle.back();
+        d.idle.pop_back();
+        return;
+      }
+      d.staged += bytes;
+      if (d.made == kMostSlots || d.staged < kSlotsAfter) return;
+      d.idle.reserve(kMostSlots);  // giving a set back does not allocate
+      d.staged = 0;
+      ++d.made;
+    }
+    CopySlots* s = new (std::nothrow) CopySlots{c->device};
+    bool ok = s && cudaHostAlloc(reinterpret_cast<void**>(&s->bytes), kSlotBytes * kCopySlots,
+                                 cudaHostAllocPortable) == cudaSuccess;
+    for (int i = 0; ok && i < kCopySlots; ++i)
+      ok = cudaEventCreateWithFlags(&s->done[i], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) {
+      s_ = s;
+      return;
+    }
+    cudaGetLastError();  // no pinned memory to be had: the driver's staging
+    delete s;
+    std::lock_guard<std::mutex> lk(pool.mu);
+    --pool.devices[c->device].made;
+  }
+  ~SlotLease() {
+    if (!s_) return;
+    SlotPool& pool = slot_pool();
+    std::lock_guard<std::mutex> lk(pool.mu);
+    pool.devices[s_->device].idle.push_back(s_);
+  }
+  SlotLease(const SlotLease&) = delete;
+  SlotLease& operator=(const SlotLease&) = delete;
+  explicit operator bool() const { return s_ != nullptr; }
+  char* slot(size_t i) const { return s_->bytes + i % kCopySlots * kSlotBytes; }
+  cudaEvent_t done(size_t i) const { return s_->done[i % kCopySlots]; }
+
+ private:
+  CopySlots* s_ = nullptr;
+};
 
 void parallel_memcpy(char* dst, const char* src, size_t n) {
   constexpr int kParts = 8;
-#pragma omp parallel for schedule(static) num_threads(kParts)
+#pragma omp parallel for schedule(static) num_threads(copy_threads())
   for (int t = 0; t < kParts; ++t) {
     const size_t a = n * t / kParts, b = n * (t + 1) / kParts;
     std::memcpy(dst + a, src + a, b - a);
@@ -105,6 +184,24 @@ void parallel_memcpy(char* dst, const char* src, size_t n) {
 }
 
 }  // namespace
+
+int copy_threads() {
+  static const int n = std::max(1, std::min(8, omp_get_num_procs()));
+  return n;
+}
+
+void release_copy_slots(int device) {
+  std::vector<CopySlots*> sets;
+  {
+    SlotPool& pool = slot_pool();
+    std::lock_guard<std::mutex> lk(pool.mu);
+    SlotPool::Device& d = pool.devices[device];
+    sets.swap(d.idle);
+    d.made -= (int)sets.size();
+    d.staged = 0;
+  }
+  for (CopySlots* s : sets) delete s;
+}
 
 void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
@@ -117,21 +214,21 @@ void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
     std::memcpy(dst, c->pinned, bytes);
     return;
   }
-  if (through_slots(c, dst, bytes)) {
+  if (SlotLease slots{c, dst, bytes}) {
     const size_t n = (bytes + kSlotBytes - 1) / kSlotBytes;
     auto size = [&](size_t i) { return std::min(kSlotBytes, bytes - i * kSlotBytes); };
     for (size_t i = 0; i < n + kCopySlots - 1; ++i) {
       if (i < n) {
-        const int s = (int)(i % kCopySlots);
-        KT_CUDA(cudaMemcpyAsync(c->slots + s * kSlotBytes, static_cast<const char*>(src) + i * kSlotBytes, size(i),
+        // (A copy that had the slots before may still read them, on another stream.)
+        if (i < kCopySlots) KT_CUDA(cudaEventSynchronize(slots.done(i)));
+        KT_CUDA(cudaMemcpyAsync(slots.slot(i), static_cast<const char*>(src) + i * kSlotBytes, size(i),
                                 cudaMemcpyDeviceToHost, c->stream));
-        KT_CUDA(cudaEventRecord(c->slot_done[s], c->stream));
+        KT_CUDA(cudaEventRecord(slots.done(i), c->stream));
       }
       if (i + 1 < kCopySlots) continue;  // keep kCopySlots - 1 copies ahead
       const size_t k = i + 1 - kCopySlots;
-      const int s = (int)(k % kCopySlots);
-      KT_CUDA(cudaEventSynchronize(c->slot_done[s]));
-      parallel_memcpy(static_cast<char*>(dst) + k * kSlotBytes, c->slots + s * kSlotBytes, size(k));
+      KT_CUDA(cudaEventSynchronize(slots.done(k)));
+      parallel_memcpy(static_cast<char*>(dst) + k * kSlotBytes, slots.slot(k), size(k));
     }
     return;
   }
@@ -142,15 +239,13 @@ void copy_d2h(Ctx* c, void* dst, const void* src, size_t bytes) {
 void copy_h2d(Ctx* c, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
   c->h2d_bytes += bytes;
-  if (through_slots(c, src, bytes)) {
+  if (SlotLease slots{c, src, bytes}) {
     for (size_t at = 0, i = 0; at < bytes; at += kSlotBytes, ++i) {
-      const int s = (int)(i % kCopySlots);
       const size_t n = std::min(kSlotBytes, bytes - at);
-      KT_CUDA(cudaEventSynchronize(c->slot_done[s]));
-      parallel_memcpy(c->slots + s * kSlotBytes, static_cast<const char*>(src) + at, n);
-      KT_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + at, c->slots + s * kSlotBytes, n, cudaMemcpyHostToDevice,
-                              c->stream));
-      KT_CUDA(cudaEventRecord(c->slot_done[s], c->stream));
+      KT_CUDA(cudaEventSynchronize(slots.done(i)));
+      parallel_memcpy(slots.slot(i), static_cast<const char*>(src) + at, n);
+      KT_CUDA(cudaMemcpyAsync(static_cast<char*>(dst) + at, slots.slot(i), n, cudaMemcpyHostToDevice, c->stream));
+      KT_CUDA(cudaEventRecord(slots.done(i), c->stream));
     }
     return;
   }
