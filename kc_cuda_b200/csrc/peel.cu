@@ -1297,16 +1297,27 @@ struct Peeler {
                               c->stream));
     KT_LAUNCHED(c);
     na = m;
-    threads = kLevelThreads;
-    auto rows_smem = [&] { return s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, threads); };
-    while (threads > 256 && rows_smem() > kRowsSmem) threads /= 2;
     coop_grid = 0;
     build_table();
-    smem = table.get() ? sizeof(RowBatch) : rows_smem();
     if (c->opt.persistent || s->W) {
       allow_max_dynamic_smem(kernel());
+      // The threads of a block that leave most warps on an SM beside the rows'
+      // shared memory, the larger number where they are equal.  (Beyond some 1,700
+      // words one block of 512 fits, three of 256 or seven of 128, and a round of
+      // decrements waits for its chains of accesses: 36M edges on 60,000 vertices
+      // 2,493 ms with 16 warps, 1,730 with 24, 1,530 with 28.)
       int per_sm = 0;
-      KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel(), (int)threads, smem));
+      threads = 0;
+      for (unsigned t = kLevelThreads; t >= 128; t /= 2) {
+        const size_t want = table.get() ? sizeof(RowBatch) : s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, t);
+        if (t > 128 && want > kRowsSmem) continue;
+        int fit = 0;
+        KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel(), (int)t, want));
+        if (threads && fit * t <= per_sm * threads) continue;
+        per_sm = fit;
+        threads = t;
+        smem = want;
+      }
       // A warp counts eight edges at once, or looks up kJobWide entries a lane.
       coop_grid = coop_blocks_for(std::min(coop_blocks(c, per_sm), kMaxGrid), s->m, threads / 4);
     }
