@@ -918,11 +918,12 @@ __global__ void __launch_bounds__(kLevelThreads, 2)
         continue;
       }
       const uint32_t thr = A.gthr_max ? __ldcg(A.gthr_max) : V.thr;
-      // (Beyond short rows a factor of 2: decrements dealt one per lane cost
-      // half of what the option's scale was set for; 64 mix graphs in a batch
-      // 167.9 ms without it, 163.9 with 2, 165.4 with 5.  Counts over short rows
-      // are cheaper too: the Chung-Lu solve 18.0 ms without it, 18.2 with 2.)
-      const double scale = A.R.W <= kShortRow ? 1.0 : 2.0;
+      // (A factor of 2 for unions with rows beyond the short ones, whose graphs'
+      // thresholds are at most thr, many of them well below it: 64 mix graphs in a
+      // batch 167.9 ms without it, 163.9 with 2, 165.4 with 5.  For one graph thr is
+      // its own: 8.5M edges on 12,000 vertices 43 ms without a factor, 58 with 2; the
+      // Chung-Lu solve, short rows, 18.0 and 18.2.)
+      const double scale = A.gthr && A.R.W > kShortRow ? 2.0 : 1.0;
       const bool recount = A.R.bits && (double)nf * (double)(thr > 0 ? thr : 1) * (double)A.gamma >
                                            scale * (double)alive * (double)A.wavg;
       pending += nf;

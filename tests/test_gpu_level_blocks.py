@@ -1,6 +1,8 @@
 """Truss levels over the longest bitset rows, where a block has 128 threads
 instead of 512 (the rows' shared memory), at both sides of that line and up to
-the most vertices that have bitsets."""
+the most vertices that have bitsets; and when a round counts anew."""
+import re
+
 import numpy as np
 import pytest
 
@@ -31,4 +33,20 @@ def test_levels_over_long_rows(n, capfd):
         assert "(n %d, W %d)" % (n, ((n + 31) // 32 + 3) & ~3) in capfd.readouterr().err
         ctx.set_option("recount_gamma", 1)
         assert np.array_equal(g.trussness(), want)
+        g.free()
+
+
+def test_one_graph_counts_anew_where_decrements_cost_more(capfd):
+    """Rounds that take a few per cent of a graph's edges: counting the others
+    anew costs less than closing the triangles of those (with the factor that a
+    union's largest threshold asks for, the last climb counted in no round)."""
+    rng = np.random.default_rng(4000)
+    u, v = np.nonzero(np.triu(rng.random((4000, 4000), dtype=np.float32) < 0.08, 1))
+    with K.Context(0) as ctx:
+        g = ctx.load_edges(np.stack([u, v], 1))
+        ctx.set_option("verbose", 1)
+        got = g.kmax_truss()
+        recounts = [int(x) for x in re.findall(r"rounds \((\d+) recount\)", capfd.readouterr().err)]
+        assert got == O.solve_edges(g.edges())
+        assert sum(recounts) >= 4
         g.free()
