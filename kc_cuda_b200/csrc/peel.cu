@@ -231,6 +231,37 @@ __device__ __forceinline__ void close_common(const PeelArgs& A, const Level& V, 
   }
 }
 
+// The whole rows, each lane closing the set bits of its own words: where a
+// frontier edge has far fewer common neighbours (at most thr) than its rows have
+// words, a step of 32 words has few and hardly two in a word, and dealing them
+// costs more than it spreads (36M edges on 60,000 vertices, thresholds up to 23,
+// rows of 1,876 words: 1,530 -> 1,330 ms; 1.2M on 12,000: 4.9 -> 4.3; with a
+// line at 4 instead of 8 words a neighbour the same).
+constexpr uint32_t kOwnWords = 8;
+
+__device__ __forceinline__ void close_own_words(const PeelArgs& A, const Level& V, uint32_t e, uint32_t x, uint32_t y,
+                                                uint32_t thr, uint32_t W, uint32_t r, uint32_t* next,
+                                                unsigned long long* ncnt, uint32_t& ndec) {
+  const uint32_t *rx = A.R.bits + A.R.off(x), *ry = A.R.bits + A.R.off(y);
+  const uint64_t ox = A.off[x], oy = A.off[y];
+  for (uint32_t i = lane_id(); i < ((W + 31) & ~31u); i += 32) {
+    uint32_t m = i < W ? __ldcg(rx + i) & __ldcg(ry + i) : 0u;
+    while (__any_sync(kFull, m)) {
+      bool pa = false, pb = false;
+      uint32_t a = 0, b = 0;
+      if (m) {
+        const uint32_t col = i * 32 + __ffs(m) - 1;
+        m &= m - 1;
+        a = A.eid[ox + A.R.rank(x, col)];
+        b = A.eid[oy + A.R.rank(y, col)];
+        close_triangle(A, V, e, a, b, r, thr, pa, pb, ndec);
+      }
+      push_warp_full(pa, a, next, ncnt, A.cap, &A.words->err);
+      push_warp_full(pb, b, next, ncnt, A.cap, &A.words->err);
+    }
+  }
+}
+
 // One frontier edge, one warp.  Pushes into next / ncnt; adds the edge's
 // alive degrees and its decrements to the per-thread tallies.
 __device__ __forceinline__ void peel_edge(const PeelArgs& A, const Level& V, uint32_t e, uint32_t r, uint32_t* next,
@@ -256,7 +287,11 @@ __device__ __forceinline__ void peel_edge(const PeelArgs& A, const Level& V, uin
     // Dense rows shorter than the two lists: AND the two bitset rows, 32
     // words a step.
     const uint32_t W = A.R.words(x);
-    for (uint32_t w0 = 0; w0 < W; w0 += 32) close_common(A, V, e, x, y, thr, W, w0, 32, r, next, ncnt, ndec);
+    if (W >= kOwnWords * thr) {
+      close_own_words(A, V, e, x, y, thr, W, r, next, ncnt, ndec);
+    } else {
+      for (uint32_t w0 = 0; w0 < W; w0 += 32) close_common(A, V, e, x, y, thr, W, w0, 32, r, next, ncnt, ndec);
+    }
     tdec += ndec;
     return;
   }
@@ -766,6 +801,13 @@ struct PeelTeam {
   uint64_t bit0, bit_words;  // its bitset rows
   float wavg;
 };
+// Rows from this many words on (16,000 vertices): blocks of 256 threads, five to
+// an SM where the rows' shared memory allows, with fewer registers a thread.  Rounds
+// there are mostly merges and intersections of long rows, a chain of accesses per
+// warp, and take as long as there are few warps: 5M edges on 20,000 vertices 37.5 ms
+// with 32 warps on an SM, 33.0 with 40; 10M on 40,000 133.9 and 122.6.  Shorter rows
+// are recounted more, which spilled registers slow down.
+constexpr uint32_t kWideRow = 512;
 constexpr unsigned kMaxPeelTeams = 32;  // (their results are read through the context's pinned words)
 
 __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcnt, uint32_t* gmin, uint32_t* kmax,
@@ -793,15 +835,15 @@ __device__ __forceinline__ void record_group(uint32_t g, unsigned long long* gcn
 // removes a few edges took 105 us (a core of 1,311 vertices, 609,432 edges), now
 // 43 us.  Dense mode uses W words of shared memory per warp for the recount
 // rounds.
-// Two blocks of 512 threads per SM: a barrier of 296 blocks takes 1.6 us, of 592
+// Two blocks of 512 threads per SM (of long rows: kWideRow): a barrier of 296 blocks takes 1.6 us, of 592
 // blocks of 256 threads 2.3 (64 mix graphs: 29.6 -> 29.1 ms of levels; one
 // block of 1024 threads waits longer for its own warps on small graphs).
 //
 // kTeams: the graphs of a union by teams of blocks, as in the core
 // decomposition (Peeler::init_teams): 64 cores of up to 1,340 vertices, 3.9M
 // edges, in step 516 rounds and 15.1 ms, by teams 232 at most and 10.7.
-template <bool kLists, bool kTeams>
-__global__ void __launch_bounds__(kLevelThreads, 2)
+template <bool kLists, bool kTeams, unsigned kThreads, unsigned kBlocks>
+__global__ void __launch_bounds__(kThreads, kBlocks)
     k_levels(const __grid_constant__ PeelArgs all, const __grid_constant__ LevelsArgs all_levels) {
   extern __shared__ __align__(16) uint32_t dense_smem[];
   __shared__ __align__(16) unsigned char args_store[sizeof(PeelArgs)], levels_store[sizeof(LevelsArgs)];
@@ -1304,12 +1346,14 @@ struct Peeler {
       allow_max_dynamic_smem(kernel());
       // The threads of a block that leave most warps on an SM beside the rows'
       // shared memory, the larger number where they are equal.  (Beyond some 1,700
-      // words one block of 512 fits, three of 256 or seven of 128, and a round of
+      // words one block of 512 would fit, three of 256 or seven of 128, and a round of
       // decrements waits for its chains of accesses: 36M edges on 60,000 vertices
       // 2,493 ms with 16 warps, 1,730 with 24, 1,530 with 28.)
       int per_sm = 0;
+      const unsigned widest = s->W < kWideRow ? kLevelThreads : kLevelThreads / 2;
+      const unsigned most = s->W < kWideRow ? 2 * kLevelThreads : 5 * (kLevelThreads / 2);  // by registers
       threads = 0;
-      for (unsigned t = kLevelThreads; t >= 128; t /= 2) {
+      for (unsigned t = widest; t >= 128 && per_sm * threads < most; t /= 2) {
         const size_t want = table.get() ? sizeof(RowBatch) : s->W <= kShortRow ? 0 : dense_smem_bytes(s->W, t);
         if (t > 128 && want > kRowsSmem) continue;
         int fit = 0;
@@ -1325,8 +1369,10 @@ struct Peeler {
   }
 
   const void* kernel() const {
-    if (table.get()) return (const void*)k_levels<true, false>;
-    return teams.empty() ? (const void*)k_levels<false, false> : (const void*)k_levels<false, true>;
+    if (table.get()) return (const void*)k_levels<true, false, kLevelThreads, 2>;
+    if (!teams.empty()) return (const void*)k_levels<false, true, kLevelThreads, 2>;
+    return s->W < kWideRow ? (const void*)k_levels<false, false, kLevelThreads, 2>
+                           : (const void*)k_levels<false, false, kLevelThreads / 2, 5>;
   }
 
   // List mode: the edge hash table, 8 to 20 bytes an edge, when the budget
@@ -1600,7 +1646,7 @@ struct Peeler {
       words[g + 1] = words[g] + (uint64_t)s->group_n[g] * (((s->group_n[g] + 31) / 32 + 3) & ~3u);
     }
     const std::vector<uint64_t> at = gather_offsets(c, s->off.as<uint64_t>(), starts);
-    const void* by_teams = (const void*)k_levels<false, true>;
+    const void* by_teams = (const void*)k_levels<false, true, kLevelThreads, 2>;
     allow_max_dynamic_smem(by_teams);
     int per_sm = 0;
     KT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, by_teams, (int)threads, smem));

@@ -1,6 +1,8 @@
-"""Truss levels over the longest bitset rows, where a block has 128 threads
-instead of 512 (the rows' shared memory), at both sides of that line and up to
-the most vertices that have bitsets; and when a round counts anew."""
+"""Truss levels over long bitset rows, where a block has 256 or 128 threads
+instead of 512 (the rows' shared memory), at both sides of the lines and up to
+the most vertices that have bitsets, with common neighbours dealt to a warp's
+lanes and closed by the lanes whose words hold them; and when a round counts
+anew."""
 import re
 
 import numpy as np
@@ -12,7 +14,7 @@ import kc_cuda_b200 as K
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [50_000, 57_000, 60_001, 65_536])
+@pytest.mark.parametrize("n", [16_200, 16_384, 50_000, 57_000, 60_001, 65_536])
 def test_levels_over_long_rows(n, capfd):
     rng = np.random.default_rng(n)
     ring = np.stack([np.arange(n), (np.arange(n) + 1) % n])  # every vertex has an edge
