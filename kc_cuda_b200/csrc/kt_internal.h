@@ -157,10 +157,6 @@ class DBuf {
   size_t bytes_ = 0;
 };
 
-struct Stats {
-  kt_stats s{};
-};
-
 constexpr size_t kPinnedBytes = 4096;
 
 struct Ctx {
@@ -251,8 +247,6 @@ void zero(Ctx* c, void* dptr, size_t bytes);
 void scan_u32_to_u64(Ctx* c, const uint32_t* in, uint64_t* out, uint64_t n);
 // Exclusive scan of n uint32 values into uint32 (out may alias in).
 void scan_u32(Ctx* c, const uint32_t* in, uint32_t* out, uint64_t n);
-// Sum of n uint32 values (device result in *dsum, also returned).
-uint64_t reduce_u32(Ctx* c, const uint32_t* in, uint64_t n);
 // Bits [lo, hi) of a key.
 struct BitField {
   int lo, hi;

@@ -1,4 +1,4 @@
-// Device-wide scans, reductions and the sorted-unique compaction.
+// Device-wide scans and the sorted-unique compaction.
 //
 // Scans and compactions (compact.cuh) take one pass over the data in one
 // launch: tiles of 2048 items (256 threads x 8) find their prefix by decoupled
@@ -99,15 +99,6 @@ void scan_impl(Ctx* c, const Tin* in, Tout* out, uint64_t n) {
   if (tiles > 1) end_lookback(c, tiles);
 }
 
-__global__ void k_reduce_u32(const uint32_t* __restrict__ in, uint64_t n, unsigned long long* out) {
-  __shared__ uint64_t tmp[33];
-  uint64_t s = 0;
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    s += in[i];
-  s = block_sum<uint64_t>(s, tmp);
-  if (threadIdx.x == 0 && s) atomicAdd(out, (unsigned long long)s);
-}
-
 // Distinct keys of a sorted list, ~0 dropped.
 struct DistinctKey {
   const uint64_t* in;
@@ -122,16 +113,6 @@ struct DistinctKey {
 
 void scan_u32(Ctx* c, const uint32_t* in, uint32_t* out, uint64_t n) { scan_impl<uint32_t, uint32_t>(c, in, out, n); }
 void scan_u32_to_u64(Ctx* c, const uint32_t* in, uint64_t* out, uint64_t n) { scan_impl<uint32_t, uint64_t>(c, in, out, n); }
-
-uint64_t reduce_u32(Ctx* c, const uint32_t* in, uint64_t n) {
-  DBuf acc(c, 8);
-  zero(c, acc.get(), 8);
-  if (n) {
-    k_reduce_u32<<<grid_for(n, 256, 4 * 148 * 8), 256, 0, c->stream>>>(in, n, acc.as<unsigned long long>());
-    KT_LAUNCHED(c);
-  }
-  return read_word<uint64_t>(c, acc.as<uint64_t>());
-}
 
 uint64_t unique_sorted_u64(Ctx* c, const uint64_t* in, uint64_t* out, uint64_t n) {
   return compact(c, n, DistinctKey{in}, out);
