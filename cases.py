@@ -4,7 +4,7 @@
 
 Cases (each fits in a few GB of device memory, inputs larger than L2):
   dense-support   Erdos-Renyi G(n=40000, M=48,000,000 draws), seed 7: one
-                  kt_edge_support call -> k_dense_support<64> on ~46M edges
+                  kt_edge_support call -> k_dense_support on ~46M edges
                   (bitset rows of 1250 words).
   core55k-support Erdos-Renyi G(n=55455, M=95,000,000 draws), seed 7: one
                   kt_edge_support call -> k_dense_support on ~92M edges with
@@ -12,11 +12,11 @@ Cases (each fits in a few GB of device memory, inputs larger than L2):
                   shape of the bench graph's search core (55,455 vertices,
                   92.1M edges).
   er1m-support    Erdos-Renyi G(n=1,000,000, M=64,000,000 draws), seed 7: one
-                  kt_edge_support call in list mode -> k_support_bitmap
+                  kt_edge_support call in list mode -> k_support_filter
                   (average degree ~128, the shape of the mix's largest
                   Erdos-Renyi graphs).
   rmat21-solve    R-MAT scale 21, edge factor 32, seed 2, cliques 80/120/200:
-                  one kt_solve_staged (every stage; peel kernel k_cascade<8>).
+                  one kt_solve_staged (every stage; peel kernel k_levels).
   rmat16-solve    config-1 graph (R-MAT scale 16, edge factor 16, seed 1, K30).
   rmat24-solve    the bench graph (R-MAT scale 24, edge factor 32, seed 2,
                   cliques 80/120/200; 15.5 GB of TSV staged on the device).
@@ -29,7 +29,7 @@ Cases (each fits in a few GB of device memory, inputs larger than L2):
                   (k_core_levels on the union, grouped support and peel).
   mix-largest     the --count largest of mix graphs 0..4095 (by draws) in one
                   kt_batch_run; --alone also solves them one at a time.
---verbose prints the solver's stage decisions and per-level cascades
+--verbose prints the solver's stage decisions and the levels' launches
 (--verbose-alone: also for the graphs solved one at a time).
 """
 from __future__ import annotations

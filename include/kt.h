@@ -314,6 +314,8 @@ typedef struct kt_stats {
   uint64_t kernel_launches;       /* kernels this context launched since kt_stats_reset */
   uint64_t core_vertices, core_edges;       /* search-phase subgraph */
   uint64_t predict_vertices, predict_edges; /* prediction-phase subgraph */
+  /* levels, rounds: of the truss peels.  Where teams of blocks take the graphs
+   * of a union, a peel counts those of the team that took most. */
   uint32_t cmax, kmax_lower_bound, levels, rounds;
   uint64_t support_bytes, peel_bytes;       /* algorithmic bytes of the last solve: a merge
                                                intersection's reads (support); list reads and

@@ -9,15 +9,15 @@
 //   ascending order.  The rows are the lines themselves, as the reference
 //   builds them by concatenation (init_graph, src/kc_gpu.cpp:38-65, degrees
 //   from run lengths at src/kc_gpu.cpp:283-302): one pass checks the order,
-//   writes the adjacency and the row offsets; a second pass checks symmetry
-//   (every arc (y -> x) with x < y is found in row x by binary search, and
-//   the arcs with x > y are as many as those with x < y) and writes the
-//   canonical edge list, which is the x > y arcs in line order.  Any check
-//   that fails sends the records to the general route; nothing is modified
-//   before that decision.
+//   writes the adjacency and the row offsets; a second one, once the arcs with
+//   x > y are known to be as many as those with x < y, writes the former, in
+//   line order, as the canonical edge list and the latter transposed; a radix
+//   sort of those by their high half compares them, in its last pass, with
+//   the edge list (symmetry).  Any check that fails sends the records to the
+//   general route; nothing is modified before that decision.
 // * General route -- records in any order with repeats and self-loops:
-//   canonical keys min << 32 | max (~0 = no edge) radix sorted over
-//   2*ceil(log2 n) bits, repeats dropped by a sorted-unique compaction, and
+//   canonical keys min << 32 | max (~0 = no edge) radix sorted over the bits
+//   that ids below n use, repeats dropped by a sorted-unique compaction, and
 //   the symmetric CSR filled from the unique list: degrees with warp-
 //   aggregated atomics (runs of equal u in the sorted list collapse to one
 //   atomic), an exclusive scan for the uint64 row offsets, and a cursor

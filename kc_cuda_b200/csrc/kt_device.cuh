@@ -182,14 +182,14 @@ struct Crew {
 
 // Bounded grid barrier for kernels launched with cudaLaunchCooperativeKernel
 // (which guarantees that every block is resident).  Every block (or every
-// block of the crew that `w` belongs to) must call it the same number of times.  A wait longer than `timeout_ns` sets
-// kDevErrBarrier and returns; callers test the returned flag and leave the
-// kernel, so a mismatch can never hang the device.  Returns true when no
-// error is flagged.
+// block of the crew that `w` belongs to) must call it the same number of times.
+// A wait longer than `timeout_ns` sets kDevErrBarrier and returns; callers test
+// the returned flag and leave the kernel, so a mismatch can never hang the
+// device.  Returns true when no error is flagged.
 //
 // One thread per block arrives with one atomic -- block 0 adds what flips bit
 // 31 once the others' ones are in, so the word needs no reset and no second
-// atomic -- and polls (error, phase) as one 64-bit word.  Only that thread
+// atomic, the arrival of CUDA's cooperative groups' grid sync -- and polls (error, phase) as one 64-bit word.  Only that thread
 // touches the barrier's words: what every thread needs after it (the flag, and
 // with grid_barrier_read up to N device counters) comes from it through
 // __syncthreads_and and shared memory.  Several thousand warps loading one
